@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>:
             right_state<DIM>(bc.type, bc.state, s1, s2, n, gamma, cov, (decltype(gamma))prm.rgas);
           }
           R F[NEQ];
-          const R sp = checked_speed(prm, riemann<DIM>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e, pb);
+          const R sp = checked_speed(prm, riemann<DIM, R, G == 3 && P == 1>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e, pb);
           lmax = fmax(lmax, sp);
           const R* Bo = sB[lf][side ? q2 : q];
           const R wq = sW[q];
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>:
             right_state<DIM>(bc.type, bc.state, s1, s2, n, gamma, cov, (decltype(gamma))prm.rgas);
           }
           R F[NEQ];
-          const R sp = checked_speed(prm, riemann<DIM>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e, pb);
+          const R sp = checked_speed(prm, riemann<DIM, R, G == 3 && P == 1>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e, pb);
           lmax = fmax(lmax, sp);
           const R* Bo = sB[lf][side ? q2 : q];
           const R wq = sW[q];

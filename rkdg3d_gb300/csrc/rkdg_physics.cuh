@@ -104,60 +104,91 @@ __device__ __forceinline__ R max_char_speed(const R* s, R gamma, R b) {
   return fsq(fdv(v2, den)) + c;
 }
 
-// FP32 pointwise state quantities with one reciprocal of the density and one
-// of the covolume factor: r = 1/rho, q = 1/(1 - rho b), the pressure (FP64
-// where E - |m|^2/(2 rho) cancels, as pressure() does) and |u| + c.  Returns
-// false where StateIsPhysicalSay fails (rho < 0, E <= 0, perfect-gas p <= 0,
-// NaN).  Same quantities as the double path, rounded in a different order.
-template <int DIM>
-__device__ __forceinline__ bool state_f32(const float* s, float gamma, float b, float& r, float& q,
-                                          float& p, float& speed) {
-  const float den = s[0], E = s[1 + DIM];
-  if (!(den >= 0.0f) || !(E > 0.0f)) return false;
-  r = __fdividef(1.0f, den);
-  float m2 = 0.0f;
+// 1/x: double rounded to nearest, float the hardware approximation.
+template <typename R>
+__device__ __forceinline__ R rcp(R x) {
+  return R(1) / x;
+}
+template <>
+__device__ __forceinline__ float rcp<float>(float x) {
+  return __fdividef(1.0f, x);
+}
+
+// Pointwise state quantities with one reciprocal of the density and one of
+// the covolume factor (none for a perfect gas): r = 1/rho, q = 1/(1 - rho b),
+// the pressure (float: FP64 where E - |m|^2/(2 rho) cancels, as pressure()
+// does) and u2 = |u|^2.  Returns false where StateIsPhysicalSay fails
+// (rho < 0, E <= 0, perfect-gas p <= 0, NaN).  An FP64 quotient takes 8-9
+// instructions of a pipe that issues two per clock and SM; the flux formulas
+// written with their own quotients spent more than half of the FP64 stage
+// kernels in 18-23 of them per face point.
+template <int DIM, typename R>
+__device__ __forceinline__ bool eos_state(const R* s, R gamma, R b, R& r, R& q, R& p, R& u2) {
+  const R den = s[0], E = s[1 + DIM];
+  if (!(den >= R(0)) || !(E > R(0))) return false;
+  r = rcp(den);
+  R m2 = R(0);
 #pragma unroll
-  for (int d = 0; d < DIM; d++) m2 = fmaf(s[1 + d], s[1 + d], m2);
-  const float v2 = m2 * r;  // |m|^2 / rho
-  const float ie = E - 0.5f * v2;
-  if (!((gamma - 1.0f) * ie > 0.0f)) return false;
-  q = __fdividef(1.0f, 1.0f - den * b);
-  if (fabsf(ie) < 1e-3f * fabsf(E)) {
-    double m2d = 0.0;
+  for (int d = 0; d < DIM; d++) m2 += s[1 + d] * s[1 + d];
+  const R v2 = m2 * r;  // |m|^2 / rho
+  const R ie = E - R(0.5) * v2;
+  const R pg = (gamma - R(1)) * ie;
+  if (!(pg > R(0))) return false;
+  q = b == R(0) ? R(1) : rcp(R(1) - den * b);
+  p = pg * q;
+  if constexpr (std::is_same<R, float>::value) {
+    if (fabsf(ie) < 1e-3f * fabsf(E)) {
+      double m2d = 0.0;
 #pragma unroll
-    for (int d = 0; d < DIM; d++) m2d += (double)s[1 + d] * (double)s[1 + d];
-    p = (float)(((double)gamma - 1.0) * ((double)E - 0.5 * m2d / (double)den) /
-                (1.0 - (double)den * (double)b));
-  } else {
-    p = (gamma - 1.0f) * ie * q;
+      for (int d = 0; d < DIM; d++) m2d += (double)s[1 + d] * (double)s[1 + d];
+      p = (float)(((double)gamma - 1.0) * ((double)E - 0.5 * m2d / (double)den) /
+                  (1.0 - (double)den * (double)b));
+    }
   }
-  speed = fsq(v2 * r) + fsq(gamma * p * r * q);
+  u2 = v2 * r;
   return true;
 }
 
-// FP32 Rusanov flux (rs_rusanov.cpp:6-40) on unrotated states, built on
-// state_f32.  Returns the wave speed, or -1 for a non-physical state.
-template <int DIM>
-__device__ __forceinline__ float rusanov_f32(const float* s1, const float* s2, const float* n,
-                                             float* flux, float gamma, float b) {
+// 1/|n| of a face normal: unit to rounding in every table (two terms of the
+// series about 1), else the reciprocal root.
+template <typename R>
+__device__ __forceinline__ R inv_norm(R nn) {
+  const R d = nn - R(1);
+  if (fabs(d) < R(1e-6)) return R(1) + d * (R(0.375) * d - R(0.5));
+  return R(1) / sqrt(nn);
+}
+
+// Rusanov flux (rs_rusanov.cpp:6-40) on unrotated states.  Returns the wave
+// speed, or -1 for a non-physical state.  max(|u| + c) is the root of
+// max(|u|^2 + c^2 + 2 |u| c): three square roots for the two sides.
+template <int DIM, typename R>
+__device__ __forceinline__ R rusanov_flux(const R* s1, const R* s2, const R* n, R* flux, R gamma,
+                                          R b) {
   constexpr int NEQ = DIM + 2;
-  float r1, q1, p1, e1, r2, q2, p2, e2;
-  if (!state_f32<DIM>(s1, gamma, b, r1, q1, p1, e1)) return -1.0f;
-  if (!state_f32<DIM>(s2, gamma, b, r2, q2, p2, e2)) return -1.0f;
-  const float maxE = e1 > e2 ? e1 : e2;
-  float d1 = 0.0f, d2 = 0.0f, nn = 0.0f;
+  R r1, q1, p1, w1, r2, q2, p2, w2;
+  if (!eos_state<DIM>(s1, gamma, b, r1, q1, p1, w1)) return R(-1);
+  if (!eos_state<DIM>(s2, gamma, b, r2, q2, p2, w2)) return R(-1);
+  R maxE;
+  if constexpr (std::is_same<R, double>::value) {
+    const R c1 = gamma * p1 * r1 * q1, c2 = gamma * p2 * r2 * q2;
+    maxE = sqrt(fmax(w1 + c1 + R(2) * sqrt(w1 * c1), w2 + c2 + R(2) * sqrt(w2 * c2)));
+  } else {
+    const R e1 = fsq(w1) + fsq(gamma * p1 * r1 * q1), e2 = fsq(w2) + fsq(gamma * p2 * r2 * q2);
+    maxE = e1 > e2 ? e1 : e2;
+  }
+  R d1 = R(0), d2 = R(0), nn = R(0);
 #pragma unroll
   for (int d = 0; d < DIM; d++) {
-    d1 = fmaf(s1[1 + d], n[d], d1);
-    d2 = fmaf(s2[1 + d], n[d], d2);
-    nn = fmaf(n[d], n[d], nn);
+    d1 += s1[1 + d] * n[d];
+    d2 += s2[1 + d] * n[d];
+    nn += n[d] * n[d];
   }
-  const float h = 0.5f * rsqrtf(nn), a = 0.5f * maxE;
-  const float u1 = d1 * r1, u2 = d2 * r2;
+  const R h = R(0.5) * inv_norm(nn), a = R(0.5) * maxE;
+  const R u1 = d1 * r1, u2 = d2 * r2;
   flux[0] = h * (d1 + d2) - a * (s2[0] - s1[0]);
 #pragma unroll
   for (int d = 0; d < DIM; d++)
-    flux[1 + d] = h * (fmaf(u1, s1[1 + d], p1 * n[d]) + fmaf(u2, s2[1 + d], p2 * n[d])) -
+    flux[1 + d] = h * ((u1 * s1[1 + d] + p1 * n[d]) + (u2 * s2[1 + d] + p2 * n[d])) -
                   a * (s2[1 + d] - s1[1 + d]);
   flux[NEQ - 1] = h * (u1 * (s1[NEQ - 1] + p1) + u2 * (s2[NEQ - 1] + p2)) -
                   a * (s2[NEQ - 1] - s1[NEQ - 1]);
@@ -168,27 +199,28 @@ __device__ __forceinline__ float rusanov_f32(const float* s1, const float* s2, c
 // (FE_Evolution::GetFlux, fe_evolution.cpp:219-245).
 template <int DIM, typename R>
 __device__ __forceinline__ R flux_and_speed(const R* s, R F[DIM + 2][DIM], R gamma, R b) {
-  if constexpr (std::is_same<R, float>::value) {
-    float r, q, p, speed;
-    if (!state_f32<DIM>(s, gamma, b, r, q, p, speed)) {
-      // non-physical node: same arithmetic as the double path
-      r = __fdividef(1.0f, s[0]);
+  if constexpr (std::is_same<R, float>::value || std::is_same<R, double>::value) {
+    R r, q, p, u2;
+    if (!eos_state<DIM>(s, gamma, b, r, q, p, u2)) {
+      // non-physical node: the same quantities without the checks
+      r = rcp(s[0]);
       p = pressure<DIM>(s, gamma, b);
-      float m2 = 0.0f;
+      u2 = R(0);
 #pragma unroll
-      for (int d = 0; d < DIM; d++) m2 += s[1 + d] * s[1 + d];
-      speed = fsq(m2 * r * r) + fsq(fdv(gamma * p * r, 1.0f - s[0] * b));
+      for (int d = 0; d < DIM; d++) u2 += s[1 + d] * s[1 + d];
+      u2 = u2 * r * r;
+      q = rcp(R(1) - s[0] * b);
     }
 #pragma unroll
     for (int d = 0; d < DIM; d++) {
-      const float ud = s[1 + d] * r;
+      const R ud = s[1 + d] * r;
       F[0][d] = s[1 + d];
 #pragma unroll
       for (int i = 0; i < DIM; i++) F[1 + i][d] = s[1 + i] * ud;
       F[1 + d][d] += p;
       F[1 + DIM][d] = (s[1 + DIM] + p) * ud;
     }
-    return speed;
+    return fsq(u2) + fsq(gamma * p * r * q);
   }
   const R den = s[0];
   const R inv = fdv(R(1), den);
@@ -249,8 +281,9 @@ __device__ __forceinline__ void rotate(R* s, const R* n) {
     const R sp = n[2];
     const R cp = fsq(R(1) - sp * sp);
     const bool ok = fabs(cp) > R(1e-6);
-    const R st = ok ? fdv(n[1], cp) : R(1);
-    const R ct = ok ? fdv(n[0], cp) : R(0);
+    const R ic = fdv(R(1), cp);
+    const R st = ok ? n[1] * ic : R(1);
+    const R ct = ok ? n[0] * ic : R(0);
     const R mx = cp * ct * m[0] + cp * st * m[1] + sp * m[2];
     const R my = -st * m[0] + ct * m[1];
     const R mz = -sp * ct * m[0] - sp * st * m[1] + cp * m[2];
@@ -271,8 +304,9 @@ __device__ __forceinline__ void inverse_rotate(R* s, const R* n) {
     const R sp = n[2];
     const R cp = fsq(R(1) - sp * sp);
     const bool ok = fabs(cp) > R(1e-6);
-    const R st = ok ? fdv(n[1], cp) : R(1);
-    const R ct = ok ? fdv(n[0], cp) : R(0);
+    const R ic = fdv(R(1), cp);
+    const R st = ok ? n[1] * ic : R(1);
+    const R ct = ok ? n[0] * ic : R(0);
     const R mx = cp * ct * m[0] - st * m[1] - sp * ct * m[2];
     const R my = cp * st * m[0] + ct * m[1] - sp * st * m[2];
     const R mz = sp * m[0] + cp * m[2];
@@ -332,16 +366,150 @@ __device__ __forceinline__ void wave_speeds(const R* s1, const R* s2, R p1, R p2
   SR = uR + qR * cR;
 }
 
+// x^(1/n) for x > 0 and a small whole n: the FP32 power as a start value and one
+// step of Halley's method (cubic convergence: 1e-7 -> below 1e-19), a third of
+// the FP64 instructions of exp2(log2(x) / n).
+__device__ __forceinline__ double root_n(double x, int n, double invn) {
+  if (!(x > 1e-30 && x < 1e30)) return exp2(invn * log2(x));
+  const double y = (double)exp2f((float)invn * log2f((float)x));
+  double yn = y;
+  for (int i = 1; i < n; ++i) yn *= y;
+  const double m = n - 1, k = n + 1;
+  return y * (m * yn + k * x) / (k * yn + m * x);
+}
+
+// TRRS wave speeds (ComputeToroCharSpeeds, physics.cpp:309-350) from the
+// normal velocities, sound speeds and pressures of the two sides.  With
+//   B = cL + cR (pL/pR)^z,  A = cL + cR - (gamma - 1)/2 (uR - uL),
+// pStar / pL = (A/B)^(1/z): two powers instead of three, the second a product
+// where 1/z = 2 gamma/(gamma - 1) is whole (7 for gamma = 1.4) and the first a
+// root then.
+template <typename R>
+__device__ __forceinline__ void trrs_speeds(R uL, R uR, R cL, R cR, R pL, R pR, R gamma, R& SL, R& SR) {
+  const R gm1 = gamma - R(1);
+  const R iz = fdv(R(2) * gamma, gm1);
+  const R x = fdv(pL, pR);
+  const int n = (int)rint(iz);
+  const bool whole = n >= 2 && n <= 16 && fabs(iz - R(n)) <= R(n) * (std::is_same<R, double>::value ? R(1e-14) : R(1e-6));
+  R xz;  // (pL/pR)^z
+  if constexpr (std::is_same<R, double>::value)
+    xz = whole ? root_n(x, n, R(1) / iz) : exp2(log2(x) / iz);
+  else
+    xz = exp2f(fdv(log2f(x), iz));
+  const R a = cL + cR - R(0.5) * gm1 * (uR - uL);
+  const R t = fdv(a, cL + cR * xz);
+  R pl;  // pStar / pL
+  if (whole) {
+    pl = t;
+    for (int i = 1; i < n; ++i) pl *= t;
+  } else {
+    pl = powr(t, iz);
+  }
+  const R hg = fdv(R(0.5) * (gamma + R(1)), gamma);
+  const R pr = pl * x;
+  SL = uL - (pl > R(1) ? fsq(R(1) + hg * (pl - R(1))) * cL : cL);
+  SR = uR + (pr > R(1) ? fsq(R(1) + hg * (pr - R(1))) * cR : cR);
+}
+
+// Einfeldt wave speeds (ComputeEinfeldtCharSpeeds, physics.cpp:269-296): the
+// weights sqrt(rho) enter through t = sqrt(rhoR/rhoL) alone, and the sound
+// speeds through their squares.
+template <typename R>
+__device__ __forceinline__ void einfeldt_speeds(R uL, R uR, R cL2, R cR2, R rL, R rhoR, R& SL, R& SR) {
+  const R t = fsq(rhoR * rL);
+  const R wL = rcp(R(1) + t), wR = t * wL;
+  const R du = uR - uL;
+  const R uav = wL * uL + wR * uR;
+  const R cav = fsq(wL * cL2 + wR * cR2 + R(0.5) * wL * wR * du * du);
+  SL = uav - cav;
+  SR = uav + cav;
+}
+
+// LLF, HLL and HLLC (rs_llf.cpp:6-37, rs_hll.cpp:6-50, rs_hllc.cpp:71-161) in
+// plain arithmetic types, on the states rotated into the face frame.
+template <int DIM, typename R>
+__device__ __forceinline__ R hll_family(R* s1, R* s2, const R* n, R* flux, R gamma, R b, int rs,
+                                        int avg) {
+  constexpr int NEQ = DIM + 2;
+  R r1, q1, p1, w1, r2, q2, p2, w2;
+  if (!eos_state<DIM>(s1, gamma, b, r1, q1, p1, w1)) return R(-1);
+  if (!eos_state<DIM>(s2, gamma, b, r2, q2, p2, w2)) return R(-1);
+  rotate<DIM>(s1, n);
+  rotate<DIM>(s2, n);
+  const R u1 = s1[1] * r1, u2 = s2[1] * r2;
+  const R c1 = gamma * p1 * r1 * q1, c2 = gamma * p2 * r2 * q2;  // squares
+  R SL, SR;
+  if (avg == 1)
+    einfeldt_speeds(u1, u2, c1, c2, r1, s2[0], SL, SR);
+  else
+    trrs_speeds(u1, u2, fsq(c1), fsq(c2), p1, p2, gamma, SL, SR);
+  R ret = fmax(fabs(SL), fabs(SR));
+  // x-flux of a rotated state (ComputeFluxF, physics.cpp:198-231)
+  auto side_flux = [&](const R* s, R u, R p, R* f) {
+    f[0] = s[1];
+    f[1] = s[1] * u + p;
+#pragma unroll
+    for (int d = 1; d < DIM; d++) f[1 + d] = s[1 + d] * u;
+    f[NEQ - 1] = (s[NEQ - 1] + p) * u;
+  };
+  if (rs == 1) {
+    R f1[NEQ];
+    side_flux(s1, u1, p1, f1);
+    side_flux(s2, u2, p2, flux);
+    const R a = R(0.5) * ret;
+#pragma unroll
+    for (int i = 0; i < NEQ; ++i) flux[i] = R(0.5) * (f1[i] + flux[i]) - a * (s2[i] - s1[i]);
+  } else if (SL >= R(0)) {
+    side_flux(s1, u1, p1, flux);
+  } else if (SR <= R(0)) {
+    side_flux(s2, u2, p2, flux);
+  } else if (rs == 2) {
+    R f1[NEQ];
+    side_flux(s1, u1, p1, f1);
+    side_flux(s2, u2, p2, flux);
+    const R inv = rcp(SR - SL), pp = SL * SR;
+#pragma unroll
+    for (int i = 0; i < NEQ; ++i)
+      flux[i] = (SR * f1[i] - SL * flux[i] + pp * (s2[i] - s1[i])) * inv;
+  } else {
+    const R k1 = SL - u1, k2 = SR - u2;
+    const R sStar = fdv(p2 - p1 + s1[1] * k1 - s2[1] * k2, s1[0] * k1 - s2[0] * k2);
+    const bool left = sStar > R(0);
+    const R* st = left ? s1 : s2;
+    const R SK = left ? SL : SR, uK = left ? u1 : u2, pK = left ? p1 : p2, kK = left ? k1 : k2;
+    R sK[NEQ];
+#pragma unroll
+    for (int i = 0; i < NEQ; ++i) sK[i] = st[i];
+    side_flux(sK, uK, pK, flux);
+    const R extra = SK * (pK + sK[0] * kK * (sStar - uK));
+    const R inv = rcp(SK - sStar);
+#pragma unroll
+    for (int i = 0; i < NEQ; ++i) {
+      const R v = sStar * (sK[i] * SK - flux[i]);
+      flux[i] = (i == 1 ? v + extra : (i == DIM + 1 ? v + sStar * extra : v)) * inv;
+    }
+  }
+  if (rs == 3) ret = SL > SR ? SL : SR;
+  inverse_rotate<DIM>(flux, n);
+  return ret;
+}
+
 // RiemannSolver*::Eval (rs_rusanov.cpp:6-40, rs_llf.cpp:6-37, rs_hll.cpp:6-50,
 // rs_hllc.cpp:71-161).  s1, s2 are working copies (rotated in place, as the
 // reference does through const_cast); n is the unit normal from side 1 to
 // side 2.  Returns the solver's wave speed, or -1 for a non-physical state.
-template <int DIM, typename R>
+// float and double take the forms above; dual numbers the plain restatement
+// below, and so does float where PLAIN is set: the FP32 Q1 quads, whose
+// batched limited runs pass through thousands of elements that sit within
+// FP32 rounding of the limiter's +-1e-3 switches, so that any other rounding of
+// the flux moves their results by up to 2% in single elements.
+template <int DIM, typename R, bool PLAIN = false>
 __device__ __forceinline__ R riemann(R* s1, R* s2, const R* n, R* flux, R gamma, R b, int rs,
                                      int avg) {
   constexpr int NEQ = DIM + 2;
-  if constexpr (std::is_same<R, float>::value) {
-    if (rs == 0) return rusanov_f32<DIM>(s1, s2, n, flux, gamma, b);
+  if constexpr (std::is_same<R, float>::value || std::is_same<R, double>::value) {
+    if (rs == 0) return rusanov_flux<DIM>(s1, s2, n, flux, gamma, b);
+    if constexpr (!PLAIN || std::is_same<R, double>::value) return hll_family<DIM>(s1, s2, n, flux, gamma, b, rs, avg);
   }
   if (!state_is_physical_say<DIM>(s1, gamma)) return R(-1);
   if (!state_is_physical_say<DIM>(s2, gamma)) return R(-1);
@@ -395,12 +563,8 @@ __device__ __forceinline__ R riemann(R* s1, R* s2, const R* n, R* flux, R gamma,
     } else {
       const R inv = fdv(R(1), SR - SL);
 #pragma unroll
-      for (int i = 0; i < NEQ; ++i) {
-        if constexpr (std::is_same<R, float>::value)
-          flux[i] = (SR * f1[i] - SL * f2[i] + SL * SR * (s2[i] - s1[i])) * inv;
-        else
-          flux[i] = (SR * f1[i] - SL * f2[i] + SL * SR * (s2[i] - s1[i])) / (SR - SL);
-      }
+      for (int i = 0; i < NEQ; ++i)
+        flux[i] = (SR * f1[i] - SL * f2[i] + SL * SR * (s2[i] - s1[i])) * inv;
     }
     ret = maxE;
   } else {
