@@ -57,6 +57,10 @@ struct RefTables {
   int perm[RKDG_MAX_PERM][RKDG_MAX_NQF];     // elem1 point -> elem2 point
   double Bl[RKDG_MAX_NFPE][RKDG_MAX_NQL][RKDG_MAX_ND];  // limiter face points
   double Bv[RKDG_MAX_NV][RKDG_MAX_ND];       // element vertices
+  // the same for the FP32 limiter, node-major: float pairs of Bl at point
+  // lf * nql + q, and Bv rounded
+  float2 Bl32[RKDG_MAX_ND][RKDG_MAX_NFPE * RKDG_MAX_NQL];
+  float Bv32[RKDG_MAX_ND][RKDG_MAX_NV];
   double wmean[RKDG_MAX_ND];                 // cell-mean weights (sum = 1)
   // 1D tables for the sum-factorised tensor kernels
   double l1d[RKDG_MAX_NQF][8];   // 1D basis at 1D face-rule points  [a][j]

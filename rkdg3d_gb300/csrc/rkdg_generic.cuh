@@ -799,355 +799,43 @@ __device__ __forceinline__ void shu_indicator(const LimParams& prm, const R* __r
   }
 }
 
-// Limiter::update for one element (limiter.cpp:22-94): stencil = the element
-// and its face neighbours (ElementToElementTable, limiter.cpp:115-123), the
-// BJ-family indicator at the order-2 points of its interior faces
-// (indicator_bj.cpp:88-200, updateYMin 15-86), then LimiterMultiplier::limit
-// (limiter_multiplier.cpp:12-99, including the nd-fold application of the
-// density factor, quirks Q4/Q5, and the last-hope vertex check) or
-// LimiterFinDiff::limit (limiter_findiff.cpp:3-33, last equation only, Q6).
-// The update reads only this element's values and the cell means, so it is
-// done in place.  DS = true: the values are a float pair (u = hi, ulo = lo)
-// and the multiplier update runs in double-single arithmetic.  The indicator
-// takes its branch decisions (face-point value minus mean against the +-1e-3
-// switches, stencil min/max) on the values the state holds: in FP64 for a
-// double state; for a float state in double-single arithmetic (face-point
-// values from the float state and its low word with the float-pair basis
-// table, about 44 significant bits, so a switch differs from FP64 only within
-// ~1e-13 relative of its threshold), and the ratio and limiter function,
-// which only scale the float multiplier, in FP32.  GB300's FP64 rate is a
-// small fraction of its FP32 rate, and an FP64 indicator made the limiter
-// the FP32 path's largest kernel.
+// LimiterFinDiff::limit (limiter_findiff.cpp:3-33) with the Shu indicator, one
+// thread per element: the element becomes its mean where the last equation's
+// indicator is below 0.999 (the Multi limiter is rejected with Shu).
 template <int G, int P, typename R, bool DS>
 __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>::ND>(),
                                   generic_min_blocks<R, El<G, P>::NEQ * El<G, P>::ND, true>())
-    k_limit_generic(const LimParams prm, R* __restrict__ u, float* __restrict__ ulo) {
+    k_limit_shu(const LimParams prm, R* __restrict__ u, float* __restrict__ ulo) {
   using E = El<G, P>;
-  constexpr int DIM = E::DIM, ND = E::ND, NEQ = E::NEQ, NFPE = E::NFPE, NQL = E::NQL, NV = E::NV;
-  constexpr bool F32 = std::is_same<R, float>::value;
-  // face-point basis: FP64, or a float pair (hi, lo) for a float state
-  __shared__ typename std::conditional<F32, float2, double>::type sBl[NFPE][NQL][ND];
-  __shared__ R sBv[NV][ND];
-  const RefTables* T = prm.tab;
-  // batched problems with a map of the active work: CTAs past it are idle
-  if (prm.act_cum && (int)(blockIdx.x * blockDim.x) >= prm.act_cum[*prm.act_n]) return;
-  for (int t = threadIdx.x; t < NFPE * NQL * ND; t += blockDim.x) {
-    const int s = t % ND, q = (t / ND) % NQL, lf = t / (ND * NQL);
-    const double b = T->Bl[lf][q][s];
-    if constexpr (F32) {
-      const float h = (float)b;
-      sBl[lf][q][s] = make_float2(h, (float)(b - (double)h));
-    } else {
-      sBl[lf][q][s] = b;
-    }
-  }
-  for (int t = threadIdx.x; t < NV * ND; t += blockDim.x) sBv[t / ND][t % ND] = (R)T->Bv[t / ND][t % ND];
-  __syncthreads();
-  const int ne = prm.ne;
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  int pmap = -1;
+  constexpr int ND = E::ND, NEQ = E::NEQ;
+  int e = blockIdx.x * blockDim.x + threadIdx.x, pmap = -1;
   if (prm.act_cum) {  // batched problems: the i-th element of the active ones
     const int na = *prm.act_n;
     if (e >= prm.act_cum[na]) return;
     e = active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, pmap);
   }
-  if (e >= ne) return;
-  const long long NDa = prm.ndofs;
-  R gamma = (R)prm.gamma, cov = (R)prm.covolume;
-  if (prm.prob) {
-    const int pb = prm.act_cum ? pmap : prm.prob[e];
-    if (!prm.pactive[pb]) return;
-    if constexpr (F32) {
-      gamma = prm.pgamma32 ? prm.pgamma32[pb] : (R)prm.pgamma[pb];
-      cov = prm.pcov32 ? prm.pcov32[pb] : (R)prm.pcov[pb];
-    } else {
-      gamma = (R)prm.pgamma[pb];
-      cov = (R)prm.pcov[pb];
-    }
-  }
-  R el[NEQ][ND];
-  float lo[DS ? NEQ : 1][DS ? ND : 1];
+  if (e >= prm.ne) return;
+  if (prm.prob && !prm.pactive[prm.act_cum ? pmap : prm.prob[e]]) return;
+  R sv[NEQ];
+  shu_indicator<G, P, DS>(prm, u, ulo, e, sv);
+  if (!(sv[NEQ - 1] < R(0.999))) return;
 #pragma unroll
   for (int k = 0; k < NEQ; ++k) {
-    ld_row<ND>(u + k * NDa + (long long)e * ND, el[k]);
-    if constexpr (DS) ld_row<ND>(ulo + k * NDa + (long long)e * ND, lo[k]);
-  }
-  R um[NEQ];
-  float umh[NEQ], uml[NEQ];
-#pragma unroll
-  for (int k = 0; k < NEQ; ++k) {
-    if constexpr (F32) {
-      const float2 m = prm.means32[(long long)k * ne + e];
-      um[k] = m.x;
-      umh[k] = m.x;
-      uml[k] = m.y;
+    R h;
+    float l = 0.0f;
+    if constexpr (std::is_same<R, float>::value) {
+      const float2 m = prm.means32[(long long)k * prm.ne + e];
+      h = m.x;
+      l = m.y;
     } else {
-      const double m = prm.means[(long long)k * ne + e];
-      um[k] = (R)m;
-      umh[k] = (float)m;
-      uml[k] = (float)(m - (double)umh[k]);
-    }
-  }
-  // the indicator's results: FP64, or FP32 for a float state (they only
-  // scale the FP32 multiplier and feed FinDiff's 0.999 test, where no float
-  // lies between 0.999 and its FP32 rounding)
-  using IndT = typename std::conditional<F32, float, double>::type;
-  IndT minValue;
-  IndT elind[NEQ];
-  if (prm.indicator == 0) {
-    minValue = 1.0;
-#pragma unroll
-    for (int k = 0; k < NEQ; ++k) elind[k] = 1.0;
-  } else if (prm.indicator == 1) {
-    minValue = 0.0;
-#pragma unroll
-    for (int k = 0; k < NEQ; ++k) elind[k] = 0.0;
-  } else if (prm.indicator == 3) {
-    R sv[NEQ];
-    shu_indicator<G, P, DS>(prm, u, ulo, e, sv);
-#pragma unroll
-    for (int k = 0; k < NEQ; ++k) elind[k] = (IndT)sv[k];
-    minValue = 1.0;  // FinDiff only: the Multi limiter is rejected with Shu
-  } else {
-    // stencil min / max of the means, started from the element's own mean
-    // clamped to +-1e9: FP64, or for the float path float pairs compared
-    // lexicographically (a normalised pair orders as its value)
-    using MeanT = typename std::conditional<F32, float2, double>::type;
-    MeanT mI[NEQ], MI[NEQ];
-    IndT yMin[NEQ];
-    double umd[NEQ];
-#pragma unroll
-    for (int k = 0; k < NEQ; ++k) {
-      if constexpr (F32) {
-        const float2 own = make_float2(umh[k], uml[k]);
-        const float2 big = make_float2(1e9f, 0.0f), small = make_float2(-1e9f, 0.0f);
-        mI[k] = mean_lt(own, big) ? own : big;
-        MI[k] = mean_lt(small, own) ? own : small;
-      } else {
-        umd[k] = prm.means[(long long)k * ne + e];
-        mI[k] = umd[k] < 1e9 ? umd[k] : 1e9;
-        MI[k] = umd[k] > -1e9 ? umd[k] : -1e9;
-      }
-      yMin[k] = 1e9;
-    }
-    for (int lf = 0; lf < NFPE; ++lf) {
-      const int nb = prm.fnbr[lf * ne + e];
-      if (nb < 0) continue;
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) {
-        const MeanT v = load_mean<F32>(prm, (long long)k * ne + nb);
-        if (mean_lt(v, mI[k])) mI[k] = v;
-        if (mean_lt(MI[k], v)) MI[k] = v;
-      }
-    }
-    // hanging faces: the elements across them are stencil cells
-    // (ElementToElementTable, limiter.cpp:118-123) and the element's own
-    // slave or master faces carry indicator points (limiter.cpp:125-161)
-    unsigned ncfaces = 0;
-    if (prm.ncidx && prm.ncidx[e] >= 0) {
-      const int row = prm.ncidx[e];
-      for (int c = prm.nc_ptr[row]; c < prm.nc_ptr[row + 1]; ++c) {
-        const int f = prm.nc_ent[c] >> 1, side = prm.nc_ent[c] & 1;
-        const int nb = prm.nc_face[f * 4 + (side ? 0 : 2)];
-        ncfaces |= 1u << prm.nc_face[f * 4 + (side ? 3 : 1)];
-#pragma unroll
-        for (int k = 0; k < NEQ; ++k) {
-          const MeanT v = load_mean<F32>(prm, (long long)k * ne + nb);
-          if (mean_lt(v, mI[k])) mI[k] = v;
-          if (mean_lt(MI[k], v)) MI[k] = v;
-        }
-      }
-    }
-    if constexpr (F32) {
-      // double-single: the +-1e-3 switches as float pairs, the numerators of
-      // the ratio (stencil max / min minus the mean) rounded to FP32
-      const float th = 1e-3f, tl = (float)(1e-3 - (double)1e-3f);
-      float nMax[NEQ], nMin[NEQ], yMf[NEQ];
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) {
-        nMax[k] = (MI[k].x - umh[k]) + (MI[k].y - uml[k]);
-        nMin[k] = (mI[k].x - umh[k]) + (mI[k].y - uml[k]);
-        yMf[k] = 1e9f;
-      }
-      for (int lf = 0; lf < NFPE; ++lf) {
-        const int nb = prm.fnbr[lf * ne + e];
-        if (nb < 0 && !((ncfaces >> lf) & 1u)) continue;  // only interior faces carry indicator points
-#pragma unroll
-        for (int q = 0; q < NQL; ++q) {
-#pragma unroll
-          for (int k = 0; k < NEQ; ++k) {
-            // value at the point minus the mean, as a float pair
-            float sh = -umh[k], sl = -uml[k];
-#pragma unroll
-            for (int j = 0; j < ND; ++j) {
-              const float2 bq = sBl[lf][q][j];
-              const float x = (float)el[k][j];
-              const float ph = x * bq.x;
-              float pl = fmaf(x, bq.x, -ph);
-              pl = fmaf(x, bq.y, pl);
-              if constexpr (DS) pl = fmaf(lo[k][j], bq.x, pl);
-              float t, er;
-              two_sum(sh, ph, t, er);
-              er += sl + pl;
-              sh = t + er;
-              sl = er - (sh - t);
-            }
-            const bool above = sh > th || (sh == th && sl > tl);
-            const bool below = sh < -th || (sh == -th && sl < -tl);
-            const float y = above ? nMax[k] / sh : (below ? nMin[k] / sh : 1.0f);
-            if (prm.function == 0) {
-              yMf[k] = fminf(fminf(y, yMf[k]), 1.0f);
-            } else if (prm.function == 1) {
-              const float yc = (y * y + 2.0f * y) / (y * y + y + 2.0f);
-              yMf[k] = fminf(yc, yMf[k]);
-            } else {
-              const float ys = 1.5f;
-              const float yr = y / ys;
-              const float yc = y < 1.0f ? y + (3.0f - 2.0f * ys) * yr * yr + (ys - 2.0f) * yr * yr * yr : 1.0f;
-              yMf[k] = fminf(yc, yMf[k]);
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) yMin[k] = yMf[k];
-    } else {
-      for (int lf = 0; lf < NFPE; ++lf) {
-        const int nb = prm.fnbr[lf * ne + e];
-        if (nb < 0 && !((ncfaces >> lf) & 1u)) continue;  // only interior faces carry indicator points
-#pragma unroll
-        for (int q = 0; q < NQL; ++q) {
-#pragma unroll
-          for (int k = 0; k < NEQ; ++k) {
-            double v = 0.0;
-#pragma unroll
-            for (int j = 0; j < ND; ++j) {
-              v += (double)el[k][j] * sBl[lf][q][j];
-              if constexpr (DS) v += (double)lo[k][j] * sBl[lf][q][j];
-            }
-            const double diff = v - umd[k];
-            double y;
-            if (diff > 1e-3)
-              y = (MI[k] - umd[k]) / diff;
-            else if (diff < -1e-3)
-              y = (mI[k] - umd[k]) / diff;
-            else
-              y = 1.0;
-            if (prm.function == 0) {
-              yMin[k] = y < yMin[k] ? y : yMin[k];
-              yMin[k] = yMin[k] > 1.0 ? 1.0 : yMin[k];
-            } else if (prm.function == 1) {
-              const double yc = (y * y + 2.0 * y) / (y * y + y + 2.0);
-              yMin[k] = yc < yMin[k] ? yc : yMin[k];
-            } else {
-              const double ys = 1.5;
-              const double yr = y / ys;
-              const double yc = y < 1.0 ? y + (3.0 - 2.0 * ys) * yr * yr + (ys - 2.0) * yr * yr * yr : 1.0;
-              yMin[k] = yc < yMin[k] ? yc : yMin[k];
-            }
-          }
-        }
-      }
+      h = prm.means[(long long)k * prm.ne + e];
     }
 #pragma unroll
-    for (int k = 0; k < NEQ; ++k) elind[k] = yMin[k];
-    minValue = yMin[0];
-  }
-  if (prm.limiter == 1) {
-    if constexpr (G != 2) {
-      if (prm.quirks & 2) {
-        // linearize (limiter_multiplier.cpp:101-178): mean + centre gradient
-        // . (x_j - c); a linear state is its own linearisation, so once here
-        // equals the reference's application before every multiplier pass
-#pragma unroll
-        for (int k = 0; k < NEQ; ++k) {
-          double g[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-          for (int d = 0; d < DIM; ++d)
-#pragma unroll
-            for (int j = 0; j < ND; ++j) {
-              double v = (double)el[k][j];
-              if constexpr (DS) v += (double)lo[k][j];
-              g[d] += v * T->dcen[j][d];
-            }
-          const double m = mean_value(prm, (long long)k * ne + e);
-#pragma unroll
-          for (int j = 0; j < ND; ++j) {
-            double v = m;
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) v -= g[d] * (0.5 - T->xlin[j][d]);
-            el[k][j] = (R)v;
-            if constexpr (DS) lo[k][j] = (float)(v - (double)(float)v);
-          }
-        }
-      }
+    for (int j = 0; j < ND; ++j) {
+      const long long i = k * prm.ndofs + (long long)e * ND + j;
+      u[i] = h;
+      if constexpr (DS) ulo[i] = l;
     }
-    const int reps = (prm.quirks & 1) ? 1 : ND;
-#pragma unroll
-    for (int k = 0; k < NEQ; ++k)
-      for (int r = 0; r < reps; ++r)
-#pragma unroll
-        for (int j = 0; j < ND; ++j) {
-          if constexpr (DS) {
-            float h = (float)el[k][j], l = lo[k][j];
-            ds_add(h, l, -umh[k], -uml[k]);
-            float ph, pl;
-            ds_mul_f(h, l, (float)minValue, ph, pl);
-            ds_add(ph, pl, umh[k], uml[k]);
-            el[k][j] = (R)ph;
-            lo[k][j] = pl;
-          } else {
-            el[k][j] = um[k] + (R)minValue * (el[k][j] - um[k]);
-          }
-        }
-    if (prm.last_hope) {
-      for (int v = 0; v < NV; ++v) {
-        R fv[NEQ];
-#pragma unroll
-        for (int k = 0; k < NEQ; ++k) {
-          R s = R(0);
-#pragma unroll
-          for (int j = 0; j < ND; ++j) {
-            s += el[k][j] * sBv[v][j];
-            if constexpr (DS) s += lo[k][j] * sBv[v][j];
-          }
-          fv[k] = s;
-        }
-        if (!state_is_physical<DIM>(fv, gamma, cov)) {
-#pragma unroll
-          for (int k = 0; k < NEQ; ++k)
-#pragma unroll
-            for (int j = 0; j < ND; ++j) {
-              if constexpr (DS) {
-                el[k][j] = (R)umh[k];
-                lo[k][j] = uml[k];
-              } else {
-                el[k][j] = um[k];
-              }
-            }
-        }
-      }
-    }
-  } else {
-    const bool totalInd = elind[NEQ - 1] < IndT(0.999);
-    if (totalInd) {
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k)
-#pragma unroll
-        for (int j = 0; j < ND; ++j) {
-          if constexpr (DS) {
-            el[k][j] = (R)umh[k];
-            lo[k][j] = uml[k];
-          } else {
-            el[k][j] = um[k];
-          }
-        }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < NEQ; ++k) {
-    st_row<ND>(u + k * NDa + (long long)e * ND, el[k]);
-    if constexpr (DS) st_row<ND>(ulo + k * NDa + (long long)e * ND, lo[k]);
   }
 }
 

@@ -6,6 +6,7 @@
 
 #include "rkdg_generic.cuh"
 #include "rkdg_launch.h"
+#include "rkdg_limit.cuh"
 
 namespace rkdg {
 
@@ -33,19 +34,34 @@ cudaError_t launch_rhs_t(int prec, const RhsParams& prm, const void* u, const vo
   return cudaGetLastError();
 }
 
+// Threads per CTA of the limiter: the tuned value, or 128, halved while a
+// small mesh would leave SMs without a CTA.
+inline int limit_block(int tuned, int ne, int lanes) {
+  if (tuned >= 32 && tuned <= kGenericMaxBlock && tuned % 32 == 0) return tuned;
+  int b = 128;
+  while (b > 32 && (long long)ne * lanes < 152LL * b) b >>= 1;
+  return b;
+}
+
+template <int G, int P, typename R, bool DS>
+cudaError_t launch_limit_mode(const LimParams& prm, R* u, float* ulo, cudaStream_t st) {
+  using T = LimTeam<G, P>;
+  if (prm.indicator == 3) {
+    const int blk = std::min(generic_block(prm.block), generic_max_block<R, El<G, P>::NEQ * El<G, P>::ND>());
+    k_limit_shu<G, P, R, DS><<<(prm.ne + blk - 1) / blk, blk, 0, st>>>(prm, u, ulo);
+    return cudaGetLastError();
+  }
+  static_assert(T::template smem_bytes<R, DS>(T::MAX_BLOCK) <= 48 * 1024, "shared memory of the largest CTA");
+  const int blk = limit_block(prm.block, prm.ne, T::L), epb = blk / T::L;
+  k_limit_team<G, P, R, DS><<<(prm.ne + epb - 1) / epb, blk, T::template smem_bytes<R, DS>(blk), st>>>(prm, u, ulo);
+  return cudaGetLastError();
+}
+
 template <int G, int P>
 cudaError_t launch_limit_t(int mode, const LimParams& prm, void* u, float* ulo, cudaStream_t st) {
-  constexpr int NVAL = El<G, P>::NEQ * El<G, P>::ND;
-  const int blk = mode == 0 ? generic_block(prm.block)
-                            : std::min(generic_block(prm.block), generic_max_block<float, NVAL>());
-  const int grid = (prm.ne + blk - 1) / blk;
-  if (mode == 0)
-    k_limit_generic<G, P, double, false><<<grid, blk, 0, st>>>(prm, (double*)u, nullptr);
-  else if (mode == 1)
-    k_limit_generic<G, P, float, false><<<grid, blk, 0, st>>>(prm, (float*)u, nullptr);
-  else
-    k_limit_generic<G, P, float, true><<<grid, blk, 0, st>>>(prm, (float*)u, ulo);
-  return cudaGetLastError();
+  if (mode == 0) return launch_limit_mode<G, P, double, false>(prm, (double*)u, nullptr, st);
+  if (mode == 1) return launch_limit_mode<G, P, float, false>(prm, (float*)u, nullptr, st);
+  return launch_limit_mode<G, P, float, true>(prm, (float*)u, ulo, st);
 }
 
 template <int G, int P>

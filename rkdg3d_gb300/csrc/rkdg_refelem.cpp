@@ -466,6 +466,14 @@ bool build_ref_tables(int geom, int p, RefTables& T, std::vector<FacePoint>* fpt
       B.eval(kRefVert[g][v], phi.data(), nullptr);
       for (int s = 0; s < nd; ++s) T.Bv[v][s] = phi[s];
     }
+    for (int s = 0; s < nd; ++s) {
+      for (int lf = 0; lf < nfpe; ++lf)
+        for (int q = 0; q < f.n; ++q) {
+          const double b = T.Bl[lf][q][s];
+          T.Bl32[s][lf * f.n + q] = {(float)b, (float)(b - (double)(float)b)};
+        }
+      for (int v = 0; v < nv; ++v) T.Bv32[s][v] = (float)T.Bv[v][s];
+    }
   }
   return true;
 }
