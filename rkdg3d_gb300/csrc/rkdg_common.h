@@ -11,6 +11,9 @@
 struct alignas(8) float2 {
   float x, y;
 };
+struct alignas(8) int2 {
+  int x, y;
+};
 #endif
 
 #define RKDG_MAX_ND 27    // hex Q2 = 27 nodes
@@ -126,6 +129,24 @@ struct HexOpsPair {
   HexOps<double> d;
 };
 
+// Operators of the planar (triangle, quadrilateral) kernels, in device memory.
+// Quadrilaterals use the sparse 1D forms: lend (basis at 0
+// and 1), md[i][m] = d1[i][m] / w_i and mb[side][i] = lend[side][i] / w_i.
+// Triangles the dense ones: b[lf][q][j] traces, md[r][m][i] = (M^-1 D_r)[i][m]
+// and mb[lf][q][i] = (M^-1)[i][:] . B[lf][q][:] w_q.
+template <typename R>
+struct PlanarOps {
+  R b[54];
+  R md[72];
+  R mb[54];
+  R lend[8];
+  R wm[16];  // cell-mean weights
+};
+struct PlanarOpsPair {
+  PlanarOps<float> f;
+  PlanarOps<double> d;
+};
+
 // Schedule of one CTA of the shared-face hexahedral team kernel: the CTA's
 // 24 element slots (a compact group of elements in Morton order of their
 // centres) and the rounds in which the slots visit their six faces.  A face
@@ -235,6 +256,15 @@ struct RhsParams {
   // [dim*dim + 1][nd][ne] in the kernel's precision (null: egeo per element)
   const void* ngeo;
   HexOpsPair hops;      // hexahedra (order <= 2): 1D operators
+  // planar elements: the faces in the order of their Elem1, flist[f] =
+  // (Elem1 * 8 + its local face, (Elem2 * 8 + its local face) * 2 + 1 where
+  // Elem2 runs through the points backwards, or -1), and per element face
+  // fref[lf][e] = face * 4 + 2 on the Elem2 side + 1 where its points run
+  // backwards; fslot holds the fluxes [neq][nface * nqf]
+  int nface;
+  const int2* flist;
+  const int* fref;
+  const PlanarOpsPair* pops;
 };
 
 // Hanging (nonconforming) faces of an adapted mesh.  Each slave face is

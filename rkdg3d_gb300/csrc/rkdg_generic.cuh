@@ -1,7 +1,6 @@
-// Generic (dense reference-operator) element kernels: one thread per element.
-//
-// Used for every supported (geometry, order) pair; hexahedra additionally
-// have sum-factorised kernels (rkdg_hex.cuh).  Reference operators live in
+// Generic (dense reference-operator) element kernels, one thread per element,
+// and what the kernels share: float-pair arithmetic, row loads, the wave-speed
+// reductions and the Runge-Kutta epilogue.  Reference operators live in
 // shared memory, converted to the arithmetic type R.  The right-hand side of
 // one element is the reference's FE_Evolution::Mult restricted to that
 // element (fe_evolution.cpp:102-216): every face of the element computes the
@@ -104,8 +103,10 @@ __device__ __forceinline__ void st_row(T* __restrict__ p, const T* v) {
   for (int i = 0; i < N; i += W) st_vec<W>(p + i, v + i);
 }
 
+// The plain read first: thousands of CTAs end on one address, and once a large
+// value is there most of them need no atomic.
 __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* addr, double v) {
-  if (!(v > 0.0)) return;
+  if (!(v > 0.0) || (unsigned long long)__double_as_longlong(v) <= *(volatile unsigned long long*)addr) return;
   atomicMax(addr, (unsigned long long)__double_as_longlong(v));
 }
 
@@ -319,6 +320,8 @@ __device__ __forceinline__ void epilogue(const EpiParams<R>& ep, long long base_
 }
 
 // ---- right-hand side --------------------------------------------------------
+// One thread per element, for the FP32 Q1 quads (the other planar elements run
+// rkdg_planar.cuh): their flux is rounded as it always was, see riemann().
 template <int G, int P, typename R>
 __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>::ND>(),
                                   generic_min_blocks<R, El<G, P>::NEQ * El<G, P>::ND, false>())
@@ -389,129 +392,71 @@ __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>:
     for (int k = 0; k < NEQ; ++k)
 #pragma unroll
       for (int s = 0; s < ND; ++s) acc[k][s] = R(0);
-    // small float elements (Q1 quads, P1 triangles): the element's own rows
-    // are loaded once, with vector loads, for its faces and volume term, and
-    // each neighbour's rows once per face
-    constexpr bool HOIST = std::is_same<R, float>::value && NEQ * ND <= 16;
-    R own[HOIST ? NEQ : 1][HOIST ? ND : 1];
-    if constexpr (HOIST) {
+    // the element's own rows are loaded once, with vector loads, for its faces
+    // and volume term, and each neighbour's rows once per face
+    R own[NEQ][ND];
 #pragma unroll
-      for (int k = 0; k < NEQ; ++k) ld_row<ND>(u + k * NDa + (long long)e * ND, own[k]);
-    }
+    for (int k = 0; k < NEQ; ++k) ld_row<ND>(u + k * NDa + (long long)e * ND, own[k]);
     const R* fg = (const R*)prm.fgeo;
     for (int lf = 0; lf < NFPE; ++lf) {
       const int nb = prm.fnbr[lf * ne + e];
       if (nb == -1) continue;
       const int code = prm.fcode[lf * ne + e];
-      if constexpr (HOIST) {
-        R n[DIM];
+      R n[DIM];
 #pragma unroll
-        for (int c = 0; c < DIM; ++c) n[c] = fg[(long long)(lf * (DIM + 1) + c) * ne + e];
-        const R jac = fg[(long long)(lf * (DIM + 1) + DIM) * ne + e];
-        const int side = (code >> 3) & 1, lfo = code & 7, pid = code >> 4;
-        // sw: this element is side 2 of the face (the trace order of the
-        // Riemann solver), as in the general path below
-        const bool sw = nb >= 0 && side;
-        R nbr[NEQ][ND];
+      for (int c = 0; c < DIM; ++c) n[c] = fg[(long long)(lf * (DIM + 1) + c) * ne + e];
+      const R jac = fg[(long long)(lf * (DIM + 1) + DIM) * ne + e];
+      const int side = (code >> 3) & 1, lfo = code & 7, pid = code >> 4;
+      // sw: this element is side 2 of the face (the trace order of the
+      // Riemann solver), as in the general path below
+      const bool sw = nb >= 0 && side;
+      R nbr[NEQ][ND];
+      if (nb >= 0) {
+#pragma unroll
+        for (int k = 0; k < NEQ; ++k) ld_row<ND>(u + k * NDa + (long long)nb * ND, nbr[k]);
+      }
+      const R sg = side ? R(1) : R(-1);
+      for (int q = 0; q < NQF; ++q) {
+        const int q2 = sPerm[pid][q];
+        R to[NEQ], tn[NEQ], s1[NEQ], s2[NEQ];
+        const R* Bw = sB[lf][sw ? q2 : q];
+#pragma unroll
+        for (int k = 0; k < NEQ; ++k) {
+          R v = R(0);
+#pragma unroll
+          for (int j = 0; j < ND; ++j) v += own[k][j] * Bw[j];
+          to[k] = v;
+        }
         if (nb >= 0) {
-#pragma unroll
-          for (int k = 0; k < NEQ; ++k) ld_row<ND>(u + k * NDa + (long long)nb * ND, nbr[k]);
-        }
-        const R sg = side ? R(1) : R(-1);
-        for (int q = 0; q < NQF; ++q) {
-          const int q2 = sPerm[pid][q];
-          R to[NEQ], tn[NEQ], s1[NEQ], s2[NEQ];
-          const R* Bw = sB[lf][sw ? q2 : q];
+          const R* Bn = sB[lfo][sw ? q : q2];
 #pragma unroll
           for (int k = 0; k < NEQ; ++k) {
             R v = R(0);
 #pragma unroll
-            for (int j = 0; j < ND; ++j) v += own[k][j] * Bw[j];
-            to[k] = v;
+            for (int j = 0; j < ND; ++j) v += nbr[k][j] * Bn[j];
+            tn[k] = v;
           }
-          if (nb >= 0) {
-            const R* Bn = sB[lfo][sw ? q : q2];
-#pragma unroll
-            for (int k = 0; k < NEQ; ++k) {
-              R v = R(0);
-#pragma unroll
-              for (int j = 0; j < ND; ++j) v += nbr[k][j] * Bn[j];
-              tn[k] = v;
-            }
-#pragma unroll
-            for (int k = 0; k < NEQ; ++k) {
-              s1[k] = sw ? tn[k] : to[k];
-              s2[k] = sw ? to[k] : tn[k];
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < NEQ; ++k) s1[k] = to[k];
-            const BCSlot& bc = prm.bc[-2 - nb];
-            right_state<DIM>(bc.type, bc.state, s1, s2, n, gamma, cov, (decltype(gamma))prm.rgas);
-          }
-          R F[NEQ];
-          const R sp = checked_speed(prm, riemann<DIM, R, G == 3 && P == 1>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e, pb);
-          lmax = fmax(lmax, sp);
-          const R* Bo = sB[lf][side ? q2 : q];
-          const R wq = sW[q];
 #pragma unroll
           for (int k = 0; k < NEQ; ++k) {
-            const R t = sg * (F[k] * wq) * jac;
-#pragma unroll
-            for (int j = 0; j < ND; ++j) acc[k][j] += t * Bo[j];
+            s1[k] = sw ? tn[k] : to[k];
+            s2[k] = sw ? to[k] : tn[k];
           }
+        } else {
+#pragma unroll
+          for (int k = 0; k < NEQ; ++k) s1[k] = to[k];
+          const BCSlot& bc = prm.bc[-2 - nb];
+          right_state<DIM>(bc.type, bc.state, s1, s2, n, gamma, cov, (decltype(gamma))prm.rgas);
         }
-      } else {
-        R n[DIM];
+        R F[NEQ];
+        const R sp = checked_speed(prm, riemann<DIM, R, true>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e, pb);
+        lmax = fmax(lmax, sp);
+        const R* Bo = sB[lf][side ? q2 : q];
+        const R wq = sW[q];
 #pragma unroll
-        for (int c = 0; c < DIM; ++c) n[c] = fg[(long long)(lf * (DIM + 1) + c) * ne + e];
-        const R jac = fg[(long long)(lf * (DIM + 1) + DIM) * ne + e];
-        const int side = (code >> 3) & 1, lfo = code & 7, pid = code >> 4;
-        int e1 = e, lf1 = lf, e2 = nb, lf2 = lfo;
-        if (nb >= 0 && side) {
-          e1 = nb;
-          lf1 = lfo;
-          e2 = e;
-          lf2 = lf;
-        }
-        const R sg = side ? R(1) : R(-1);
-        for (int q = 0; q < NQF; ++q) {
-          const int q2 = sPerm[pid][q];
-          R s1[NEQ], s2[NEQ];
-          const R* B1 = sB[lf1][q];
+        for (int k = 0; k < NEQ; ++k) {
+          const R t = sg * (F[k] * wq) * jac;
 #pragma unroll
-          for (int k = 0; k < NEQ; ++k) {
-            const R* uk = u + k * NDa + (long long)e1 * ND;
-            R v = R(0);
-#pragma unroll
-            for (int s = 0; s < ND; ++s) v += uk[s] * B1[s];
-            s1[k] = v;
-          }
-          if (nb >= 0) {
-            const R* B2 = sB[lf2][q2];
-#pragma unroll
-            for (int k = 0; k < NEQ; ++k) {
-              const R* uk = u + k * NDa + (long long)e2 * ND;
-              R v = R(0);
-#pragma unroll
-              for (int s = 0; s < ND; ++s) v += uk[s] * B2[s];
-              s2[k] = v;
-            }
-          } else {
-            const BCSlot& bc = prm.bc[-2 - nb];
-            right_state<DIM>(bc.type, bc.state, s1, s2, n, gamma, cov, (decltype(gamma))prm.rgas);
-          }
-          R F[NEQ];
-          const R sp = checked_speed(prm, riemann<DIM, R, G == 3 && P == 1>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e, pb);
-          lmax = fmax(lmax, sp);
-          const R* Bo = sB[lf][side ? q2 : q];
-          const R wq = sW[q];
-#pragma unroll
-          for (int k = 0; k < NEQ; ++k) {
-            const R t = sg * (F[k] * wq) * jac;
-#pragma unroll
-            for (int s = 0; s < ND; ++s) acc[k][s] += t * Bo[s];
-          }
+          for (int j = 0; j < ND; ++j) acc[k][j] += t * Bo[j];
         }
       }
     }
@@ -534,12 +479,7 @@ __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>:
         }
         R st[NEQ];
 #pragma unroll
-        for (int k = 0; k < NEQ; ++k) {
-          if constexpr (HOIST)
-            st[k] = own[k][m];
-          else
-            st[k] = u[k * NDa + (long long)e * ND + m];
-        }
+        for (int k = 0; k < NEQ; ++k) st[k] = own[k][m];
         R F[NEQ][DIM];
         const R sp = flux_and_speed<DIM>(st, F, gamma, cov);
         lmax = fmax(lmax, sp);

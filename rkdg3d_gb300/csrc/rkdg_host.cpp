@@ -52,6 +52,11 @@ struct rkdg_ctx {
   int gen_block = 0;    // RKDG_TUNE_GENERIC_BLOCK
   double* d_fslot = nullptr;  // face-pass flux slots (split hexahedral variant)
   size_t fslot_n = 0;
+  // planar elements: faces in the order of their Elem1 (see RhsParams)
+  int nface = 0;
+  int2* d_flist = nullptr;
+  int* d_fref = nullptr;
+  rkdg::PlanarOpsPair* d_pops = nullptr;
   HexTeamSched* d_hsched = nullptr;  // per-CTA schedules of the shared-face hexahedral kernel
   int hsched_rounds = 0;
   HexTile* d_htile = nullptr;  // tiles of the face-once hexahedral kernel
@@ -215,6 +220,10 @@ void free_mesh(rkdg_ctx* c) {
   c->adj_n = 0;
   dfree(c->d_fslot);
   c->fslot_n = 0;
+  dfree(c->d_flist);
+  dfree(c->d_fref);
+  dfree(c->d_pops);
+  c->nface = 0;
   dfree(c->d_hsched);
   c->hsched_rounds = 0;
   dfree(c->d_htile);
@@ -324,6 +333,10 @@ RhsParams rhs_params(rkdg_ctx* c, int prec, int faces_only, int slot) {
   P.err = c->d_err;
   P.block = c->gen_block;
   P.fslot = c->d_fslot;
+  P.nface = c->nface;
+  P.flist = c->d_flist;
+  P.fref = c->d_fref;
+  P.pops = c->d_pops;
   P.hsched = c->d_hsched;
   P.htile = c->d_htile;
   P.tcb = c->d_tcb;
@@ -386,18 +399,21 @@ cudaError_t launch_rhs_nc(rkdg_ctx* c, int prec, const RhsParams& P, const void*
 }
 
 // Kernels one right-hand-side launch issues (the split hexahedral variant
-// runs a face pass and an element pass; it is the FP64 Q1 default).
+// runs a face pass and an element pass; it is the FP64 Q1 default; planar
+// elements but the FP32 Q1 quads a face pass and a node pass).
 int rhs_kernels(const rkdg_ctx* c, const RhsParams& P) {
   const bool fp64 = P.fgeo == (const void*)c->d_fgeo64;
+  if (c->geom != RKDG_GEOM_CUBE)
+    return P.faces_only || (c->geom == RKDG_GEOM_SQUARE && c->p == 1 && !fp64) ? 1 : 2;
   const bool split = c->hex_variant == 3 || (c->hex_variant == 0 && c->p == 1 && fp64);
   return (c->geom == RKDG_GEOM_CUBE && split && P.fslot && !P.faces_only) ? 2 : 1;
 }
 
-// Flux slots of the split hexahedral variant: [ne][6][neq][nqf] values of
-// the widest precision.
+// Flux slots, in the widest precision: [ne][6][neq][nqf] for the split
+// hexahedral variant, [neq][nface * nqf] for planar elements.
 int ensure_fslot(rkdg_ctx* c) {
-  if (c->geom != RKDG_GEOM_CUBE) return RKDG_OK;
-  const size_t n = (size_t)c->ne * 6 * c->neq * c->tab.nqf;
+  const size_t n = c->geom == RKDG_GEOM_CUBE ? (size_t)c->ne * 6 * c->neq * c->tab.nqf
+                                             : (size_t)c->nface * c->neq * c->tab.nqf;
   if (c->d_fslot && c->fslot_n == n) return RKDG_OK;
   dfree(c->d_fslot);
   c->fslot_n = 0;
@@ -512,6 +528,56 @@ std::vector<float> tc_volume_operators(const RefTables& T) {
         out[(size_t)(r * 2 + 1) * 1024 + o] = lo;
       }
   return out;
+}
+
+// Faces and operators of the planar kernels (see RhsParams, PlanarOps).
+void planar_tables(const rkdg_ctx* c, std::vector<int2>& flist, std::vector<int>& fref,
+                   rkdg::PlanarOpsPair& ops) {
+  const RefTables& T = c->tab;
+  const int ne = c->ne, nfpe = c->nfpe, nd = c->nd, nqf = T.nqf, n1 = c->p + 1;
+  fref.assign((size_t)nfpe * ne, 0);
+  flist.reserve((size_t)nfpe * ne / 2 + ne / 4 + 16);
+  for (int e = 0; e < ne; ++e)
+    for (int lf = 0; lf < nfpe; ++lf) {
+      const size_t i = (size_t)lf * ne + e;
+      const int e2 = c->h_fnbr[i], code = c->h_fcode[i];
+      if (e2 >= 0 && ((code >> 3) & 1)) continue;  // the Elem2 side
+      const int f = (int)flist.size();
+      int2 r = {e * 8 + lf, -1};
+      fref[i] = f * 4;
+      if (e2 >= 0) {
+        const int lf2 = code & 7, rev = T.perm[code >> 4][0] != 0;
+        r.y = (e2 * 8 + lf2) * 2 + rev;
+        fref[(size_t)lf2 * ne + e2] = f * 4 + 2 + rev;
+      }
+      flist.push_back(r);
+    }
+  rkdg::PlanarOps<double>& D = ops.d;
+  std::memset(&ops, 0, sizeof ops);
+  for (int j = 0; j < nd; ++j) D.wm[j] = T.wmean[j];
+  if (c->geom == RKDG_GEOM_SQUARE) {
+    for (int i = 0; i < n1; ++i) {
+      for (int m = 0; m < n1; ++m) D.md[i * n1 + m] = T.d1[i][m] / T.w1[i];
+      for (int sd = 0; sd < 2; ++sd) {
+        D.lend[sd * n1 + i] = T.lend[sd][i];
+        D.mb[sd * n1 + i] = T.lend[sd][i] / T.w1[i];
+      }
+    }
+  } else {
+    for (int i = 0; i < nd; ++i) {
+      for (int r = 0; r < 2; ++r)
+        for (int m = 0; m < nd; ++m)
+          for (int j = 0; j < nd; ++j) D.md[(r * nd + m) * nd + i] += T.Minv[i][j] * T.D[r][j][m];
+      for (int lf = 0; lf < nfpe; ++lf)
+        for (int q = 0; q < nqf; ++q) {
+          D.b[(lf * nqf + q) * nd + i] = T.B[lf][q][i];
+          for (int j = 0; j < nd; ++j) D.mb[(lf * nqf + q) * nd + i] += T.Minv[i][j] * T.B[lf][q][j] * T.wf[q];
+        }
+    }
+  }
+  const double* src = reinterpret_cast<const double*>(&ops.d);
+  float* dst = reinterpret_cast<float*>(&ops.f);
+  for (size_t i = 0; i < sizeof ops.d / sizeof(double); ++i) dst[i] = (float)src[i];
 }
 
 int check_device_error(rkdg_ctx* c) {
@@ -1399,7 +1465,20 @@ int rkdg_upload_mesh(rkdg_ctx* c, const rkdg_mesh_desc* m) {
   c->has_mesh = true;
   int st = refresh_fnbr(c);
   if (st) return st;
-  if (c->hex_variant == 3 || c->p == 1) {  // the split hexahedral kernels
+  if (dim == 2) {
+    std::vector<int2> flist;
+    std::vector<int> fref;
+    rkdg::PlanarOpsPair ops;
+    planar_tables(c, flist, fref, ops);
+    c->nface = (int)flist.size();
+    CUDA_TRY(c, dalloc(c->d_flist, flist.size()));
+    CUDA_TRY(c, dalloc(c->d_fref, fref.size()));
+    CUDA_TRY(c, dalloc(c->d_pops, 1));
+    CUDA_TRY(c, cudaMemcpy(c->d_flist, flist.data(), flist.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, cudaMemcpy(c->d_fref, fref.data(), fref.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, cudaMemcpy(c->d_pops, &ops, sizeof ops, cudaMemcpyHostToDevice));
+  }
+  if (dim == 2 || c->hex_variant == 3 || c->p == 1) {  // face-pass kernels
     const int st = ensure_fslot(c);
     if (st) return st;
   }

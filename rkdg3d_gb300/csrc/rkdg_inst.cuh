@@ -7,6 +7,7 @@
 #include "rkdg_generic.cuh"
 #include "rkdg_launch.h"
 #include "rkdg_limit.cuh"
+#include "rkdg_planar.cuh"
 
 namespace rkdg {
 
@@ -18,29 +19,51 @@ inline int generic_block(int b) {
   return (b >= 32 && b <= kGenericMaxBlock && b % 32 == 0) ? b : kGenericBlock;
 }
 
-template <int G, int P>
-cudaError_t launch_rhs_t(int prec, const RhsParams& prm, const void* u, const void* ep,
-                         cudaStream_t st) {
-  constexpr int NVAL = El<G, P>::NEQ * El<G, P>::ND;
-  const int blk = prec == 0 ? generic_block(prm.block)
-                            : std::min(generic_block(prm.block), generic_max_block<float, NVAL>());
-  const int grid = (prm.ne + blk - 1) / blk;
-  if (prec == 0)
-    k_rhs_generic<G, P, double><<<grid, blk, 0, st>>>(prm, (const double*)u,
-                                                      *(const EpiParams<double>*)ep);
-  else
-    k_rhs_generic<G, P, float><<<grid, blk, 0, st>>>(prm, (const float*)u,
-                                                     *(const EpiParams<float>*)ep);
+// Threads per CTA of a pass over n work items: at most `most`, halved while a
+// small mesh would leave SMs without a CTA.
+inline int spread_block(long long n, int most) {
+  int b = most;
+  while (b > 32 && n < 152LL * b) b >>= 1;
+  return b;
+}
+
+template <int G, int P, typename R>
+cudaError_t launch_planar(const RhsParams& prm, const R* u, const EpiParams<R>& ep, cudaStream_t st) {
+  if (!prm.flist || !prm.fslot) return cudaErrorInvalidValue;
+  const long long npt = (long long)prm.nface * El<G, P>::NQF;
+  const int blk = spread_block(npt, 128);
+  const unsigned grid = (unsigned)((npt + blk - 1) / blk);
+  if (prm.faces_only) {
+    k_face_planar<G, P, R, true><<<grid, blk, 0, st>>>(prm, u);
+    return cudaGetLastError();
+  }
+  k_face_planar<G, P, R, false><<<grid, blk, 0, st>>>(prm, u);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  using S = Planar<G, P>;
+  k_node_planar<G, P, R><<<(prm.ne + S::EPB - 1) / S::EPB, S::NT, 0, st>>>(prm, u, ep);
   return cudaGetLastError();
 }
 
-// Threads per CTA of the limiter: the tuned value, or 128, halved while a
-// small mesh would leave SMs without a CTA.
+template <int G, int P>
+cudaError_t launch_rhs_t(int prec, const RhsParams& prm, const void* u, const void* ep,
+                         cudaStream_t st) {
+  if (prec == 0) return launch_planar<G, P, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st);
+  if constexpr (G == 3 && P == 1) {
+    constexpr int NVAL = El<G, P>::NEQ * El<G, P>::ND;
+    const int blk = std::min(generic_block(prm.block), generic_max_block<float, NVAL>());
+    k_rhs_generic<G, P, float><<<(prm.ne + blk - 1) / blk, blk, 0, st>>>(prm, (const float*)u,
+                                                                       *(const EpiParams<float>*)ep);
+    return cudaGetLastError();
+  } else {
+    return launch_planar<G, P, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
+  }
+}
+
+// Threads per CTA of the limiter: the tuned value, or by the mesh's size.
 inline int limit_block(int tuned, int ne, int lanes) {
   if (tuned >= 32 && tuned <= kGenericMaxBlock && tuned % 32 == 0) return tuned;
-  int b = 128;
-  while (b > 32 && (long long)ne * lanes < 152LL * b) b >>= 1;
-  return b;
+  return spread_block((long long)ne * lanes, 128);
 }
 
 template <int G, int P, typename R, bool DS>
