@@ -155,8 +155,8 @@ int rkdg_set_tableau(rkdg_ctx* ctx, int s, const double* a, const double* b,
 int rkdg_set_precision(rkdg_ctx* ctx, int precision);
 /* Kernel tuning knobs (no counterpart in the reference; set by hand or by
  * rkdg_autotune).  RKDG_TUNE_HEX_KERNEL: 0 default, 1 warp per element,
- * 2 five-lane team per element, 3 five-lane team face pass (each face once,
- * into per-element flux slots the context allocates) + element pass,
+ * 2 five-lane team per element, 3 face pass (each face once, its moments into
+ * per-face slots) + node pass, the FP64 default,
  * 4 five-lane team over Morton-ordered groups of 24 elements whose faces
  * inside the group are evaluated once (order <= 2 hexahedra; the plain team
  * kernel when the mesh's face graph needs more than 8 rounds), 5 face-once

@@ -11,8 +11,8 @@
 struct alignas(8) float2 {
   float x, y;
 };
-struct alignas(8) int2 {
-  int x, y;
+struct alignas(16) int4 {
+  int x, y, z, w;
 };
 #endif
 
@@ -65,6 +65,7 @@ struct RefTables {
   float2 Bl32[RKDG_MAX_ND][RKDG_MAX_NFPE * RKDG_MAX_NQL];
   float Bv32[RKDG_MAX_ND][RKDG_MAX_NV];
   double wmean[RKDG_MAX_ND];                 // cell-mean weights (sum = 1)
+  float2 wmean32[RKDG_MAX_ND];               // the same as float pairs
   // 1D tables for the sum-factorised tensor kernels
   double l1d[RKDG_MAX_NQF][8];   // 1D basis at 1D face-rule points  [a][j]
   double w1d[8];                 // 1D face-rule weights
@@ -123,6 +124,11 @@ struct HexOps {
   R minv1[9];  // [N1][N1]  1D inverse mass
   R w1[3];     // 1D node weights
   R wf[16];    // face-rule weights
+  // with the 1D inverse mass 1/w_i (the Gauss-Legendre mass matrix is diagonal)
+  R lw[12];    // [NQ1][N1] l1d[a][i] w1d[a] / w_i
+  R md[9];     // [N1][N1]  d1[i][m] / w_i
+  R mb[6];     // [2][N1]   lend[side][i] / w_i
+  R iw[3];     // 1 / w_i
 };
 struct HexOpsPair {
   HexOps<float> f;
@@ -238,7 +244,7 @@ struct RhsParams {
   const int* act_n;
   const int* poff;
   int block;            // threads per CTA of the generic kernels (0: default)
-  void* fslot;          // hexahedral face-pass flux slots [ne][6][neq][nqf] (or null)
+  void* fslot;          // fluxes / moments of the face-pass kernels (see flist below)
   const HexTeamSched* hsched;  // shared-face hexahedral kernel: one entry per CTA (or null)
   const HexTile* htile;        // face-once tiled hexahedral kernel: one entry per CTA (or null)
   int ntile;
@@ -256,14 +262,19 @@ struct RhsParams {
   // [dim*dim + 1][nd][ne] in the kernel's precision (null: egeo per element)
   const void* ngeo;
   HexOpsPair hops;      // hexahedra (order <= 2): 1D operators
-  // planar elements: the faces in the order of their Elem1, flist[f] =
-  // (Elem1 * 8 + its local face, (Elem2 * 8 + its local face) * 2 + 1 where
-  // Elem2 runs through the points backwards, or -1), and per element face
-  // fref[lf][e] = face * 4 + 2 on the Elem2 side + 1 where its points run
-  // backwards; fslot holds the fluxes [neq][nface * nqf]
+  // face-pass kernels (planar elements and hexahedra): the faces in the order
+  // of their Elem1, flist[f] = (Elem1, Elem2 or -1, local face of Elem1 + 8 *
+  // that of Elem2 + 64 * orientation, 0), and each element's faces.
+  // Planar: orientation 1 where Elem2 runs through the points backwards,
+  // fref[lf][e] = face * 4 + 2 on the Elem2 side + 1 where the points run
+  // backwards, fslot the fluxes [neq][nface * nqf].  Hexahedra: orientation =
+  // square_op code from Elem1's to Elem2's tensor indices, fref = face * 2 + 1
+  // on the Elem2 side, fop[lf][e] the code from the element's own indices to
+  // Elem1's, fslot the moments [neq][nface][(p+1)^2].
   int nface;
-  const int2* flist;
+  const int4* flist;
   const int* fref;
+  const unsigned char* fop;
   const PlanarOpsPair* pops;
 };
 

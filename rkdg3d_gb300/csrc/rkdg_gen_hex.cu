@@ -3,6 +3,7 @@
 // (rkdg_hex.cuh) for the FP64 path, plus the generic limiter and cell-mean
 // kernels.
 #include "rkdg_hex.cuh"
+#include "rkdg_hex_faces.cuh"
 #include "rkdg_hex_team.cuh"
 #include "rkdg_inst.cuh"
 
@@ -48,17 +49,6 @@ static cudaError_t launch_hex_team(const RhsParams& prm, const R* u, const EpiPa
   return launch_hex_team_mode<P, R, 0>(prm, u, ep, st);
 }
 
-// Face pass then element pass (each face evaluated once); falls back to the
-// fused kernel without a slot buffer and for the face-only evaluation.
-template <int P, typename R>
-static cudaError_t launch_hex_split(const RhsParams& prm, const R* u, const EpiParams<R>& ep,
-                                    cudaStream_t st) {
-  if (!prm.fslot || prm.faces_only) return launch_hex_team_mode<P, R, 0>(prm, u, ep, st);
-  cudaError_t e = launch_hex_team_mode<P, R, 1>(prm, u, ep, st);
-  if (e != cudaSuccess) return e;
-  return launch_hex_team_mode<P, R, 2>(prm, u, ep, st);
-}
-
 // Shared-face rounds (each face inside a CTA evaluated once); the fused
 // kernel where the context holds no schedule.
 template <int P, typename R>
@@ -68,26 +58,40 @@ static cudaError_t launch_hex_shared(const RhsParams& prm, const R* u, const Epi
   return launch_hex_team_mode<P, R, 3>(prm, u, ep, st);
 }
 
+// Face pass and node pass (rkdg_hex_faces.cuh).
+template <int P, typename R>
+static cudaError_t launch_hex_faces(const RhsParams& prm, const R* u, const EpiParams<R>& ep,
+                                    cudaStream_t st) {
+  using S = HexFaces<P>;
+  if (!prm.flist || !prm.fslot) return cudaErrorInvalidValue;
+  const int grid = (prm.nface + S::FB - 1) / S::FB;
+  if (prm.faces_only) {
+    k_face_hex<P, R, true><<<grid, S::NT, 0, st>>>(prm, u);
+    return cudaGetLastError();
+  }
+  k_face_hex<P, R, false><<<grid, S::NT, 0, st>>>(prm, u);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  k_node_hex<P, R><<<(prm.ne + S::EPB - 1) / S::EPB, S::NTN, 0, st>>>(prm, u, ep);
+  return cudaGetLastError();
+}
+
 // Defaults (64^3 periodic pulse on a GB300, per RK step): FP32 Q2 -- the
 // face-once tiled kernel (2.39 ms against 3.15 for the fused team kernel);
 // FP32 Q1 -- the fused team kernel (1.39 ms against 1.57 split and 1.42
-// shared-face); FP64 Q1 -- face pass + element pass, whose
-// FP64 fluxes are evaluated once per face (21.6 ms against 27.4 shared-face
-// and 36.3 fused; the fused kernel where the context holds no flux slots);
-// FP64 Q2 -- shared-face rounds (55.7 ms against 68.3 fused and 125.5 warp
-// per element).
+// shared-face); FP64 -- face pass and node pass.
 template <>
 cudaError_t launch_rhs_t<5, 1>(int prec, const RhsParams& prm, const void* u, const void* ep,
                                cudaStream_t st) {
   if (prec == 0)
-    return launch_hex_split<1, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st);
+    return launch_hex_faces<1, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st);
   return launch_hex_team<1, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
 }
 template <>
 cudaError_t launch_rhs_t<5, 2>(int prec, const RhsParams& prm, const void* u, const void* ep,
                                cudaStream_t st) {
   if (prec == 0)
-    return launch_hex_shared<2, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st);
+    return launch_hex_faces<2, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st);
   if (prm.htile) return launch_hex_tile(2, 1, prm, u, ep, st);
   return launch_hex_team<2, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
 }
@@ -101,7 +105,7 @@ template cudaError_t launch_means_t<5, 2>(int, int, long long, const RefTables*,
 
 // The hexahedral right-hand-side kernels, selectable for tests and the
 // autotuner (0 = default choice above, 1 = warp-per-element sum
-// factorisation, 2 = team kernel, 3 = face pass + element pass, 4 = team
+// factorisation, 2 = team kernel, 3 = face pass + node pass, 4 = team
 // kernel with shared-face rounds, 5 = face-once tiled kernel where the
 // context holds tiles, 6 = the tiled kernel with the volume contraction on
 // the tensor cores for FP32 Q2, else the default).
@@ -118,10 +122,10 @@ cudaError_t launch_hex_variant(int variant, int p, int prec, const RhsParams& pr
   }
   if (variant == 3) {
     if (p == 1)
-      return prec == 0 ? launch_hex_split<1, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st)
-                       : launch_hex_split<1, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
-    return prec == 0 ? launch_hex_split<2, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st)
-                     : launch_hex_split<2, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
+      return prec == 0 ? launch_hex_faces<1, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st)
+                       : launch_hex_faces<1, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
+    return prec == 0 ? launch_hex_faces<2, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st)
+                     : launch_hex_faces<2, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
   }
   if (variant == 1) {
     if (p == 1)

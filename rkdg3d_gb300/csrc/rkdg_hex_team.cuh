@@ -48,13 +48,11 @@ struct TeamSize {
   // the team-parallel stores (30 lanes) and the warp-parallel flux reads (two
   // teams of 16 points) fall in distinct banks
   // MODE 0 (fused right-hand side) needs both; MODE 3 (shared-face rounds)
-  // both plus the slot's 24 face-geometry values; MODE 1 (face pass) the two
-  // traces only; MODE 2 (element pass) the volume fluxes only.
+  // both plus the slot's 24 face-geometry values.
   static constexpr int XF = 3 * NEQ * NQF, XV = 3 * NEQ * ND;
   template <int MODE>
   __host__ __device__ static constexpr int xch() {
-    return MODE == 1 ? 2 * NEQ * NQF
-                     : (MODE == 2 ? XV : (MODE == 3 ? (XF + 24 > XV ? XF + 24 : XV) : (XF > XV ? XF : XV)));
+    return MODE == 3 ? (XF + 24 > XV ? XF + 24 : XV) : (XF > XV ? XF : XV);
   }
   // row stride: a multiple of 32 words with room for the offsets (team t + 1
   // may start up to 11 words earlier within its row than team t)
@@ -77,7 +75,7 @@ struct TeamSize {
   // resident CTAs per SM the register allocation is bounded for
   template <typename R, int MODE>
   __host__ __device__ static constexpr int min_ctas() {
-    return sizeof(R) == 4 ? (MODE == 1 ? 5 : 4) : 2;
+    return sizeof(R) == 4 ? 4 : 2;
   }
 };
 
@@ -431,11 +429,8 @@ __device__ __forceinline__ void team_traces(const int LF, const R* __restrict__ 
 // elements, spread over the 32 lanes (point pt of the warp = team pt / NQF,
 // point pt % NQF); arguments in Elem1, Elem2 order with the Elem1-outward
 // normal (face_integrator.cpp:11-276), boundary faces through the boundary
-// condition's right state.  MODE 0 writes sign * w_q * |J_f| * Fhat to the
-// team's Fh[q*NEQ + k] in its own tensor order.  MODE 1 (face pass) handles
-// only the faces the element owns (Elem1 of an interior face, or a boundary
-// face) and writes the value into the flux slots of both elements
-// (prm.fslot[element][local face][k][tensor point]) with each side's sign.
+// condition's right state.  Writes sign * w_q * |J_f| * Fhat to the team's
+// Fh[q*NEQ + k] in its own tensor order.
 template <int P, typename R, int MODE>
 __device__ __forceinline__ void warp_fluxes(const int LF, const RhsParams& prm, int lane, int wel0,
                                             int nel, R* wx, const R* wf,
@@ -454,7 +449,6 @@ __device__ __forceinline__ void warp_fluxes(const int LF, const RhsParams& prm, 
     if (nb == -1) continue;
     const int code = sfcd[el][LF];
     const int side = (code >> 3) & 1, lfo = code & 7, pid = code >> 4;
-    if (MODE == 1 && side) continue;  // the face's Elem1 evaluates it
     R* To = wx + t * XSTR + S::xoff(t);
     const R* Tn = To + NEQ * NQF;
     R* Fh = To + 2 * NEQ * NQF;
@@ -464,7 +458,7 @@ __device__ __forceinline__ void warp_fluxes(const int LF, const RhsParams& prm, 
     for (int c = 0; c < 3; ++c) n[c] = __ldg(fg + (long long)c * prm.ne);
     const R jac = __ldg(fg + 3LL * prm.ne);
     R s1[NEQ], s2[NEQ];
-    int own = fab[LF][q], other = 0;
+    int own = fab[LF][q];
     if (nb >= 0) {
       const int q2 = perm[pid][q];
       const int a1 = side ? fab[lfo][q] : fab[LF][q];
@@ -477,7 +471,6 @@ __device__ __forceinline__ void warp_fluxes(const int LF, const RhsParams& prm, 
         s2[kk] = T2[a2 * NEQ + kk];
       }
       if (side) own = a2;
-      other = a2;
     } else {
 #pragma unroll
       for (int kk = 0; kk < NEQ; ++kk) s1[kk] = To[own * NEQ + kk];
@@ -487,22 +480,9 @@ __device__ __forceinline__ void warp_fluxes(const int LF, const RhsParams& prm, 
     R F[NEQ];
     const R sp = checked_speed(prm, riemann<3>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e0 + el);
     lmax = fmax(lmax, sp);
-    if constexpr (MODE == 1) {
-      R* fs = (R*)prm.fslot;
-      const R w = wf[q] * jac;
-      R* so = fs + ((long long)(e0 + el) * 6 + LF) * (NEQ * NQF) + own;
+    const R w = (side ? R(1) : R(-1)) * wf[q] * jac;
 #pragma unroll
-      for (int kk = 0; kk < NEQ; ++kk) so[kk * NQF] = -w * F[kk];
-      if (nb >= 0) {
-        R* sn = fs + ((long long)nb * 6 + lfo) * (NEQ * NQF) + other;
-#pragma unroll
-        for (int kk = 0; kk < NEQ; ++kk) sn[kk * NQF] = w * F[kk];
-      }
-    } else {
-      const R w = (side ? R(1) : R(-1)) * wf[q] * jac;
-#pragma unroll
-      for (int kk = 0; kk < NEQ; ++kk) Fh[own * NEQ + kk] = w * F[kk];
-    }
+    for (int kk = 0; kk < NEQ; ++kk) Fh[own * NEQ + kk] = w * F[kk];
   }
 }
 
@@ -645,11 +625,8 @@ __device__ __forceinline__ void shared_rounds(const RhsParams& prm, const R* __r
 }
 
 // MODE 0: the whole right-hand side of the CTA's elements (every face
-// evaluated by both its elements).  MODE 1 + MODE 2 (two launches): a face pass
-// that evaluates each face once into per-element flux slots, then an element
-// pass that lifts the six slots and adds the volume term, inverse mass and
-// Runge-Kutta epilogue.  MODE 3: the CTA's slots hold the elements its
-// schedule names, and faces inside the CTA are evaluated once
+// evaluated by both its elements).  MODE 3: the CTA's slots hold the elements
+// its schedule lists, and the faces are visited in the schedule's rounds
 // (shared_rounds); volume term and epilogue as MODE 0.
 template <int P, typename R, int MODE>
 __global__ void __launch_bounds__(128, TeamSize<P>::template min_ctas<R, MODE>())
@@ -732,37 +709,20 @@ __global__ void __launch_bounds__(128, TeamSize<P>::template min_ctas<R, MODE>()
     }
     shared_rounds<P, R>(prm, u, NDa, *sS, sX, sRowOff, xch, su, el, act, k, tL1, tLend, tWf, sPerm,
                         sFab, sFnb, sFcd, gamma, cov, lmax, acc);
-  } else if constexpr (MODE != 2) {
+  } else {
     // the warp steps through the six faces together: traces per team, the
-    // numerical fluxes over all 32 lanes, the lifting per team again (MODE 0)
+    // numerical fluxes over all 32 lanes, the lifting per team again
 #pragma unroll 1
     for (int lf = 0; lf < 6; ++lf) {
       const int nb = act ? sFnb[el][lf] : -1;
-      const bool mine = nb != -1 && (MODE == 0 || ((sFcd[el][lf] >> 3) & 1) == 0);
-      if (MODE == 1 && !__any_sync(0xffffffffu, mine)) continue;
-      if (mine)
+      if (nb != -1)
         team_traces<P, R>(lf, u, NDa, k, su, xch, tL1, tLend, nb, sFcd[el][lf], sU, e0, nel);
       __syncwarp();
       warp_fluxes<P, R, MODE>(lf, prm, lane, wel0, nel, wx, tWf, sPerm, sFab, sFnb, sFcd, e0, gamma,
                               cov, lmax);
       __syncwarp();
-      if (MODE == 0 && nb != -1 && !prm.faces_only)
+      if (nb != -1 && !prm.faces_only)
         team_lift_axis<P, NEQ>(lf, xch + 2 * NEQ * NQF + k, tL1, tLend, acc);
-    }
-    if constexpr (MODE == 1) {
-      block_max_commit<R>(lmax, prm.mcs);
-      return;
-    }
-  } else if (act) {
-    // lift the six flux slots the face pass wrote for this element
-    const R* fs = (const R*)prm.fslot + (long long)e * 6 * (NEQ * NQF) + k * NQF;
-#pragma unroll 1
-    for (int lf = 0; lf < 6; ++lf) {
-      if (sFnb[el][lf] == -1) continue;
-      R fv[NQF];
-#pragma unroll
-      for (int q = 0; q < NQF; ++q) fv[q] = __ldg(fs + lf * (NEQ * NQF) + q);
-      team_lift_axis<P, 1>(lf, fv, tL1, tLend, acc);
     }
   }
   // neighbours inside the tile were read from the staged DOFs, which the

@@ -50,12 +50,13 @@ struct rkdg_ctx {
   int precision = RKDG_FP64;
   int hex_variant = 0;  // RKDG_TUNE_HEX_KERNEL
   int gen_block = 0;    // RKDG_TUNE_GENERIC_BLOCK
-  double* d_fslot = nullptr;  // face-pass flux slots (split hexahedral variant)
-  size_t fslot_n = 0;
-  // planar elements: faces in the order of their Elem1 (see RhsParams)
+  // faces in the order of their Elem1 (see RhsParams)
   int nface = 0;
-  int2* d_flist = nullptr;
+  int4* d_flist = nullptr;
   int* d_fref = nullptr;
+  unsigned char* d_fop = nullptr;
+  double* d_fcoef = nullptr;  // fluxes / moments of the face-pass kernels
+  size_t fcoef_n = 0;
   rkdg::PlanarOpsPair* d_pops = nullptr;
   HexTeamSched* d_hsched = nullptr;  // per-CTA schedules of the shared-face hexahedral kernel
   int hsched_rounds = 0;
@@ -218,10 +219,11 @@ void free_mesh(rkdg_ctx* c) {
   dfree(c->d_pmcs);
   dfree(c->d_adj);
   c->adj_n = 0;
-  dfree(c->d_fslot);
-  c->fslot_n = 0;
   dfree(c->d_flist);
   dfree(c->d_fref);
+  dfree(c->d_fop);
+  dfree(c->d_fcoef);
+  c->fcoef_n = 0;
   dfree(c->d_pops);
   c->nface = 0;
   dfree(c->d_hsched);
@@ -332,10 +334,11 @@ RhsParams rhs_params(rkdg_ctx* c, int prec, int faces_only, int slot) {
   P.mcs = c->d_mcs + slot;
   P.err = c->d_err;
   P.block = c->gen_block;
-  P.fslot = c->d_fslot;
+  P.fslot = c->d_fcoef;
   P.nface = c->nface;
   P.flist = c->d_flist;
   P.fref = c->d_fref;
+  P.fop = c->d_fop;
   P.pops = c->d_pops;
   P.hsched = c->d_hsched;
   P.htile = c->d_htile;
@@ -361,6 +364,12 @@ RhsParams rhs_params(rkdg_ctx* c, int prec, int faces_only, int slot) {
         H.w1[j] = T.w1[j];
       }
       for (int q = 0; q < nq1 * nq1; ++q) H.wf[q] = T.wf[q];
+      for (int i = 0; i < n1; ++i) {
+        H.iw[i] = 1.0 / T.w1[i];
+        for (int a = 0; a < nq1; ++a) H.lw[a * n1 + i] = T.l1d[a][i] * T.w1d[a] / T.w1[i];
+        for (int m = 0; m < n1; ++m) H.md[i * n1 + m] = T.d1[i][m] / T.w1[i];
+        for (int sd = 0; sd < 2; ++sd) H.mb[sd * n1 + i] = T.lend[sd][i] / T.w1[i];
+      }
     };
     fill(P.hops.f);
     fill(P.hops.d);
@@ -398,27 +407,26 @@ cudaError_t launch_rhs_nc(rkdg_ctx* c, int prec, const RhsParams& P, const void*
   return rkdg::launch_rhs_v(c->hex_variant, c->geom, c->p, prec, P, in, ep, c->stream);
 }
 
-// Kernels one right-hand-side launch issues (the split hexahedral variant
-// runs a face pass and an element pass; it is the FP64 Q1 default; planar
-// elements but the FP32 Q1 quads a face pass and a node pass).
+// Kernels one right-hand-side launch issues: a face pass and a node pass
+// (the face pass alone for the wave speed), one kernel on FP32 Q1 quads and for
+// FP32 and the selected variants of hexahedra but that of the two passes.
 int rhs_kernels(const rkdg_ctx* c, const RhsParams& P) {
   const bool fp64 = P.fgeo == (const void*)c->d_fgeo64;
-  if (c->geom != RKDG_GEOM_CUBE)
-    return P.faces_only || (c->geom == RKDG_GEOM_SQUARE && c->p == 1 && !fp64) ? 1 : 2;
-  const bool split = c->hex_variant == 3 || (c->hex_variant == 0 && c->p == 1 && fp64);
-  return (c->geom == RKDG_GEOM_CUBE && split && P.fslot && !P.faces_only) ? 2 : 1;
+  if (P.faces_only) return 1;
+  if (c->geom == RKDG_GEOM_CUBE) return c->hex_variant == 3 || (c->hex_variant == 0 && fp64) ? 2 : 1;
+  return c->geom == RKDG_GEOM_SQUARE && c->p == 1 && !fp64 ? 1 : 2;
 }
 
-// Flux slots, in the widest precision: [ne][6][neq][nqf] for the split
-// hexahedral variant, [neq][nface * nqf] for planar elements.
-int ensure_fslot(rkdg_ctx* c) {
-  const size_t n = c->geom == RKDG_GEOM_CUBE ? (size_t)c->ne * 6 * c->neq * c->tab.nqf
-                                             : (size_t)c->nface * c->neq * c->tab.nqf;
-  if (c->d_fslot && c->fslot_n == n) return RKDG_OK;
-  dfree(c->d_fslot);
-  c->fslot_n = 0;
-  CUDA_TRY(c, dalloc(c->d_fslot, n));
-  c->fslot_n = n;
+// Fluxes (planar) or moments (hexahedra) of the face-pass kernels, in the
+// widest precision.
+int ensure_fcoef(rkdg_ctx* c) {
+  const int per = c->geom == RKDG_GEOM_CUBE ? (c->p + 1) * (c->p + 1) : c->tab.nqf;
+  const size_t n = (size_t)c->nface * c->neq * per;
+  if (c->d_fcoef && c->fcoef_n == n) return RKDG_OK;
+  dfree(c->d_fcoef);
+  c->fcoef_n = 0;
+  CUDA_TRY(c, dalloc(c->d_fcoef, n));
+  c->fcoef_n = n;
   return RKDG_OK;
 }
 
@@ -530,28 +538,75 @@ std::vector<float> tc_volume_operators(const RefTables& T) {
   return out;
 }
 
-// Faces and operators of the planar kernels (see RhsParams, PlanarOps).
-void planar_tables(const rkdg_ctx* c, std::vector<int2>& flist, std::vector<int>& fref,
-                   rkdg::PlanarOpsPair& ops) {
+// square_op of rkdg_hex_faces.cuh on the host.
+int square_op_host(int op, int i, int j, int n) {
+  const int a = (op & 1) ? j : i, b = (op & 1) ? i : j;
+  return ((op & 2) ? n - 1 - a : a) + n * ((op & 4) ? n - 1 - b : b);
+}
+
+// Faces of the face-pass kernels in the order of their Elem1 (see RhsParams).
+bool face_tables(const rkdg_ctx* c, std::vector<int4>& flist, std::vector<int>& fref,
+                 std::vector<unsigned char>& fop) {
   const RefTables& T = c->tab;
-  const int ne = c->ne, nfpe = c->nfpe, nd = c->nd, nqf = T.nqf, n1 = c->p + 1;
+  const int ne = c->ne, nfpe = c->nfpe;
+  const bool hex = c->geom == RKDG_GEOM_CUBE;
   fref.assign((size_t)nfpe * ne, 0);
+  if (hex) fop.assign((size_t)nfpe * ne, 0);
   flist.reserve((size_t)nfpe * ne / 2 + ne / 4 + 16);
+  // orientation codes per (lf1, lf2, permutation), filled when first met
+  const int n = T.nq1;
+  std::vector<signed char> code(hex ? 36 * RKDG_HEX_MAX_PERM : 0, -1);
+  signed char inverse[8];
+  for (int o = 0; hex && o < 8; ++o)
+    for (int v = 0; v < 8; ++v) {
+      bool ok = true;
+      for (int t = 0; t < n * n && ok; ++t) {
+        const int w = square_op_host(o, t % n, t / n, n);
+        ok = square_op_host(v, w % n, w / n, n) == t;
+      }
+      if (ok) inverse[o] = (signed char)v;
+    }
   for (int e = 0; e < ne; ++e)
     for (int lf = 0; lf < nfpe; ++lf) {
       const size_t i = (size_t)lf * ne + e;
-      const int e2 = c->h_fnbr[i], code = c->h_fcode[i];
-      if (e2 >= 0 && ((code >> 3) & 1)) continue;  // the Elem2 side
+      const int e2 = c->h_fnbr[i], fc = c->h_fcode[i];
+      if (e2 >= 0 && ((fc >> 3) & 1)) continue;  // the Elem2 side
       const int f = (int)flist.size();
-      int2 r = {e * 8 + lf, -1};
-      fref[i] = f * 4;
+      int4 r = {e, -1, lf, 0};
+      fref[i] = f * (hex ? 2 : 4);
       if (e2 >= 0) {
-        const int lf2 = code & 7, rev = T.perm[code >> 4][0] != 0;
-        r.y = (e2 * 8 + lf2) * 2 + rev;
-        fref[(size_t)lf2 * ne + e2] = f * 4 + 2 + rev;
+        const int lf2 = fc & 7, pid = fc >> 4;
+        const size_t i2 = (size_t)lf2 * ne + e2;
+        int op = T.perm[pid][0] != 0;
+        if (hex) {
+          signed char& o = code[(lf * 6 + lf2) * RKDG_HEX_MAX_PERM + pid];
+          for (int v = 0; v < 8 && o < 0; ++v) {
+            bool ok = true;
+            for (int q = 0; q < T.nqf && ok; ++q) {
+              const int t1 = T.fab[lf][q];
+              ok = square_op_host(v, t1 % n, t1 / n, n) == T.fab[lf2][T.perm[pid][q]];
+            }
+            if (ok) o = (signed char)v;
+          }
+          if (o < 0) return false;
+          op = o;
+          fref[i2] = f * 2 + 1;
+          fop[i2] = (unsigned char)inverse[op];
+        } else {
+          fref[i2] = f * 4 + 2 + op;
+        }
+        r.y = e2;
+        r.z = lf + 8 * lf2 + 64 * op;
       }
       flist.push_back(r);
     }
+  return true;
+}
+
+// Operators of the planar kernels (see PlanarOps).
+void planar_tables(const rkdg_ctx* c, rkdg::PlanarOpsPair& ops) {
+  const RefTables& T = c->tab;
+  const int nfpe = c->nfpe, nd = c->nd, nqf = T.nqf, n1 = c->p + 1;
   rkdg::PlanarOps<double>& D = ops.d;
   std::memset(&ops, 0, sizeof ops);
   for (int j = 0; j < nd; ++j) D.wm[j] = T.wmean[j];
@@ -1004,10 +1059,6 @@ int rkdg_set_solver_quirks(rkdg_ctx* c, int flags) {
 int rkdg_set_tuning(rkdg_ctx* c, int key, int value) {
   if (!c) return RKDG_ERR_INVALID;
   if (key == RKDG_TUNE_HEX_KERNEL && value >= 0 && value <= 6) {
-    if (value == 3 && c->has_mesh) {
-      const int st = ensure_fslot(c);
-      if (st) return st;
-    }
     c->hex_variant = value;
     return RKDG_OK;
   }
@@ -1465,23 +1516,30 @@ int rkdg_upload_mesh(rkdg_ctx* c, const rkdg_mesh_desc* m) {
   c->has_mesh = true;
   int st = refresh_fnbr(c);
   if (st) return st;
-  if (dim == 2) {
-    std::vector<int2> flist;
+  {
+    std::vector<int4> flist;
     std::vector<int> fref;
-    rkdg::PlanarOpsPair ops;
-    planar_tables(c, flist, fref, ops);
+    std::vector<unsigned char> fop;
+    if (!face_tables(c, flist, fref, fop))
+      return fail(c, RKDG_ERR_INVALID, "face points of two hexahedra do not match");
     c->nface = (int)flist.size();
     CUDA_TRY(c, dalloc(c->d_flist, flist.size()));
     CUDA_TRY(c, dalloc(c->d_fref, fref.size()));
-    CUDA_TRY(c, dalloc(c->d_pops, 1));
-    CUDA_TRY(c, cudaMemcpy(c->d_flist, flist.data(), flist.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, cudaMemcpy(c->d_flist, flist.data(), flist.size() * sizeof(int4), cudaMemcpyHostToDevice));
     CUDA_TRY(c, cudaMemcpy(c->d_fref, fref.data(), fref.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CUDA_TRY(c, cudaMemcpy(c->d_pops, &ops, sizeof ops, cudaMemcpyHostToDevice));
+    if (!fop.empty()) {
+      CUDA_TRY(c, dalloc(c->d_fop, fop.size()));
+      CUDA_TRY(c, cudaMemcpy(c->d_fop, fop.data(), fop.size(), cudaMemcpyHostToDevice));
+    }
+    if (dim == 2) {
+      rkdg::PlanarOpsPair ops;
+      planar_tables(c, ops);
+      CUDA_TRY(c, dalloc(c->d_pops, 1));
+      CUDA_TRY(c, cudaMemcpy(c->d_pops, &ops, sizeof ops, cudaMemcpyHostToDevice));
+    }
   }
-  if (dim == 2 || c->hex_variant == 3 || c->p == 1) {  // face-pass kernels
-    const int st = ensure_fslot(c);
-    if (st) return st;
-  }
+  st = ensure_fcoef(c);
+  if (st) return st;
   if ((c->quirks & RKDG_LIMITER_LINEARIZE) && c->lim == RKDG_LIM_MULTI &&
       c->geom != RKDG_GEOM_TRIANGLE && !c->tab.lin_ok)
     return fail(c, RKDG_ERR_UNSUPPORTED,
@@ -2100,7 +2158,7 @@ long long rkdg_kernel_launches(rkdg_ctx* c) { return c ? c->launches : -1; }
 // limiter when one is active) on the caller's state, times them with CUDA
 // events on the context's stream and keeps the fastest.  Candidates: the
 // hexahedral kernel (warp per element with 8 elements per CTA, five-lane team
-// with 24, or the team face pass + element pass) or, on triangles and quads,
+// with 24, face pass + node pass, tiles, ...) or, on triangles and quads,
 // 64 / 128 / 256 elements per CTA.
 int rkdg_autotune(rkdg_ctx* c, const double* x, int* hex_kernel, int* generic_block,
                   int* limiter_block) {
@@ -2152,7 +2210,6 @@ int rkdg_autotune(rkdg_ctx* c, const double* x, int* hex_kernel, int* generic_bl
     return read_mcs(c, 0, nullptr);  // reports a non-physical input state
   };
   if (c->geom == RKDG_GEOM_CUBE) {
-    if ((st = ensure_fslot(c))) return st;
     int best = 0;
     float tbest = 0.0f;
     for (int v = 1; v <= 6; ++v) {
@@ -2164,10 +2221,6 @@ int rkdg_autotune(rkdg_ctx* c, const double* x, int* hex_kernel, int* generic_bl
       if (best == 0 || ms < tbest) best = v, tbest = ms;
     }
     c->hex_variant = best;
-    if (best != 3) {
-      dfree(c->d_fslot);
-      c->fslot_n = 0;
-    }
   } else {
     int best = 0;
     float tbest = 0.0f;

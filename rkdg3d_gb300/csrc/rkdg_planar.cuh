@@ -78,12 +78,12 @@ __global__ void __launch_bounds__(128)
   R lmax = R(0);
   int pb = -1;
   bool live = f < prm.nface;
-  int2 face = make_int2(0, 0);
+  int4 face = make_int4(0, -1, 0, 0);
   int e1 = 0;
   R gamma = (R)prm.gamma, cov = (R)prm.covolume;
   if (live) {
     face = prm.flist[f];
-    e1 = face.x >> 3;
+    e1 = face.x;
     if (prm.prob) {
       pb = prm.prob[e1];
       live = prm.pactive[pb] != 0;
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(128)
     }
   }
   if (live) {
-    const int lf1 = face.x & 7;
+    const int lf1 = face.z & 7;
     const R* fg = (const R*)prm.fgeo;
     R n[DIM];
 #pragma unroll
@@ -134,8 +134,7 @@ __global__ void __launch_bounds__(128)
     trace(e1, lf1, q, s1);
     bool none = false;
     if (face.y >= 0) {
-      const int e2 = face.y >> 4, lf2 = (face.y >> 1) & 7;
-      trace(e2, lf2, (face.y & 1) ? NQF - 1 - q : q, s2);
+      trace(face.y, (face.z >> 3) & 7, (face.z >> 6) ? NQF - 1 - q : q, s2);
     } else {
       const int nb = prm.fnbr[lf1 * ne + e1];
       none = nb == -1;  // no integrator
@@ -175,9 +174,12 @@ __device__ __forceinline__ void epi_node(const EpiParams<R>& ep, long long idx, 
     return;
   }
   if constexpr (std::is_same<R, double>::value) {
-    double v = ep.base ? ep.base[idx] : 0.0;
-    for (int j = 0; j < ep.nprev; ++j) v += (ep.cprev[j] * dts) * ep.kprev[j][idx];
-    v += (ep.ccur * dts) * y;
+    // the increment first: one rounding at the state's size
+    double v = (ep.ccur * dts) * y;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (j < ep.nprev) v += (ep.cprev[j] * dts) * ep.kprev[j][idx];
+    if (ep.base) v += ep.base[idx];
     if (ep.kout) ep.kout[idx] = y;
     if (ep.out64) ep.out64[idx] = v;
     if (ep.out32) ep.out32[idx] = (float)v;
