@@ -24,7 +24,7 @@ bool adjoint_supported(int geom, int p) {
 template <int G, int P>
 static cudaError_t minv_t(int ne, long long ndofs, const RefTables* tab, const double* egeo,
                           const double* kb, double* r, cudaStream_t st) {
-  k_minv_apply<G, P><<<(ne + 127) / 128, 128, 0, st>>>(ne, ndofs, tab, egeo, kb, r);
+  k_minv_apply<G, P><<<(unsigned)((ndofs + 127) / 128), 128, 0, st>>>(ne, ndofs, tab, egeo, kb, r);
   return cudaGetLastError();
 }
 cudaError_t launch_minv_apply(int geom, int p, int ne, long long ndofs, const RefTables* tab,
@@ -35,14 +35,21 @@ cudaError_t launch_minv_apply(int geom, int p, int ne, long long ndofs, const Re
 }
 
 template <int G, int P>
-static cudaError_t rhs_vjp_t(const RhsParams& prm, const double* u, const double* r, double* ub,
-                             cudaStream_t st) {
-  k_rhs_vjp<G, P><<<(prm.ne + 63) / 64, 64, 0, st>>>(prm, u, r, ub);
+static cudaError_t rhs_vjp_t(const RhsParams& prm, const double* u, const double* r, double* gb,
+                             int boundary, double* ub, cudaStream_t st) {
+  using S = VjpSize<G, P>;
+  const long long npt = (long long)prm.nface * El<G, P>::NQF;
+  int blk = 128;  // smaller CTAs while a small mesh would leave SMs without one
+  while (blk > 32 && npt < 152LL * blk) blk >>= 1;
+  k_face_vjp<G, P><<<(unsigned)((npt + blk - 1) / blk), blk, 0, st>>>(prm, u, r, gb);
+  if (boundary) k_bface_vjp<G, P><<<(unsigned)((npt + 63) / 64), 64, 0, st>>>(prm, u, r, gb);
+  k_node_vjp<G, P><<<(prm.ne + S::EPB - 1) / S::EPB, S::NT, 0, st>>>(prm, u, r, gb, ub);
   return cudaGetLastError();
 }
 cudaError_t launch_rhs_vjp(int geom, int p, const RhsParams& prm, const double* u, const double* r,
-                           double* ub, cudaStream_t st) {
-#define CALL_RV(G, P) rhs_vjp_t<G, P>(prm, u, r, ub, st)
+                           double* gb, int boundary, double* ub, cudaStream_t st) {
+  if (!prm.flist || !gb) return cudaErrorInvalidValue;
+#define CALL_RV(G, P) rhs_vjp_t<G, P>(prm, u, r, gb, boundary, ub, st)
   RKDG_ADJ_DISPATCH(CALL_RV)
 #undef CALL_RV
 }

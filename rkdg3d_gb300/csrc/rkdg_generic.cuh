@@ -114,19 +114,18 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* addr, doub
 // block (the MPI_Allreduce(MAX) of main.cpp:543 on one device).
 template <typename R>
 __device__ __forceinline__ void block_max_commit(R v, unsigned long long* dst) {
-  double vd = (double)v;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) vd = fmax(vd, __shfl_xor_sync(0xffffffffu, vd, o));
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  __shared__ double redd[32];
-  if (lane == 0) redd[w] = vd;
+  __shared__ R redd[32];
+  if (lane == 0) redd[w] = v;
   __syncthreads();
   if (w == 0) {
     const int nw = (blockDim.x + 31) >> 5;
-    double x = lane < nw ? redd[lane] : 0.0;
+    R x = lane < nw ? redd[lane] : R(0);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
-    if (lane == 0) atomic_max_nonneg(dst, x);
+    if (lane == 0) atomic_max_nonneg(dst, (double)x);
   }
 }
 

@@ -35,7 +35,7 @@ struct HexFaces {
   static constexpr int N1 = P + 1, NQ1 = P + 2, ND = N1 * N1 * N1, NQF = NQ1 * NQ1, NF2 = N1 * N1,
                        NEQ = 5;
   static constexpr int FB = P == 2 ? 16 : 24, NT = 256;  // faces and threads of a face-pass CTA
-  static constexpr int QS = NQF | 1;                     // odd row stride in shared memory
+  static constexpr int QS = NQF | 1, NDS = ND | 1;       // odd row strides in shared memory
   // node pass: elements and threads (whole warps) per CTA
   static constexpr int EPB = P == 2 ? 7 : 24, NTN = 192;
   static_assert(FB * 2 * NEQ <= NT && FB * NQF <= NT && EPB * ND <= NTN && NTN % 32 == 0, "one round each");
@@ -54,32 +54,52 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
   using S = HexFaces<P>;
   constexpr int N1 = S::N1, NQ1 = S::NQ1, NQF = S::NQF, NF2 = S::NF2, NEQ = S::NEQ, FB = S::FB,
                 ND = S::ND, QS = S::QS;
+  // float: the faces' elements are staged coalesced (a thread per value); with
+  // FP64 the loads hide behind the FP64 pipe and the threads read their rows
+  constexpr bool STAGE = std::is_same<R, float>::value;
+  constexpr int NROW = FB * 2 * NEQ;  // (variable, side, face)
   __shared__ R sT[2][NEQ][FB][QS];
+  __shared__ R sU[STAGE ? NROW * S::NDS : 1];
+  __shared__ int4 sF[FB];
   const HexOps<R>& H = hex_ops<R>(prm.hops);
   const int tid = threadIdx.x, f0 = blockIdx.x * FB, nface = prm.nface, ne = prm.ne;
   const long long NDa = prm.ndofs;
-  // traces, in each side's own tensor order a + NQ1 b
-  if (tid < FB * 2 * NEQ) {
+  if (tid < FB) sF[tid] = f0 + tid < nface ? prm.flist[f0 + tid] : make_int4(-1, -1, 0, 0);
+  __syncthreads();
+  if constexpr (STAGE) {
+    // one row of ND values per warp and load (Q1: four), all in flight at once
+    constexpr int RPW = 32 / ND, NG = 2 * FB / RPW, IT = (NG + S::NT / 32 - 1) / (S::NT / 32);
+    const int warp = tid >> 5, lane = tid & 31, sub = lane / ND, i = lane - sub * ND;
+    R tmp[IT][NEQ];
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      const int g = warp + it * (S::NT / 32), r = g * RPW + sub;
+      const bool on = g < NG && sub < RPW;
+      const int e = on ? (r >= FB ? sF[r - FB].y : sF[r].x) : -1;
+      const R* p = u + (long long)e * ND + i;
+#pragma unroll
+      for (int k = 0; k < NEQ; ++k) tmp[it][k] = e >= 0 ? __ldg(p + k * NDa) : R(0);
+    }
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      const int g = warp + it * (S::NT / 32), r = g * RPW + sub;
+      if (g < NG && sub < RPW) {
+#pragma unroll
+        for (int k = 0; k < NEQ; ++k) sU[(k * 2 * FB + r) * S::NDS + i] = tmp[it][k];
+      }
+    }
+    __syncthreads();
+  }
+  // traces, in each side's own tensor order a + NQ1 b; the face list is sorted
+  // by the faces' normal axis, so a warp takes one of the three orders
+  if (tid < NROW) {
     const int k = tid / (2 * FB), r = tid - k * 2 * FB, side = r / FB, fl = r - side * FB;
-    const int4 fc = f0 + fl < nface ? prm.flist[f0 + fl] : make_int4(-1, -1, 0, 0);
+    const int4 fc = sF[fl];
     const int e = side ? fc.y : fc.x;
     if (e >= 0) {
       const int lf = side ? (fc.z >> 3) & 7 : fc.z & 7;
-      const int ax = hex_face_axis(lf), sd = hex_face_side(lf);
-      const int sn = ax == 0 ? 1 : (ax == 1 ? N1 : NF2), s0 = ax == 0 ? N1 : 1, s1 = ax == 2 ? N1 : NF2;
-      const R* ue = u + k * NDa + (long long)e * ND;
-      R le[N1], v[NF2];
-#pragma unroll
-      for (int j = 0; j < N1; ++j) le[j] = sd ? H.lend[N1 + j] : H.lend[j];
-#pragma unroll
-      for (int i0 = 0; i0 < N1; ++i0)
-#pragma unroll
-        for (int i1 = 0; i1 < N1; ++i1) {
-          R s = R(0);
-#pragma unroll
-          for (int j = 0; j < N1; ++j) s += le[j] * __ldg(ue + j * sn + i0 * s0 + i1 * s1);
-          v[i0 * N1 + i1] = s;
-        }
+      R v[NF2];
+      team_contract_s_axis<P>(lf, STAGE ? sU + tid * S::NDS : u + k * NDa + (long long)e * ND, H.lend, v);
       team_interp<P, 1>(v, H.l1d, &sT[side][k][fl][0]);
     }
   }
@@ -88,7 +108,7 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
   if (tid < FB * NQF) {
     const int fl = tid / NQF, t1 = tid - fl * NQF;
     if (f0 + fl < nface) {
-      const int4 fc = prm.flist[f0 + fl];
+      const int4 fc = sF[fl];
       const int lf1 = fc.z & 7;
       const R* fg = (const R*)prm.fgeo + (long long)(lf1 * 4) * ne + fc.x;
       R n[3], s1[NEQ], s2[NEQ], F[NEQ];
@@ -100,7 +120,7 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
       for (int k = 0; k < NEQ; ++k) s1[k] = sT[0][k][fl][t1];
       bool none = false;
       if (fc.y >= 0) {
-        const int t2 = square_op(fc.z >> 6, t1 % NQ1, t1 / NQ1, NQ1);
+        const int op = fc.z >> 6, t2 = op ? square_op(op, t1 % NQ1, t1 / NQ1, NQ1) : t1;
 #pragma unroll
         for (int k = 0; k < NEQ; ++k) s2[k] = sT[1][k][fl][t2];
       } else {
@@ -126,7 +146,10 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
   }
   if constexpr (!SPEED) {
     __syncthreads();
-    // moments with the tangential basis, M1^-1 of both directions included
+    // moments with the tangential basis, M1^-1 of both directions included;
+    // the second side's traces are done with
+    R* sO = &sT[1][0][0][0];  // [NEQ][FB][NF2]
+    static_assert(NF2 <= QS, "moments fit the traces' place");
     if (tid < FB * NEQ) {
       const int k = tid / FB, fl = tid - k * FB;
       if (f0 + fl < nface) {
@@ -145,7 +168,7 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
             w[i0][b] = s;
           }
         }
-        R* out = (R*)prm.fslot + ((long long)k * nface + f0 + fl) * NF2;
+        R* out = sO + (k * FB + fl) * NF2;
 #pragma unroll
         for (int i1 = 0; i1 < N1; ++i1)
 #pragma unroll
@@ -156,6 +179,13 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
             out[i0 + N1 * i1] = s;
           }
       }
+    }
+    __syncthreads();
+    const int nval = min(FB, nface - f0) * NF2;
+#pragma unroll
+    for (int t0 = 0; t0 < NEQ * FB * NF2; t0 += S::NT) {
+      const int t = t0 + tid, k = t / (FB * NF2), r = t - k * (FB * NF2);
+      if (k < NEQ && r < nval) ((R*)prm.fslot)[((long long)k * nface + f0) * NF2 + r] = sO[t];
     }
   }
   block_max_commit<R>(lmax, prm.mcs);
@@ -169,31 +199,37 @@ __global__ void __launch_bounds__(HexFaces<P>::NTN)
   constexpr int N1 = S::N1, NF2 = S::NF2, ND = S::ND, NEQ = S::NEQ, EPB = S::EPB, NT = S::NTN;
   constexpr int NP = ND | 1;
   __shared__ R sG[3][NEQ][EPB * NP];
-  __shared__ R sMD[N1 * N1], sMB[2 * N1];
+  __shared__ R sMD[N1 * N1], sMB[2 * N1], sGeo[EPB][11];  // adj(J), 1/det J
   const HexOps<R>& H = hex_ops<R>(prm.hops);
   const int tid = threadIdx.x, ne = prm.ne;
   const long long NDa = prm.ndofs;
   const int sl = tid / ND, i = tid - sl * ND;
   const int e = blockIdx.x * EPB + sl;
   const bool live = sl < EPB && e < ne;
+  for (int t = tid; t < EPB * 10; t += NT) {
+    const int c = t / EPB, s = t - c * EPB;
+    if (blockIdx.x * EPB + s < ne)
+      sGeo[s][c] = __ldg((const R*)prm.egeo + (long long)c * ne + blockIdx.x * EPB + s);
+  }
   if (tid < N1 * N1) sMD[tid] = H.md[tid];
   if (tid < 2 * N1) sMB[tid] = H.mb[tid];
   const long long own = (long long)e * ND + i;
   R lmax = R(0), idet = R(0), acc[NEQ];
 #pragma unroll
   for (int k = 0; k < NEQ; ++k) acc[k] = R(0);
+  R st[NEQ];
   if (live) {
-    R st[NEQ];
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) st[k] = u[k * NDa + own];
-    const R* eg = (const R*)prm.egeo + e;
-    idet = eg[9LL * ne];
+  }
+  __syncthreads();
+  if (live) {
+    idet = sGeo[sl][9];
     R F[NEQ][3];
     lmax = flux_and_speed<3>(st, F, (R)prm.gamma, (R)prm.covolume);
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-      const R a0 = eg[(long long)(3 * r) * ne], a1 = eg[(long long)(3 * r + 1) * ne],
-              a2 = eg[(long long)(3 * r + 2) * ne];
+      const R a0 = sGeo[sl][3 * r], a1 = sGeo[sl][3 * r + 1], a2 = sGeo[sl][3 * r + 2];
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) sG[r][k][sl * NP + i] = a0 * F[k][0] + a1 * F[k][1] + a2 * F[k][2];
     }
@@ -206,11 +242,11 @@ __global__ void __launch_bounds__(HexFaces<P>::NTN)
 #pragma unroll
     for (int lf = 0; lf < 6; ++lf) {
       constexpr int AX[6] = {2, 1, 0, 1, 0, 2}, SD[6] = {0, 0, 1, 1, 0, 1};
-      const int ref = prm.fref[lf * ne + e], op = prm.fop[lf * ne + e];
+      const int ref = prm.fref[lf * ne + e], op = prm.fop ? prm.fop[lf * ne + e] : 0;
       const int t0 = AX[lf] == 0 ? jy : jx, t1 = AX[lf] == 2 ? jy : jz;
       const R b = sMB[SD[lf] * N1 + (AX[lf] == 0 ? jx : (AX[lf] == 1 ? jy : jz))];
       const R c = (ref & 1) ? b : -b;
-      const R* p = fx + (long long)(ref >> 1) * NF2 + square_op(op, t0, t1, N1);
+      const R* p = fx + (long long)(ref >> 1) * NF2 + (op ? square_op(op, t0, t1, N1) : t0 + N1 * t1);
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) acc[k] += c * __ldg(p + k * nf);
     }

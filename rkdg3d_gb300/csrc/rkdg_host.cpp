@@ -51,7 +51,7 @@ struct rkdg_ctx {
   int hex_variant = 0;  // RKDG_TUNE_HEX_KERNEL
   int gen_block = 0;    // RKDG_TUNE_GENERIC_BLOCK
   // faces in the order of their Elem1 (see RhsParams)
-  int nface = 0;
+  int nface = 0, nbface = 0;  // nbface: faces without a second element
   int4* d_flist = nullptr;
   int* d_fref = nullptr;
   unsigned char* d_fop = nullptr;
@@ -544,7 +544,8 @@ int square_op_host(int op, int i, int j, int n) {
   return ((op & 2) ? n - 1 - a : a) + n * ((op & 4) ? n - 1 - b : b);
 }
 
-// Faces of the face-pass kernels in the order of their Elem1 (see RhsParams).
+// Faces of the face-pass kernels in the order of their Elem1, hexahedra by
+// normal axis first (see RhsParams).
 bool face_tables(const rkdg_ctx* c, std::vector<int4>& flist, std::vector<int>& fref,
                  std::vector<unsigned char>& fop) {
   const RefTables& T = c->tab;
@@ -566,8 +567,12 @@ bool face_tables(const rkdg_ctx* c, std::vector<int4>& flist, std::vector<int>& 
       }
       if (ok) inverse[o] = (signed char)v;
     }
-  for (int e = 0; e < ne; ++e)
+  static const int axis[6] = {2, 1, 0, 1, 0, 2};  // of a hexahedron's local faces
+  bool turned = false;
+  for (int ax = 0; ax < (hex ? 3 : 1); ++ax)
+   for (int e = 0; e < ne; ++e)
     for (int lf = 0; lf < nfpe; ++lf) {
+      if (hex && axis[lf] != ax) continue;
       const size_t i = (size_t)lf * ne + e;
       const int e2 = c->h_fnbr[i], fc = c->h_fcode[i];
       if (e2 >= 0 && ((fc >> 3) & 1)) continue;  // the Elem2 side
@@ -592,6 +597,7 @@ bool face_tables(const rkdg_ctx* c, std::vector<int4>& flist, std::vector<int>& 
           op = o;
           fref[i2] = f * 2 + 1;
           fop[i2] = (unsigned char)inverse[op];
+          turned |= op != 0;
         } else {
           fref[i2] = f * 4 + 2 + op;
         }
@@ -600,6 +606,7 @@ bool face_tables(const rkdg_ctx* c, std::vector<int4>& flist, std::vector<int>& 
       }
       flist.push_back(r);
     }
+  if (!turned) fop.clear();  // every face's two elements index it alike
   return true;
 }
 
@@ -1523,6 +1530,8 @@ int rkdg_upload_mesh(rkdg_ctx* c, const rkdg_mesh_desc* m) {
     if (!face_tables(c, flist, fref, fop))
       return fail(c, RKDG_ERR_INVALID, "face points of two hexahedra do not match");
     c->nface = (int)flist.size();
+    c->nbface = 0;
+    for (const int4& f : flist) c->nbface += f.y < 0;
     CUDA_TRY(c, dalloc(c->d_flist, flist.size()));
     CUDA_TRY(c, dalloc(c->d_fref, fref.size()));
     CUDA_TRY(c, cudaMemcpy(c->d_flist, flist.data(), flist.size() * sizeof(int4), cudaMemcpyHostToDevice));
@@ -1933,14 +1942,15 @@ int rkdg_batch_run(rkdg_ctx* c, double* x, double t_end, double cfl, double dt0,
 namespace {
 
 struct Adj {
-  double *r, *ub, *zb, *acc, *w, *cross;
+  double *r, *ub, *zb, *acc, *w, *cross, *g;
   double *kb[4], *z[4], *y[4], *k[4];
 };
 
 int adj_bufs(rkdg_ctx* c, Adj& A) {
   const size_t n = (size_t)c->ndofs * c->neq;
   const size_t nvec = 5 + 16;
-  const size_t need = nvec * n + (size_t)4 * c->ne;  // + the limiter's min/max derivatives
+  // + the limiter's min/max derivatives and the face points' trace cotangents
+  const size_t need = nvec * n + (size_t)4 * c->ne + (size_t)2 * c->neq * c->nface * c->tab.nqf;
   if (c->adj_n < need) {
     CUDA_TRY(c, dalloc(c->d_adj, need));
     c->adj_n = need;
@@ -1956,6 +1966,7 @@ int adj_bufs(rkdg_ctx* c, Adj& A) {
   for (int i = 0; i < 4; ++i) { A.y[i] = p; p += n; }
   for (int i = 0; i < 4; ++i) { A.k[i] = p; p += n; }
   A.cross = p;
+  A.g = p + (size_t)4 * c->ne;
   return RKDG_OK;
 }
 
@@ -1983,12 +1994,12 @@ int limit_in_place(rkdg_ctx* c, double* x) {
 int rhs_t(rkdg_ctx* c, Adj& A, const double* y, const double* kbar, double* out) {
   CUDA_TRY(c, rkdg::launch_minv_apply(c->geom, c->p, c->ne, c->ndofs, c->d_tab, c->d_egeo64, kbar, A.r, c->stream));
   RhsParams P = rhs_params(c, 0, 0, 7);
-  CUDA_TRY(c, rkdg::launch_rhs_vjp(c->geom, c->p, P, y, A.r, out, c->stream));
+  CUDA_TRY(c, rkdg::launch_rhs_vjp(c->geom, c->p, P, y, A.r, A.g, c->nbface, out, c->stream));
   if (c->nnc) {  // the hanging faces' share, added to u_bar
     CUDA_TRY(c, rkdg::launch_nc_vjp(c->geom, c->p, P, nc_params(c), y, A.r, out, c->stream));
     c->launches += 2;
   }
-  c->launches += 2;
+  c->launches += c->nbface ? 4 : 3;
   return RKDG_OK;
 }
 

@@ -58,8 +58,10 @@ cudaError_t launch_batch_control(const BatchState& bs, cudaGraphConditionalHandl
 bool adjoint_supported(int geom, int p);
 cudaError_t launch_minv_apply(int geom, int p, int ne, long long ndofs, const RefTables* tab,
                               const double* egeo, const double* kb, double* r, cudaStream_t st);
+// gb: scratch for both sides' trace cotangents, [2][neq][nface * nqf];
+// boundary: the mesh has faces without a second element.
 cudaError_t launch_rhs_vjp(int geom, int p, const RhsParams& prm, const double* u, const double* r,
-                           double* ub, cudaStream_t st);
+                           double* gb, int boundary, double* ub, cudaStream_t st);
 // u_bar += the hanging faces' part of (dz/du)^T r (nonconforming meshes).
 cudaError_t launch_nc_vjp(int geom, int p, const RhsParams& prm, const NcParams& nc, const double* u,
                           const double* r, double* ub, cudaStream_t st);
