@@ -52,14 +52,11 @@ struct FluxSide {
 
 // Rusanov (rs_rusanov.cpp:6-40) on unrotated states.
 template <int DIM>
-__device__ __forceinline__ void rusanov_vjp(FluxSide<DIM>& A, FluxSide<DIM>& B, const double* n,
+__device__ __forceinline__ void rusanov_vjp(FluxSide<DIM>& A, FluxSide<DIM>& B, const Frame<DIM, double>& fr,
                                             const double* fb, double gamma) {
   constexpr int NEQ = DIM + 2;
-  double nn = 0.0;
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) nn += n[d] * n[d];
-  const double h = 0.5 * inv_norm(nn);
-  const double cA = sqrt(A.c2(gamma)), cB = sqrt(B.c2(gamma)), vA = sqrt(A.u2), vB = sqrt(B.u2);
+  const double h = fr.h, *n = fr.n;
+  const double cA = root(A.c2(gamma)), cB = root(B.c2(gamma)), vA = root(A.u2), vB = root(B.u2);
   const bool left = vA + cA > vB + cB;
   const double a = 0.5 * (left ? vA + cA : vB + cB);
   double ab = 0.0;  // cotangent of max(|u| + c)
@@ -91,8 +88,8 @@ __device__ __forceinline__ void rusanov_vjp(FluxSide<DIM>& A, FluxSide<DIM>& B, 
   // one side holds the maximum: no indexed copies
   auto speed = [&](FluxSide<DIM>& S, bool on) {
     const double e = on ? ab : 0.0;
-    S.cb += on ? e / (2.0 * c) : 0.0;
-    const double vb = v > 0.0 ? e / v : 0.0;  // 2 d|u| / d|u|^2
+    S.cb += on ? 0.5 * e * rcp(c) : 0.0;
+    const double vb = v > 0.0 ? e * rcp(v) : 0.0;  // 2 d|u| / d|u|^2
     double m2 = 0.0;
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
@@ -120,22 +117,22 @@ __device__ __forceinline__ void hll_vjp(FluxSide<DIM>& A, FluxSide<DIM>& B, cons
             qL = 1.0, qR = 1.0;
   const double gm1 = gamma - 1.0, iz = 2.0 * gamma / gm1, hg = 0.5 * (gamma + 1.0) / gamma;
   if (avg == 1) {
-    t = sqrt(B.s[0] * A.r);
-    wL = 1.0 / (1.0 + t);
+    t = root(B.s[0] * A.r);
+    wL = rcp(1.0 + t);
     wR = t * wL;
     const double du = u2 - u1, uav = wL * u1 + wR * u2;
-    cav = sqrt(wL * cA2 + wR * cB2 + 0.5 * wL * wR * du * du);
+    cav = root(wL * cA2 + wR * cB2 + 0.5 * wL * wR * du * du);
     SL = uav - cav;
     SR = uav + cav;
   } else {
-    cL = sqrt(cA2);
-    cR = sqrt(cB2);
-    x = A.p / B.p;
+    cL = root(cA2);
+    cR = root(cB2);
+    x = A.p * rcp(B.p);
     const int n = (int)rint(iz);
     const bool whole = n >= 2 && n <= 16 && fabs(iz - n) <= n * 1e-14;
-    xz = whole ? root_n(x, n, 1.0 / iz) : exp2(log2(x) / iz);
+    xz = whole ? root_n(x, n, 0.5 * gm1 / gamma) : exp2(log2(x) / iz);
     den = cL + cR * xz;
-    t = (cL + cR - 0.5 * gm1 * (u2 - u1)) / den;
+    t = (cL + cR - 0.5 * gm1 * (u2 - u1)) * rcp(den);
     if (whole) {
       pl = t;
       for (int i = 1; i < n; ++i) pl *= t;
@@ -143,8 +140,8 @@ __device__ __forceinline__ void hll_vjp(FluxSide<DIM>& A, FluxSide<DIM>& B, cons
       pl = powr(t, iz);
     }
     const double pr = pl * x;
-    if (pl > 1.0) qL = sqrt(1.0 + hg * (pl - 1.0));
-    if (pr > 1.0) qR = sqrt(1.0 + hg * (pr - 1.0));
+    if (pl > 1.0) qL = root(1.0 + hg * (pl - 1.0));
+    if (pr > 1.0) qR = root(1.0 + hg * (pr - 1.0));
     SL = u1 - qL * cL;
     SR = u2 + qR * cR;
   }
@@ -193,7 +190,7 @@ __device__ __forceinline__ void hll_vjp(FluxSide<DIM>& A, FluxSide<DIM>& B, cons
     double f1[NEQ], f2[NEQ];
     side_flux(A, u1, f1);
     side_flux(B, u2, f2);
-    const double inv = 1.0 / (SR - SL);
+    const double inv = rcp(SR - SL);
     double tot = 0.0;
 #pragma unroll
     for (int i = 0; i < NEQ; ++i) {
@@ -212,14 +209,14 @@ __device__ __forceinline__ void hll_vjp(FluxSide<DIM>& A, FluxSide<DIM>& B, cons
     flux_back(B, u2, u2b, f2);
   } else {
     const double k1 = SL - u1, k2 = SR - u2;
-    const double dn = A.s[0] * k1 - B.s[0] * k2, idn = 1.0 / dn;
+    const double dn = A.s[0] * k1 - B.s[0] * k2, idn = rcp(dn);
     const double ss = (B.p - A.p + A.s[1] * k1 - B.s[1] * k2) * idn;
     const bool left = ss > 0.0;
     double ssb = 0.0, k1b = 0.0, k2b = 0.0;
     auto star = [&](FluxSide<DIM>& S, double SK, double u, double k, double& SKb, double& ub, double& kb) {
       double f[NEQ];
       side_flux(S, u, f);
-      const double G = S.p + S.s[0] * k * (ss - u), extra = SK * G, inv = 1.0 / (SK - ss);
+      const double G = S.p + S.s[0] * k * (ss - u), extra = SK * G, inv = rcp(SK - ss);
       double tot = 0.0, skb = 0.0;
       const double eb = (fb[1] + fb[NEQ - 1] * ss) * inv;
 #pragma unroll
@@ -262,7 +259,7 @@ __device__ __forceinline__ void hll_vjp(FluxSide<DIM>& A, FluxSide<DIM>& B, cons
   }
   // wave speeds
   if (avg == 1) {
-    const double du = u2 - u1, ub = SLb + SRb, xb = (SRb - SLb) / (2.0 * cav);
+    const double du = u2 - u1, ub = SLb + SRb, xb = 0.5 * (SRb - SLb) * rcp(cav);
     double wLb = ub * u1 + xb * (cA2 + 0.5 * wR * du * du);
     const double wRb = ub * u2 + xb * (cB2 + 0.5 * wL * du * du);
     const double dub = xb * wL * wR * du;
@@ -277,22 +274,22 @@ __device__ __forceinline__ void hll_vjp(FluxSide<DIM>& A, FluxSide<DIM>& B, cons
     B.sb[0] += 0.5 * tb * t * B.r;
   } else {
     double cLb = -SLb * qL, cRb = SRb * qR;
-    double plb = pl > 1.0 ? -SLb * cL * hg / (2.0 * qL) : 0.0;
-    const double prb = pl * x > 1.0 ? SRb * cR * hg / (2.0 * qR) : 0.0;
+    double plb = pl > 1.0 ? -0.5 * SLb * cL * hg * rcp(qL) : 0.0;
+    const double prb = pl * x > 1.0 ? 0.5 * SRb * cR * hg * rcp(qR) : 0.0;
     plb += prb * x;
     double xb = prb * pl;
-    const double tb = plb * iz * pl / t, ab = tb / den, db = -ab * t;
+    const double tb = plb * iz * pl * rcp(t), ab = tb * rcp(den), db = -ab * t;
     cLb += ab + db;
     cRb += ab + db * xz;
-    xb += db * cR * xz / (iz * x);
+    xb += db * cR * xz * rcp(iz * x);
     const double dub = -0.5 * gm1 * ab;
     u1b += SLb - dub;
     u2b += SRb + dub;
-    const double ip = 1.0 / B.p;
+    const double ip = rcp(B.p);
     A.pb += xb * ip;
     B.pb -= xb * x * ip;
-    A.cb += cLb / (2.0 * cL);
-    B.cb += cRb / (2.0 * cR);
+    A.cb += 0.5 * cLb * rcp(cL);
+    B.cb += 0.5 * cRb * rcp(cR);
   }
   A.sb[1] += u1b * A.r;
   A.rb += u1b * A.s[1];
@@ -317,22 +314,23 @@ __device__ __forceinline__ void riemann_vjp(const double* s1, const double* s2, 
     f[i] = fb[i];
     g1[i] = g2[i] = 0.0;
   }
+  const Frame<DIM, double> fr = make_frame<DIM, double>(n);
   if (rs != 0) {
-    rotate<DIM>(x1, n);
-    rotate<DIM>(x2, n);
-    rotate<DIM>(f, n);
+    rotate<DIM>(x1, fr);
+    rotate<DIM>(x2, fr);
+    rotate<DIM>(f, fr);
   }
   const bool ok1 = A.load(x1, gamma, b), ok2 = B.load(x2, gamma, b);
   if (!ok1 || !ok2) return;
   if (rs == 0)
-    rusanov_vjp<DIM>(A, B, n, f, gamma);
+    rusanov_vjp<DIM>(A, B, fr, f, gamma);
   else
     hll_vjp<DIM>(A, B, f, gamma, rs, avg);
   A.finish(gamma, b);
   B.finish(gamma, b);
   if (rs != 0) {
-    inverse_rotate<DIM>(A.sb, n);
-    inverse_rotate<DIM>(B.sb, n);
+    inverse_rotate<DIM>(A.sb, fr);
+    inverse_rotate<DIM>(B.sb, fr);
   }
 #pragma unroll
   for (int i = 0; i < NEQ; ++i) {
@@ -346,8 +344,8 @@ template <int DIM>
 __device__ __forceinline__ void flux_vjp(const double* s, const double (*fb)[DIM], double gamma,
                                          double b, double* g) {
   constexpr int NEQ = DIM + 2;
-  const double r = 1.0 / s[0], p = pressure<DIM>(s, gamma, b), H = s[NEQ - 1] + p;
-  const double q = b == 0.0 ? 1.0 : 1.0 / (1.0 - s[0] * b);
+  const double r = rcp(s[0]), p = pressure<DIM>(s, gamma, b), H = s[NEQ - 1] + p;
+  const double q = b == 0.0 ? 1.0 : rcp(1.0 - s[0] * b);
   double rb = 0.0, pb = 0.0, eb = 0.0, m2 = 0.0;
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {

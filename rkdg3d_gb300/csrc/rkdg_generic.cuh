@@ -112,7 +112,8 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* addr, doub
 
 // Block-wide max of a per-thread wave speed, committed with one atomicMax per
 // block (the MPI_Allreduce(MAX) of main.cpp:543 on one device).
-template <typename R>
+// SQUARE: v is the square of a speed.
+template <typename R, bool SQUARE = false>
 __device__ __forceinline__ void block_max_commit(R v, unsigned long long* dst) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -125,7 +126,7 @@ __device__ __forceinline__ void block_max_commit(R v, unsigned long long* dst) {
     R x = lane < nw ? redd[lane] : R(0);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
-    if (lane == 0) atomic_max_nonneg(dst, (double)x);
+    if (lane == 0) atomic_max_nonneg(dst, SQUARE ? sqrt((double)x) : (double)x);
   }
 }
 
@@ -142,6 +143,8 @@ __device__ __forceinline__ void flag_error(int* err, int code, int where) {
 // only its own problem: the problem is marked failed and the others go on.
 template <typename R>
 __device__ __forceinline__ R checked_speed(const RhsParams& prm, R sp, int e, int pb = -1) {
+  if constexpr (std::is_same<R, double>::value)
+    if (__double2hiint(sp) >= 0) return sp;  // the sign on the integer pipe
   if (sp < R(0)) {
     if (!(prm.quirks & 1) || sp == R(-1)) {
       if (pb >= 0 && prm.pfail)
@@ -157,7 +160,7 @@ __device__ __forceinline__ R checked_speed(const RhsParams& prm, R sp, int e, in
 // Per-problem max wave speed for batched problems: elements of one problem
 // are contiguous, so a warp holds a few contiguous runs; a segmented shuffle
 // reduction leaves each run's max in its first lane, which commits it.
-template <typename R>
+template <typename R, bool SQUARE = false>
 __device__ __forceinline__ void segmented_max_commit(R v, int pb, unsigned long long* pmcs) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -167,7 +170,7 @@ __device__ __forceinline__ void segmented_max_commit(R v, int pb, unsigned long 
     if (lane + off < 32 && opb == pb) v = fmax(v, o);
   }
   const int prev = __shfl_up_sync(0xffffffffu, pb, 1);
-  if (pb >= 0 && (lane == 0 || prev != pb)) atomic_max_nonneg(&pmcs[pb], (double)v);
+  if (pb >= 0 && (lane == 0 || prev != pb)) atomic_max_nonneg(&pmcs[pb], SQUARE ? sqrt((double)v) : (double)v);
 }
 
 // Batched problems with a map of the active work: the i-th element of the

@@ -61,10 +61,15 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
   __shared__ R sT[2][NEQ][FB][QS];
   __shared__ R sU[STAGE ? NROW * S::NDS : 1];
   __shared__ int4 sF[FB];
+  __shared__ Frame<3, R> sFr[FB];
+  __shared__ R sJ[FB];
   const HexOps<R>& H = hex_ops<R>(prm.hops);
   const int tid = threadIdx.x, f0 = blockIdx.x * FB, nface = prm.nface, ne = prm.ne;
   const long long NDa = prm.ndofs;
-  if (tid < FB) sF[tid] = f0 + tid < nface ? prm.flist[f0 + tid] : make_int4(-1, -1, 0, 0);
+  if (tid < FB) {
+    const int4 fc = f0 + tid < nface ? prm.flist[f0 + tid] : make_int4(-1, -1, 0, 0);
+    sF[tid] = fc;
+  }
   __syncthreads();
   if constexpr (STAGE) {
     // one row of ND values per warp and load (Q1: four), all in flight at once
@@ -90,6 +95,19 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
     }
     __syncthreads();
   }
+  // the faces' frames, by the last threads (the first ones have traces to form)
+  if (tid >= S::NT - FB) {
+    const int fl = tid - (S::NT - FB);
+    const int4 fc = sF[fl];
+    if (fc.x >= 0) {
+      const R* fg = (const R*)prm.fgeo + (long long)((fc.z & 7) * 4) * ne + fc.x;
+      R n[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) n[c] = __ldg(fg + (long long)c * ne);
+      sFr[fl] = make_frame<3, R>(n);
+      sJ[fl] = __ldg(fg + 3LL * ne);
+    }
+  }
   // traces, in each side's own tensor order a + NQ1 b; the face list is sorted
   // by the faces' normal axis, so a warp takes one of the three orders
   if (tid < NROW) {
@@ -110,11 +128,7 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
     if (f0 + fl < nface) {
       const int4 fc = sF[fl];
       const int lf1 = fc.z & 7;
-      const R* fg = (const R*)prm.fgeo + (long long)(lf1 * 4) * ne + fc.x;
-      R n[3], s1[NEQ], s2[NEQ], F[NEQ];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) n[c] = __ldg(fg + (long long)c * ne);
-      const R jac = __ldg(fg + 3LL * ne);
+      R s1[NEQ], s2[NEQ], F[NEQ];
       const R gamma = (R)prm.gamma, cov = (R)prm.covolume;
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) s1[k] = sT[0][k][fl][t1];
@@ -128,19 +142,19 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
         none = nb == -1;  // no integrator
         if (!none) {
           const BCSlot& bc = prm.bc[-2 - nb];
-          right_state<3>(bc.type, bc.state, s1, s2, n, gamma, cov, (R)prm.rgas);
+          right_state<3>(bc.type, bc.state, s1, s2, sFr[fl].n, gamma, cov, (R)prm.rgas);
         }
       }
       if (none) {
 #pragma unroll
         for (int k = 0; k < NEQ; ++k) F[k] = R(0);
       } else {
-        lmax = checked_speed(prm, riemann<3>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), fc.x);
+        lmax = checked_speed(prm, riemann<3>(s1, s2, sFr[fl], F, gamma, cov, prm.rs, prm.avg), fc.x);
       }
       if constexpr (!SPEED) {
         // this thread alone reads the point it overwrites
 #pragma unroll
-        for (int k = 0; k < NEQ; ++k) sT[0][k][fl][t1] = F[k] * jac;
+        for (int k = 0; k < NEQ; ++k) sT[0][k][fl][t1] = F[k] * sJ[fl];
       }
     }
   }
@@ -199,7 +213,7 @@ __global__ void __launch_bounds__(HexFaces<P>::NTN)
   constexpr int N1 = S::N1, NF2 = S::NF2, ND = S::ND, NEQ = S::NEQ, EPB = S::EPB, NT = S::NTN;
   constexpr int NP = ND | 1;
   __shared__ R sG[3][NEQ][EPB * NP];
-  __shared__ R sMD[N1 * N1], sMB[2 * N1], sGeo[EPB][11];  // adj(J), 1/det J
+  __shared__ R sMD[N1 * N1], sGeo[EPB][11];  // sGeo: adj(J), 1/det J
   const HexOps<R>& H = hex_ops<R>(prm.hops);
   const int tid = threadIdx.x, ne = prm.ne;
   const long long NDa = prm.ndofs;
@@ -212,7 +226,7 @@ __global__ void __launch_bounds__(HexFaces<P>::NTN)
       sGeo[s][c] = __ldg((const R*)prm.egeo + (long long)c * ne + blockIdx.x * EPB + s);
   }
   if (tid < N1 * N1) sMD[tid] = H.md[tid];
-  if (tid < 2 * N1) sMB[tid] = H.mb[tid];
+  const int jx = i % N1, jy = (i / N1) % N1, jz = i / NF2;
   const long long own = (long long)e * ND + i;
   R lmax = R(0), idet = R(0), acc[NEQ];
 #pragma unroll
@@ -221,22 +235,7 @@ __global__ void __launch_bounds__(HexFaces<P>::NTN)
   if (live) {
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) st[k] = u[k * NDa + own];
-  }
-  __syncthreads();
-  if (live) {
-    idet = sGeo[sl][9];
-    R F[NEQ][3];
-    lmax = flux_and_speed<3>(st, F, (R)prm.gamma, (R)prm.covolume);
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      const R a0 = sGeo[sl][3 * r], a1 = sGeo[sl][3 * r + 1], a2 = sGeo[sl][3 * r + 2];
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) sG[r][k][sl * NP + i] = a0 * F[k][0] + a1 * F[k][1] + a2 * F[k][2];
-    }
-  }
-  __syncthreads();
-  if (live) {
-    const int jx = i % N1, jy = (i / N1) % N1, jz = i / NF2;
+    // the faces' moments, in flight with the state
     const R* fx = (const R*)prm.fslot;
     const long long nf = (long long)prm.nface * NF2;
 #pragma unroll
@@ -244,12 +243,31 @@ __global__ void __launch_bounds__(HexFaces<P>::NTN)
       constexpr int AX[6] = {2, 1, 0, 1, 0, 2}, SD[6] = {0, 0, 1, 1, 0, 1};
       const int ref = prm.fref[lf * ne + e], op = prm.fop ? prm.fop[lf * ne + e] : 0;
       const int t0 = AX[lf] == 0 ? jy : jx, t1 = AX[lf] == 2 ? jy : jz;
-      const R b = sMB[SD[lf] * N1 + (AX[lf] == 0 ? jx : (AX[lf] == 1 ? jy : jz))];
+      const int jn = AX[lf] == 0 ? jx : (AX[lf] == 1 ? jy : jz);
+      R b = H.mb[SD[lf] * N1];  // by selection: an indexed constant is read lane by lane
+#pragma unroll
+      for (int j = 1; j < N1; ++j) b = jn == j ? H.mb[SD[lf] * N1 + j] : b;
       const R c = (ref & 1) ? b : -b;
       const R* p = fx + (long long)(ref >> 1) * NF2 + (op ? square_op(op, t0, t1, N1) : t0 + N1 * t1);
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) acc[k] += c * __ldg(p + k * nf);
     }
+  }
+  __syncthreads();
+  if (live) {
+    idet = sGeo[sl][9];
+    const NodeFlux<3, R> N(st, (R)prm.gamma, (R)prm.covolume);
+    lmax = N.speed;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      R G[NEQ];
+      N.contra(st, &sGeo[sl][3 * r], G);
+#pragma unroll
+      for (int k = 0; k < NEQ; ++k) sG[r][k][sl * NP + i] = G[k];
+    }
+  }
+  __syncthreads();
+  if (live) {
 #pragma unroll
     for (int m = 0; m < N1; ++m) {
       const R d0 = sMD[jx * N1 + m], d1 = sMD[jy * N1 + m], d2 = sMD[jz * N1 + m];
@@ -310,7 +328,7 @@ __global__ void __launch_bounds__(HexFaces<P>::NTN)
       }
     }
   }
-  block_max_commit<R>(lmax, prm.mcs);
+  block_max_commit<R, std::is_same<R, double>::value>(lmax, prm.mcs);
 }
 
 }  // namespace rkdg

@@ -23,7 +23,7 @@ struct LimTeam {
     // means, values (and low words), operators, factors, gas constants, ids
     return 8 * epb * E::NEQ + (sizeof(R) + (DS ? 4 : 0)) * epb * E::NEQ * NDP +
            8 * (size_t)E::ND * NPT + sizeof(R) * (size_t)E::ND * E::NV + 16 * epb + 2 * sizeof(R) * epb +
-           2 * sizeof(int) * epb + 16;
+           2 * sizeof(int) * epb + (sizeof(R) == 8 ? 8 * epb * E::NEQ : 0) + 16;
   }
 };
 
@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
   R* sBv = sU + NEQ * EPB * NDP;                                   // [ND][NV]
   R* sG = sBv + ND * NV;                                           // [EPB] gamma, [EPB] covolume
   float* sLo = reinterpret_cast<float*>(sG + 2 * EPB);             // [NEQ][EPB][NDP]
-  int* sE = reinterpret_cast<int*>(sLo + (DS ? NEQ * EPB * NDP : 0));  // [EPB]
+  double* sL = reinterpret_cast<double*>(sLo);                     // FP64: [NEQ][EPB] means' low parts
+  int* sE = reinterpret_cast<int*>(sLo + (DS ? NEQ * EPB * NDP : (F32 ? 0 : 2 * NEQ * EPB)));  // [EPB]
   int* sF = sE + EPB;                                              // [EPB] 1 changed, 2 mean
   const int ne = prm.ne;
   const long long NDa = prm.ndofs;
@@ -359,6 +360,21 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
       }
       __syncthreads();
     }
+    if constexpr (!F32) {
+      // what rounding the mean to FP64 left out: with it the limited values
+      // average to the unrounded mean, and a limited run's rounding does not
+      // accumulate one bit of every mean per stage
+      for (int t = tid; t < EPB * NEQ; t += NT) {
+        const int s = t % EPB;
+        if (!sF[s]) continue;
+        const double* w = tab->wmn_e ? tab->wmn_e + (long long)sE[s] * ND : tab->wmean;
+        double l = 0.0;
+#pragma unroll
+        for (int j = 0; j < ND; ++j) l += w[j] * (sU[t * NDP + j] - sM[t]);
+        sL[t] = l;
+      }
+      __syncthreads();
+    }
     for (int t = tid; t < EPB * ND; t += NT) {
       const int s = t / ND, j = t - s * ND;
       if (!sF[s]) continue;
@@ -367,7 +383,8 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
         R& v = sU[(k * EPB + s) * NDP + j];
         const MeanT um = sM[k * EPB + s];
         if constexpr (!F32) {
-          v = um + sMr[s] * (v - um);
+          const double l = sL[k * EPB + s], d = v - um;
+          v = um + (l + sMr[s] * (d - l));
         } else {
           const float2 m = reinterpret_cast<float2*>(sMr)[s];
           float h = v;

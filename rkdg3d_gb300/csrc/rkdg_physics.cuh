@@ -104,14 +104,71 @@ __device__ __forceinline__ R max_char_speed(const R* s, R gamma, R b) {
   return fsq(fdv(v2, den)) + c;
 }
 
-// 1/x: double rounded to nearest, float the hardware approximation.
+// FP64 reciprocal and square root to about one ulp: the hardware's gross
+// approximation of 1/x or 1/sqrt(x) (20 bits of the mantissa) and one step of
+// Householder's method of third order, 1/(1 - e) = 1 + e + e^2 + ... and
+// 1/sqrt(1 - e) = 1 + e/2 + 3 e^2/8 + ... with the residual e < 2^-18, so that the
+// truncation lies below 2^-55.  Three and five FP64 operations against seven to
+// ten of the correctly rounded forms, in kernels that the FP64 pipe bounds.
+// Zero, subnormal, infinite, negative (root) and NaN arguments take those.
+__device__ __forceinline__ double rcp_f64(double x) {
+#ifdef __CUDA_ARCH__
+  if ((unsigned)((__double2hiint(x) & 0x7fffffff) - 0x00100000) >= 0x7fc00000u) return 1.0 / x;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+#else
+  return 1.0 / x;
+#endif
+}
+__device__ __forceinline__ double sqrt_f64(double x) {
+#ifdef __CUDA_ARCH__
+  if ((unsigned)(__double2hiint(x) - 0x00100000) >= 0x7fe00000u) return sqrt(x);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double t = x * y, e = fma(-t, y, 1.0);
+  return fma(t * e, fma(0.375, e, 0.5), t);
+#else
+  return sqrt(x);
+#endif
+}
+// 1/x and sqrt(x): double as above, float the hardware approximations.
 template <typename R>
 __device__ __forceinline__ R rcp(R x) {
-  return R(1) / x;
+  return rcp_f64(x);
 }
 template <>
 __device__ __forceinline__ float rcp<float>(float x) {
   return __fdividef(1.0f, x);
+}
+template <typename R>
+__device__ __forceinline__ R root(R x) {
+  return sqrt_f64(x);
+}
+template <>
+__device__ __forceinline__ float root<float>(float x) {
+  return fsq<float>(x);
+}
+// a / b of the flux formulas
+template <typename R>
+__device__ __forceinline__ R quot(R a, R b) {
+  return a * rcp(b);
+}
+template <>
+__device__ __forceinline__ float quot<float>(float a, float b) {
+  return __fdividef(a, b);
+}
+
+// x > 0 (ge: x >= 0), false for NaN.  A double's sign and exponent decide on the
+// integer pipe for normal numbers.
+template <bool GE, typename R>
+__device__ __forceinline__ bool positive(R x) {
+#ifdef __CUDA_ARCH__
+  if constexpr (std::is_same<R, double>::value)
+    if ((unsigned)(__double2hiint(x) - 0x00100000) < 0x7fe00000u) return true;
+#endif
+  return GE ? x >= R(0) : x > R(0);
 }
 
 // Pointwise state quantities with one reciprocal of the density and one of
@@ -125,7 +182,7 @@ __device__ __forceinline__ float rcp<float>(float x) {
 template <int DIM, typename R>
 __device__ __forceinline__ bool eos_state(const R* s, R gamma, R b, R& r, R& q, R& p, R& u2) {
   const R den = s[0], E = s[1 + DIM];
-  if (!(den >= R(0)) || !(E > R(0))) return false;
+  if (!positive<true>(den) || !positive<false>(E)) return false;
   r = rcp(den);
   R m2 = R(0);
 #pragma unroll
@@ -133,9 +190,13 @@ __device__ __forceinline__ bool eos_state(const R* s, R gamma, R b, R& r, R& q, 
   const R v2 = m2 * r;  // |m|^2 / rho
   const R ie = E - R(0.5) * v2;
   const R pg = (gamma - R(1)) * ie;
-  if (!(pg > R(0))) return false;
-  q = b == R(0) ? R(1) : rcp(R(1) - den * b);
-  p = pg * q;
+  if (!positive<false>(pg)) return false;
+  q = R(1);
+  p = pg;
+  if (b != R(0)) {
+    q = rcp(R(1) - den * b);
+    p = pg * q;
+  }
   if constexpr (std::is_same<R, float>::value) {
     if (fabsf(ie) < 1e-3f * fabsf(E)) {
       double m2d = 0.0;
@@ -148,6 +209,12 @@ __device__ __forceinline__ bool eos_state(const R* s, R gamma, R b, R& r, R& q, 
   u2 = v2 * r;
   return true;
 }
+// c^2 = gamma p / (rho (1 - rho b))
+template <typename R>
+__device__ __forceinline__ R sound2(R gamma, R p, R r, R q, R b) {
+  const R c = gamma * p * r;
+  return b != R(0) ? c * q : c;
+}
 
 // 1/|n| of a face normal: unit to rounding in every table (two terms of the
 // series about 1), else the reciprocal root.
@@ -158,40 +225,102 @@ __device__ __forceinline__ R inv_norm(R nn) {
   return R(1) / sqrt(nn);
 }
 
+// A face's normal and the rotation into its frame (RiemannSolver::Rotate,
+// rs_basic.cpp:11-67), formed once per face.  h = 1 / (2 |n|).
+template <int DIM, typename R>
+struct Frame {
+  R n[DIM], h, cp, st, ct;
+};
+template <int DIM, typename R>
+__device__ __forceinline__ Frame<DIM, R> make_frame(const R* n) {
+  Frame<DIM, R> F;
+  R nn = R(0);
+#pragma unroll
+  for (int d = 0; d < DIM; d++) {
+    F.n[d] = n[d];
+    nn += n[d] * n[d];
+  }
+  F.h = R(0.5) * inv_norm(nn);
+  F.cp = F.st = F.ct = R(0);
+  if constexpr (DIM == 3) {
+    F.cp = fsq(R(1) - n[2] * n[2]);
+    const bool ok = fabs(F.cp) > R(1e-6);
+    const R ic = fdv(R(1), F.cp);
+    F.st = ok ? n[1] * ic : R(1);
+    F.ct = ok ? n[0] * ic : R(0);
+  }
+  return F;
+}
+template <int DIM, typename R>
+__device__ __forceinline__ void rotate(R* s, const Frame<DIM, R>& F) {
+  R* m = s + 1;
+  const R* n = F.n;
+  if constexpr (DIM == 2) {
+    const R mx = n[0] * m[0] + n[1] * m[1];
+    const R my = -n[1] * m[0] + n[0] * m[1];
+    m[0] = mx;
+    m[1] = my;
+  } else {
+    const R sp = n[2], a = F.ct * m[0] + F.st * m[1];
+    const R my = -F.st * m[0] + F.ct * m[1];
+    const R mx = F.cp * a + sp * m[2];
+    const R mz = F.cp * m[2] - sp * a;
+    m[0] = mx;
+    m[1] = my;
+    m[2] = mz;
+  }
+}
+template <int DIM, typename R>
+__device__ __forceinline__ void inverse_rotate(R* s, const Frame<DIM, R>& F) {
+  R* m = s + 1;
+  const R* n = F.n;
+  if constexpr (DIM == 2) {
+    const R mx = n[0] * m[0] - n[1] * m[1];
+    const R my = n[1] * m[0] + n[0] * m[1];
+    m[0] = mx;
+    m[1] = my;
+  } else {
+    const R sp = n[2], a = F.cp * m[0] - sp * m[2];
+    const R mz = sp * m[0] + F.cp * m[2];
+    const R mx = F.ct * a - F.st * m[1];
+    const R my = F.st * a + F.ct * m[1];
+    m[0] = mx;
+    m[1] = my;
+    m[2] = mz;
+  }
+}
+
 // Rusanov flux (rs_rusanov.cpp:6-40) on unrotated states.  Returns the wave
 // speed, or -1 for a non-physical state.  max(|u| + c) is the root of
 // max(|u|^2 + c^2 + 2 |u| c): three square roots for the two sides.
 template <int DIM, typename R>
-__device__ __forceinline__ R rusanov_flux(const R* s1, const R* s2, const R* n, R* flux, R gamma,
-                                          R b) {
+__device__ __forceinline__ R rusanov_flux(const R* s1, const R* s2, const Frame<DIM, R>& fr, R* flux,
+                                          R gamma, R b) {
   constexpr int NEQ = DIM + 2;
   R r1, q1, p1, w1, r2, q2, p2, w2;
   if (!eos_state<DIM>(s1, gamma, b, r1, q1, p1, w1)) return R(-1);
   if (!eos_state<DIM>(s2, gamma, b, r2, q2, p2, w2)) return R(-1);
   R maxE;
   if constexpr (std::is_same<R, double>::value) {
-    const R c1 = gamma * p1 * r1 * q1, c2 = gamma * p2 * r2 * q2;
-    maxE = sqrt(fmax(w1 + c1 + R(2) * sqrt(w1 * c1), w2 + c2 + R(2) * sqrt(w2 * c2)));
+    const R c1 = sound2(gamma, p1, r1, q1, b), c2 = sound2(gamma, p2, r2, q2, b);
+    maxE = root(fmax(w1 + c1 + R(2) * root(w1 * c1), w2 + c2 + R(2) * root(w2 * c2)));
   } else {
     const R e1 = fsq(w1) + fsq(gamma * p1 * r1 * q1), e2 = fsq(w2) + fsq(gamma * p2 * r2 * q2);
     maxE = e1 > e2 ? e1 : e2;
   }
-  R d1 = R(0), d2 = R(0), nn = R(0);
+  R nh[DIM], d1 = R(0), d2 = R(0);
 #pragma unroll
   for (int d = 0; d < DIM; d++) {
-    d1 += s1[1 + d] * n[d];
-    d2 += s2[1 + d] * n[d];
-    nn += n[d] * n[d];
+    nh[d] = fr.h * fr.n[d];
+    d1 += s1[1 + d] * nh[d];
+    d2 += s2[1 + d] * nh[d];
   }
-  const R h = R(0.5) * inv_norm(nn), a = R(0.5) * maxE;
-  const R u1 = d1 * r1, u2 = d2 * r2;
-  flux[0] = h * (d1 + d2) - a * (s2[0] - s1[0]);
+  const R a = R(0.5) * maxE, u1 = d1 * r1, u2 = d2 * r2, ps = p1 + p2;
+  flux[0] = d1 + d2 - a * (s2[0] - s1[0]);
 #pragma unroll
   for (int d = 0; d < DIM; d++)
-    flux[1 + d] = h * ((u1 * s1[1 + d] + p1 * n[d]) + (u2 * s2[1 + d] + p2 * n[d])) -
-                  a * (s2[1 + d] - s1[1 + d]);
-  flux[NEQ - 1] = h * (u1 * (s1[NEQ - 1] + p1) + u2 * (s2[NEQ - 1] + p2)) -
-                  a * (s2[NEQ - 1] - s1[NEQ - 1]);
+    flux[1 + d] = u1 * s1[1 + d] + u2 * s2[1 + d] + ps * nh[d] - a * (s2[1 + d] - s1[1 + d]);
+  flux[NEQ - 1] = u1 * (s1[NEQ - 1] + p1) + u2 * (s2[NEQ - 1] + p2) - a * (s2[NEQ - 1] - s1[NEQ - 1]);
   return maxE;
 }
 
@@ -241,6 +370,45 @@ __device__ __forceinline__ R flux_and_speed(const R* s, R F[DIM + 2][DIM], R gam
   const R c = fsq(fdv(gamma * pres * inv, R(1) - den * b));
   return fsq(v2 * inv * inv) + c;
 }
+
+// A node's Euler flux (ComputeFlux, physics.cpp:143-168) by contravariant
+// components: a . F = (un rho, un m + p a, un (E + p)) with un = a . u.
+// speed: |u| + c, in FP64 its square (one root instead of two, taken of the
+// maximum).
+template <int DIM, typename R>
+struct NodeFlux {
+  R u[DIM], p, H, speed;
+  __device__ __forceinline__ NodeFlux(const R* s, R gamma, R b) {
+    R r, q, u2;
+    if (!eos_state<DIM>(s, gamma, b, r, q, p, u2)) {
+      // non-physical node: the same quantities without the checks
+      r = rcp(s[0]);
+      p = pressure<DIM>(s, gamma, b);
+      u2 = R(0);
+#pragma unroll
+      for (int d = 0; d < DIM; d++) u2 += s[1 + d] * s[1 + d];
+      u2 = u2 * r * r;
+      q = rcp(R(1) - s[0] * b);
+    }
+    H = s[1 + DIM] + p;
+#pragma unroll
+    for (int d = 0; d < DIM; d++) u[d] = s[1 + d] * r;
+    const R c = sound2(gamma, p, r, q, b);
+    if constexpr (std::is_same<R, double>::value)
+      speed = u2 + c + R(2) * root(u2 * c);
+    else
+      speed = fsq(u2) + fsq(c);
+  }
+  __device__ __forceinline__ void contra(const R* s, const R* a, R* G) const {
+    R un = R(0);
+#pragma unroll
+    for (int d = 0; d < DIM; d++) un += a[d] * u[d];
+    G[0] = un * s[0];
+#pragma unroll
+    for (int d = 0; d < DIM; d++) G[1 + d] = un * s[1 + d] + p * a[d];
+    G[1 + DIM] = un * H;
+  }
+};
 
 // ComputeFluxDotN (physics.cpp:171-195)
 template <int DIM, typename R>
@@ -375,7 +543,7 @@ __device__ __forceinline__ double root_n(double x, int n, double invn) {
   double yn = y;
   for (int i = 1; i < n; ++i) yn *= y;
   const double m = n - 1, k = n + 1;
-  return y * (m * yn + k * x) / (k * yn + m * x);
+  return y * (m * yn + k * x) * rcp_f64(k * yn + m * x);
 }
 
 // TRRS wave speeds (ComputeToroCharSpeeds, physics.cpp:309-350) from the
@@ -387,17 +555,17 @@ __device__ __forceinline__ double root_n(double x, int n, double invn) {
 template <typename R>
 __device__ __forceinline__ void trrs_speeds(R uL, R uR, R cL, R cR, R pL, R pR, R gamma, R& SL, R& SR) {
   const R gm1 = gamma - R(1);
-  const R iz = fdv(R(2) * gamma, gm1);
-  const R x = fdv(pL, pR);
+  const R iz = quot(R(2) * gamma, gm1);
+  const R x = quot(pL, pR);
   const int n = (int)rint(iz);
   const bool whole = n >= 2 && n <= 16 && fabs(iz - R(n)) <= R(n) * (std::is_same<R, double>::value ? R(1e-14) : R(1e-6));
   R xz;  // (pL/pR)^z
   if constexpr (std::is_same<R, double>::value)
-    xz = whole ? root_n(x, n, R(1) / iz) : exp2(log2(x) / iz);
+    xz = whole ? root_n(x, n, R(0.5) * gm1 * rcp(gamma)) : exp2(log2(x) / iz);
   else
-    xz = exp2f(fdv(log2f(x), iz));
+    xz = exp2f(quot(log2f(x), iz));
   const R a = cL + cR - R(0.5) * gm1 * (uR - uL);
-  const R t = fdv(a, cL + cR * xz);
+  const R t = quot(a, cL + cR * xz);
   R pl;  // pStar / pL
   if (whole) {
     pl = t;
@@ -405,10 +573,10 @@ __device__ __forceinline__ void trrs_speeds(R uL, R uR, R cL, R cR, R pL, R pR, 
   } else {
     pl = powr(t, iz);
   }
-  const R hg = fdv(R(0.5) * (gamma + R(1)), gamma);
+  const R hg = quot(R(0.5) * (gamma + R(1)), gamma);
   const R pr = pl * x;
-  SL = uL - (pl > R(1) ? fsq(R(1) + hg * (pl - R(1))) * cL : cL);
-  SR = uR + (pr > R(1) ? fsq(R(1) + hg * (pr - R(1))) * cR : cR);
+  SL = uL - (pl > R(1) ? root(R(1) + hg * (pl - R(1))) * cL : cL);
+  SR = uR + (pr > R(1) ? root(R(1) + hg * (pr - R(1))) * cR : cR);
 }
 
 // Einfeldt wave speeds (ComputeEinfeldtCharSpeeds, physics.cpp:269-296): the
@@ -416,11 +584,11 @@ __device__ __forceinline__ void trrs_speeds(R uL, R uR, R cL, R cR, R pL, R pR, 
 // speeds through their squares.
 template <typename R>
 __device__ __forceinline__ void einfeldt_speeds(R uL, R uR, R cL2, R cR2, R rL, R rhoR, R& SL, R& SR) {
-  const R t = fsq(rhoR * rL);
+  const R t = root(rhoR * rL);
   const R wL = rcp(R(1) + t), wR = t * wL;
   const R du = uR - uL;
   const R uav = wL * uL + wR * uR;
-  const R cav = fsq(wL * cL2 + wR * cR2 + R(0.5) * wL * wR * du * du);
+  const R cav = root(wL * cL2 + wR * cR2 + R(0.5) * wL * wR * du * du);
   SL = uav - cav;
   SR = uav + cav;
 }
@@ -428,21 +596,21 @@ __device__ __forceinline__ void einfeldt_speeds(R uL, R uR, R cL2, R cR2, R rL, 
 // LLF, HLL and HLLC (rs_llf.cpp:6-37, rs_hll.cpp:6-50, rs_hllc.cpp:71-161) in
 // plain arithmetic types, on the states rotated into the face frame.
 template <int DIM, typename R>
-__device__ __forceinline__ R hll_family(R* s1, R* s2, const R* n, R* flux, R gamma, R b, int rs,
+__device__ __forceinline__ R hll_family(R* s1, R* s2, const Frame<DIM, R>& fr, R* flux, R gamma, R b, int rs,
                                         int avg) {
   constexpr int NEQ = DIM + 2;
   R r1, q1, p1, w1, r2, q2, p2, w2;
   if (!eos_state<DIM>(s1, gamma, b, r1, q1, p1, w1)) return R(-1);
   if (!eos_state<DIM>(s2, gamma, b, r2, q2, p2, w2)) return R(-1);
-  rotate<DIM>(s1, n);
-  rotate<DIM>(s2, n);
+  rotate<DIM>(s1, fr);
+  rotate<DIM>(s2, fr);
   const R u1 = s1[1] * r1, u2 = s2[1] * r2;
-  const R c1 = gamma * p1 * r1 * q1, c2 = gamma * p2 * r2 * q2;  // squares
+  const R c1 = sound2(gamma, p1, r1, q1, b), c2 = sound2(gamma, p2, r2, q2, b);  // squares
   R SL, SR;
   if (avg == 1)
     einfeldt_speeds(u1, u2, c1, c2, r1, s2[0], SL, SR);
   else
-    trrs_speeds(u1, u2, fsq(c1), fsq(c2), p1, p2, gamma, SL, SR);
+    trrs_speeds(u1, u2, root(c1), root(c2), p1, p2, gamma, SL, SR);
   R ret = fmax(fabs(SL), fabs(SR));
   // x-flux of a rotated state (ComputeFluxF, physics.cpp:198-231)
   auto side_flux = [&](const R* s, R u, R p, R* f) {
@@ -473,7 +641,7 @@ __device__ __forceinline__ R hll_family(R* s1, R* s2, const R* n, R* flux, R gam
       flux[i] = (SR * f1[i] - SL * flux[i] + pp * (s2[i] - s1[i])) * inv;
   } else {
     const R k1 = SL - u1, k2 = SR - u2;
-    const R sStar = fdv(p2 - p1 + s1[1] * k1 - s2[1] * k2, s1[0] * k1 - s2[0] * k2);
+    const R sStar = quot(p2 - p1 + s1[1] * k1 - s2[1] * k2, s1[0] * k1 - s2[0] * k2);
     const bool left = sStar > R(0);
     const R* st = left ? s1 : s2;
     const R SK = left ? SL : SR, uK = left ? u1 : u2, pK = left ? p1 : p2, kK = left ? k1 : k2;
@@ -490,7 +658,7 @@ __device__ __forceinline__ R hll_family(R* s1, R* s2, const R* n, R* flux, R gam
     }
   }
   if (rs == 3) ret = SL > SR ? SL : SR;
-  inverse_rotate<DIM>(flux, n);
+  inverse_rotate<DIM>(flux, fr);
   return ret;
 }
 
@@ -503,13 +671,20 @@ __device__ __forceinline__ R hll_family(R* s1, R* s2, const R* n, R* flux, R gam
 // batched limited runs pass through thousands of elements that sit within
 // FP32 rounding of the limiter's +-1e-3 switches, so that any other rounding of
 // the flux moves their results by up to 2% in single elements.
+template <int DIM, typename R>
+__device__ __forceinline__ R riemann(R* s1, R* s2, const Frame<DIM, R>& fr, R* flux, R gamma, R b, int rs,
+                                     int avg) {
+  if (rs == 0) return rusanov_flux<DIM>(s1, s2, fr, flux, gamma, b);
+  return hll_family<DIM>(s1, s2, fr, flux, gamma, b, rs, avg);
+}
 template <int DIM, typename R, bool PLAIN = false>
 __device__ __forceinline__ R riemann(R* s1, R* s2, const R* n, R* flux, R gamma, R b, int rs,
                                      int avg) {
   constexpr int NEQ = DIM + 2;
   if constexpr (std::is_same<R, float>::value || std::is_same<R, double>::value) {
-    if (rs == 0) return rusanov_flux<DIM>(s1, s2, n, flux, gamma, b);
-    if constexpr (!PLAIN || std::is_same<R, double>::value) return hll_family<DIM>(s1, s2, n, flux, gamma, b, rs, avg);
+    const Frame<DIM, R> fr = make_frame<DIM, R>(n);
+    if (rs == 0) return rusanov_flux<DIM>(s1, s2, fr, flux, gamma, b);
+    if constexpr (!PLAIN || std::is_same<R, double>::value) return hll_family<DIM>(s1, s2, fr, flux, gamma, b, rs, avg);
   }
   if (!state_is_physical_say<DIM>(s1, gamma)) return R(-1);
   if (!state_is_physical_say<DIM>(s2, gamma)) return R(-1);

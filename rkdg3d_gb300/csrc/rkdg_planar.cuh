@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) F[k] = R(0);
     } else {
-      lmax = checked_speed(prm, riemann<DIM>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e1, pb);
+      lmax = checked_speed(prm, riemann<DIM>(s1, s2, make_frame<DIM, R>(n), F, gamma, cov, prm.rs, prm.avg), e1, pb);
     }
     if constexpr (!SPEED) {
       R* out = (R*)prm.fslot + t;
@@ -295,13 +295,15 @@ __global__ void __launch_bounds__(Planar<G, P>::NT)
                        : ((const R*)prm.egeo)[(long long)(r * DIM + d) * ne + e];
     idet = ng ? ng[((long long)(DIM * DIM) * ND + i) * ne + e]
               : ((const R*)prm.egeo)[(long long)(DIM * DIM) * ne + e];
-    R F[NEQ][DIM];
-    lmax = flux_and_speed<DIM>(st, F, gamma, cov);
+    const NodeFlux<DIM, R> N(st, gamma, cov);
+    lmax = N.speed;
 #pragma unroll
-    for (int r = 0; r < DIM; ++r)
+    for (int r = 0; r < DIM; ++r) {
+      R G[NEQ];
+      N.contra(st, adj[r], G);
 #pragma unroll
-      for (int k = 0; k < NEQ; ++k)
-        sG[r][k][sl * NP + i] = adj[r][0] * F[k][0] + adj[r][1] * F[k][1];
+      for (int k = 0; k < NEQ; ++k) sG[r][k][sl * NP + i] = G[k];
+    }
   }
   __syncthreads();
   if (live) {
@@ -406,10 +408,11 @@ __global__ void __launch_bounds__(Planar<G, P>::NT)
       }
     }
   }
+  constexpr bool SQ = std::is_same<R, double>::value;
   if (prm.prob)
-    segmented_max_commit<R>(lmax, live ? pb : -1, prm.pmcs);
+    segmented_max_commit<R, SQ>(lmax, live ? pb : -1, prm.pmcs);
   else
-    block_max_commit<R>(lmax, prm.mcs);
+    block_max_commit<R, SQ>(lmax, prm.mcs);
 }
 
 }  // namespace rkdg
