@@ -263,18 +263,18 @@ struct RhsParams {
   const void* ngeo;
   HexOpsPair hops;      // hexahedra (order <= 2): 1D operators
   // face-pass kernels (planar elements and hexahedra): the faces in the order
-  // of their Elem1 (hexahedra: by normal axis first), flist[f] = (Elem1, Elem2 or -1, local face of Elem1 + 8 *
+  // of their Elem1 (hexahedra: by normal axis first; boundary faces last), flist[f] = (Elem1, Elem2 or -1, local face of Elem1 + 8 *
   // that of Elem2 + 64 * orientation, 0), and each element's faces.
   // Planar: orientation 1 where Elem2 runs through the points backwards,
   // fref[lf][e] = face * 4 + 2 on the Elem2 side + 1 where the points run
   // backwards, fslot the fluxes [neq][nface * nqf].  Hexahedra: orientation =
-  // square_op code from Elem1's to Elem2's tensor indices, fref = face * 2 + 1
-  // on the Elem2 side, fop[lf][e] the code from the element's own indices to
-  // Elem1's (null: all zero), fslot the moments [neq][nface][(p+1)^2].
+  // square_op code from Elem1's to Elem2's tensor indices, fref[e][0..5] = face
+  // * 2 + 1 on the Elem2 side per local face, fref[e][6] the codes from the
+  // element's own indices to Elem1's (three bits a face), fslot the moments
+  // [nface][neq][(p+1)^2].
   int nface;
   const int4* flist;
   const int* fref;
-  const unsigned char* fop;
   const PlanarOpsPair* pops;
 };
 

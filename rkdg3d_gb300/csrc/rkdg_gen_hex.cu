@@ -65,35 +65,36 @@ static cudaError_t launch_hex_faces(const RhsParams& prm, const R* u, const EpiP
   using S = HexFaces<P>;
   if (!prm.flist || !prm.fslot) return cudaErrorInvalidValue;
   const int grid = (prm.nface + S::FB - 1) / S::FB;
-  if (prm.faces_only) {
-    k_face_hex<P, R, true><<<grid, S::NT, 0, st>>>(prm, u);
-    return cudaGetLastError();
+  if (prm.faces_only) {  // rkdg_face_speed: FP64 states only
+    if constexpr (std::is_same<R, double>::value) {
+      k_speed_hex<P><<<grid, S::NT, 0, st>>>(prm, u);
+      return cudaGetLastError();
+    }
+    return cudaErrorInvalidValue;
   }
-  k_face_hex<P, R, false><<<grid, S::NT, 0, st>>>(prm, u);
+  k_face_hex<P, R><<<grid, S::NT, 0, st>>>(prm, u);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_node_hex<P, R><<<(prm.ne + S::EPB - 1) / S::EPB, S::NTN, 0, st>>>(prm, u, ep);
   return cudaGetLastError();
 }
 
-// Defaults (64^3 periodic pulse on a GB300, per RK step): FP32 Q2 -- the
-// face-once tiled kernel (2.39 ms against 3.15 for the fused team kernel);
-// FP32 Q1 -- the fused team kernel (1.39 ms against 1.57 split and 1.42
-// shared-face); FP64 -- face pass and node pass.
+// Default for both orders and precisions: face pass and node pass.  Per RK step
+// on a GB300 in FP32: 64^3 Q2 pulse 2.16 ms against 2.31 with the face-once tiles
+// and 3.15 with the fused team kernel, 64^3 Q1 0.92 ms against 1.49 (team).
 template <>
 cudaError_t launch_rhs_t<5, 1>(int prec, const RhsParams& prm, const void* u, const void* ep,
                                cudaStream_t st) {
   if (prec == 0)
     return launch_hex_faces<1, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st);
-  return launch_hex_team<1, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
+  return launch_hex_faces<1, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
 }
 template <>
 cudaError_t launch_rhs_t<5, 2>(int prec, const RhsParams& prm, const void* u, const void* ep,
                                cudaStream_t st) {
   if (prec == 0)
     return launch_hex_faces<2, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st);
-  if (prm.htile) return launch_hex_tile(2, 1, prm, u, ep, st);
-  return launch_hex_team<2, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
+  return launch_hex_faces<2, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
 }
 
 template cudaError_t launch_limit_t<5, 1>(int, const LimParams&, void*, float*, cudaStream_t);

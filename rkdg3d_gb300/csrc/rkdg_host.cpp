@@ -54,7 +54,6 @@ struct rkdg_ctx {
   int nface = 0, nbface = 0;  // nbface: faces without a second element
   int4* d_flist = nullptr;
   int* d_fref = nullptr;
-  unsigned char* d_fop = nullptr;
   double* d_fcoef = nullptr;  // fluxes / moments of the face-pass kernels
   size_t fcoef_n = 0;
   rkdg::PlanarOpsPair* d_pops = nullptr;
@@ -103,8 +102,8 @@ struct rkdg_ctx {
   std::vector<double> h_eaff;
   float* d_egeo32 = nullptr;
   double* d_wdet = nullptr;
-  unsigned long long* d_mcs = nullptr;  // 8 slots
-  int* d_err = nullptr;                 // 2 ints
+  unsigned long long* d_mcs = nullptr;  // 8 slots, then the error words: one copy reads both
+  int* d_err = nullptr;                 // 2 ints behind the slots
   double* d_means = nullptr;
   double* d_partial = nullptr;
   // scratch state buffers
@@ -115,7 +114,7 @@ struct rkdg_ctx {
   float* d_xh = nullptr;
   float* d_xl = nullptr;
   unsigned long long* h_mcs = nullptr;  // pinned
-  int* h_err = nullptr;                 // pinned
+  int* h_err = nullptr;                 // behind h_mcs
   std::vector<double> h_ehmin;          // per-element GetElementSize(i, 1)
   // batched independent problems
   int nprob = 0;
@@ -221,7 +220,6 @@ void free_mesh(rkdg_ctx* c) {
   c->adj_n = 0;
   dfree(c->d_flist);
   dfree(c->d_fref);
-  dfree(c->d_fop);
   dfree(c->d_fcoef);
   c->fcoef_n = 0;
   dfree(c->d_pops);
@@ -338,7 +336,6 @@ RhsParams rhs_params(rkdg_ctx* c, int prec, int faces_only, int slot) {
   P.nface = c->nface;
   P.flist = c->d_flist;
   P.fref = c->d_fref;
-  P.fop = c->d_fop;
   P.pops = c->d_pops;
   P.hsched = c->d_hsched;
   P.htile = c->d_htile;
@@ -409,11 +406,11 @@ cudaError_t launch_rhs_nc(rkdg_ctx* c, int prec, const RhsParams& P, const void*
 
 // Kernels one right-hand-side launch issues: a face pass and a node pass
 // (the face pass alone for the wave speed), one kernel on FP32 Q1 quads and for
-// FP32 and the selected variants of hexahedra but that of the two passes.
+// the other selectable variants of hexahedra.
 int rhs_kernels(const rkdg_ctx* c, const RhsParams& P) {
   const bool fp64 = P.fgeo == (const void*)c->d_fgeo64;
   if (P.faces_only) return 1;
-  if (c->geom == RKDG_GEOM_CUBE) return c->hex_variant == 3 || (c->hex_variant == 0 && fp64) ? 2 : 1;
+  if (c->geom == RKDG_GEOM_CUBE) return c->hex_variant == 3 || c->hex_variant == 0 ? 2 : 1;
   return c->geom == RKDG_GEOM_SQUARE && c->p == 1 && !fp64 ? 1 : 2;
 }
 
@@ -545,14 +542,12 @@ int square_op_host(int op, int i, int j, int n) {
 }
 
 // Faces of the face-pass kernels in the order of their Elem1, hexahedra by
-// normal axis first (see RhsParams).
-bool face_tables(const rkdg_ctx* c, std::vector<int4>& flist, std::vector<int>& fref,
-                 std::vector<unsigned char>& fop) {
+// normal axis first, those without a second element last (see RhsParams).
+bool face_tables(const rkdg_ctx* c, std::vector<int4>& flist, std::vector<int>& fref) {
   const RefTables& T = c->tab;
   const int ne = c->ne, nfpe = c->nfpe;
   const bool hex = c->geom == RKDG_GEOM_CUBE;
-  fref.assign((size_t)nfpe * ne, 0);
-  if (hex) fop.assign((size_t)nfpe * ne, 0);
+  fref.assign((size_t)(hex ? 8 : nfpe) * ne, 0);
   flist.reserve((size_t)nfpe * ne / 2 + ne / 4 + 16);
   // orientation codes per (lf1, lf2, permutation), filled when first met
   const int n = T.nq1;
@@ -568,45 +563,47 @@ bool face_tables(const rkdg_ctx* c, std::vector<int4>& flist, std::vector<int>& 
       if (ok) inverse[o] = (signed char)v;
     }
   static const int axis[6] = {2, 1, 0, 1, 0, 2};  // of a hexahedron's local faces
-  bool turned = false;
-  for (int ax = 0; ax < (hex ? 3 : 1); ++ax)
-   for (int e = 0; e < ne; ++e)
-    for (int lf = 0; lf < nfpe; ++lf) {
-      if (hex && axis[lf] != ax) continue;
-      const size_t i = (size_t)lf * ne + e;
-      const int e2 = c->h_fnbr[i], fc = c->h_fcode[i];
-      if (e2 >= 0 && ((fc >> 3) & 1)) continue;  // the Elem2 side
-      const int f = (int)flist.size();
-      int4 r = {e, -1, lf, 0};
-      fref[i] = f * (hex ? 2 : 4);
-      if (e2 >= 0) {
-        const int lf2 = fc & 7, pid = fc >> 4;
-        const size_t i2 = (size_t)lf2 * ne + e2;
-        int op = T.perm[pid][0] != 0;
-        if (hex) {
-          signed char& o = code[(lf * 6 + lf2) * RKDG_HEX_MAX_PERM + pid];
-          for (int v = 0; v < 8 && o < 0; ++v) {
-            bool ok = true;
-            for (int q = 0; q < T.nqf && ok; ++q) {
-              const int t1 = T.fab[lf][q];
-              ok = square_op_host(v, t1 % n, t1 / n, n) == T.fab[lf2][T.perm[pid][q]];
+  // pass 0-2: the interior faces of an axis (planar: all); then the others,
+  // which take another way through the kernels
+  for (int pass = hex ? 0 : 2; pass < 4; ++pass)
+    for (int e = 0; e < ne; ++e)
+      for (int lf = 0; lf < nfpe; ++lf) {
+        const size_t i = (size_t)lf * ne + e;
+        const int e2 = c->h_fnbr[i], fc = c->h_fcode[i];
+        if (pass == 3 ? e2 >= 0 : (e2 < 0 || (hex && axis[lf] != pass))) continue;
+        if (e2 >= 0 && ((fc >> 3) & 1)) continue;  // the Elem2 side
+        const int f = (int)flist.size();
+        int4 r = {e, -1, lf, 0};
+        if (hex)
+          fref[(size_t)e * 8 + lf] = f * 2;
+        else
+          fref[i] = f * 4;
+        if (e2 >= 0) {
+          const int lf2 = fc & 7, pid = fc >> 4;
+          const size_t i2 = (size_t)lf2 * ne + e2;
+          int op = T.perm[pid][0] != 0;
+          if (hex) {
+            signed char& o = code[(lf * 6 + lf2) * RKDG_HEX_MAX_PERM + pid];
+            for (int v = 0; v < 8 && o < 0; ++v) {
+              bool ok = true;
+              for (int q = 0; q < T.nqf && ok; ++q) {
+                const int t1 = T.fab[lf][q];
+                ok = square_op_host(v, t1 % n, t1 / n, n) == T.fab[lf2][T.perm[pid][q]];
+              }
+              if (ok) o = (signed char)v;
             }
-            if (ok) o = (signed char)v;
+            if (o < 0) return false;
+            op = o;
+            fref[(size_t)e2 * 8 + lf2] = f * 2 + 1;
+            fref[(size_t)e2 * 8 + 6] |= inverse[op] << (3 * lf2);
+          } else {
+            fref[i2] = f * 4 + 2 + op;
           }
-          if (o < 0) return false;
-          op = o;
-          fref[i2] = f * 2 + 1;
-          fop[i2] = (unsigned char)inverse[op];
-          turned |= op != 0;
-        } else {
-          fref[i2] = f * 4 + 2 + op;
+          r.y = e2;
+          r.z = lf + 8 * lf2 + 64 * op;
         }
-        r.y = e2;
-        r.z = lf + 8 * lf2 + 64 * op;
+        flist.push_back(r);
       }
-      flist.push_back(r);
-    }
-  if (!turned) fop.clear();  // every face's two elements index it alike
   return true;
 }
 
@@ -674,11 +671,12 @@ LimParams lim_params_for(rkdg_ctx* c, bool batch) {
   return L;
 }
 
-cudaError_t zero_slot(rkdg_ctx* c, int i, bool batch) {
+// Zero n wave-speed slots from slot i.
+cudaError_t zero_slots(rkdg_ctx* c, int i, int n, bool batch) {
   if (batch)
     return cudaMemsetAsync(c->d_pmcs + (size_t)i * c->nprob, 0,
-                           (size_t)c->nprob * sizeof(unsigned long long), c->stream);
-  return cudaMemsetAsync(c->d_mcs + i, 0, sizeof(unsigned long long), c->stream);
+                           (size_t)n * c->nprob * sizeof(unsigned long long), c->stream);
+  return cudaMemsetAsync(c->d_mcs + i, 0, n * sizeof(unsigned long long), c->stream);
 }
 
 // Enqueue one Runge-Kutta step on the FP64 state x (no host synchronisation).
@@ -701,7 +699,7 @@ int enqueue_step64(rkdg_ctx* c, double* x, double dt, bool batch = false) {
     } else {
       in = c->d_y64[i % 2];
     }
-    CUDA_TRY(c, zero_slot(c, i, batch));
+    if (i == 0) CUDA_TRY(c, zero_slots(c, 0, s, batch));
     EpiParams<double> ep;
     std::memset(&ep, 0, sizeof ep);
     ep.mode = 1;
@@ -769,7 +767,7 @@ int enqueue_step32(rkdg_ctx* c, double dt, bool batch = false) {
     } else {
       in = c->d_y32[i % 2];
     }
-    CUDA_TRY(c, zero_slot(c, i, batch));
+    if (i == 0) CUDA_TRY(c, zero_slots(c, 0, s, batch));
     EpiParams<float> ep;
     std::memset(&ep, 0, sizeof ep);
     ep.mode = 1;
@@ -827,16 +825,14 @@ int enqueue_step32(rkdg_ctx* c, double dt, bool batch = false) {
 }
 
 int read_mcs(rkdg_ctx* c, int slot, double* out) {
-  CUDA_TRY(c, cudaMemcpyAsync(c->h_mcs, c->d_mcs + slot, sizeof(unsigned long long),
+  CUDA_TRY(c, cudaMemcpyAsync(c->h_mcs, c->d_mcs, 9 * sizeof(unsigned long long),
                               cudaMemcpyDeviceToHost, c->stream));
-  CUDA_TRY(c, cudaMemcpyAsync(c->h_err, c->d_err, 2 * sizeof(int), cudaMemcpyDeviceToHost,
-                              c->stream));
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   int st = check_device_error(c);
   if (st) return st;
   if (out) {
     double v;
-    unsigned long long bits = c->h_mcs[0];
+    unsigned long long bits = c->h_mcs[slot];
     std::memcpy(&v, &bits, sizeof v);
     *out = v;
   }
@@ -914,14 +910,14 @@ int rkdg_create(rkdg_ctx** out, int device) {
   c->device = device;
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc((void**)&c->d_mcs, 8 * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc((void**)&c->d_err, 2 * sizeof(int)) != cudaSuccess ||
-      cudaMallocHost((void**)&c->h_mcs, 8 * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMallocHost((void**)&c->h_err, 2 * sizeof(int)) != cudaSuccess ||
-      cudaMemset(c->d_err, 0, 2 * sizeof(int)) != cudaSuccess) {
+      cudaMalloc((void**)&c->d_mcs, 9 * sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMallocHost((void**)&c->h_mcs, 9 * sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMemset(c->d_mcs, 0, 9 * sizeof(unsigned long long)) != cudaSuccess) {
     delete c;
     return RKDG_ERR_CUDA;
   }
+  c->d_err = reinterpret_cast<int*>(c->d_mcs + 8);
+  c->h_err = reinterpret_cast<int*>(c->h_mcs + 8);
   c->own_stream = true;
   *out = c;
   return RKDG_OK;
@@ -933,9 +929,7 @@ int rkdg_destroy(rkdg_ctx* c) {
   cudaStreamSynchronize(c->stream);
   free_mesh(c);
   dfree(c->d_mcs);
-  dfree(c->d_err);
   if (c->h_mcs) cudaFreeHost(c->h_mcs);
-  if (c->h_err) cudaFreeHost(c->h_err);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return RKDG_OK;
@@ -1526,8 +1520,7 @@ int rkdg_upload_mesh(rkdg_ctx* c, const rkdg_mesh_desc* m) {
   {
     std::vector<int4> flist;
     std::vector<int> fref;
-    std::vector<unsigned char> fop;
-    if (!face_tables(c, flist, fref, fop))
+    if (!face_tables(c, flist, fref))
       return fail(c, RKDG_ERR_INVALID, "face points of two hexahedra do not match");
     c->nface = (int)flist.size();
     c->nbface = 0;
@@ -1536,10 +1529,6 @@ int rkdg_upload_mesh(rkdg_ctx* c, const rkdg_mesh_desc* m) {
     CUDA_TRY(c, dalloc(c->d_fref, fref.size()));
     CUDA_TRY(c, cudaMemcpy(c->d_flist, flist.data(), flist.size() * sizeof(int4), cudaMemcpyHostToDevice));
     CUDA_TRY(c, cudaMemcpy(c->d_fref, fref.data(), fref.size() * sizeof(int), cudaMemcpyHostToDevice));
-    if (!fop.empty()) {
-      CUDA_TRY(c, dalloc(c->d_fop, fop.size()));
-      CUDA_TRY(c, cudaMemcpy(c->d_fop, fop.data(), fop.size(), cudaMemcpyHostToDevice));
-    }
     if (dim == 2) {
       rkdg::PlanarOpsPair ops;
       planar_tables(c, ops);
@@ -1842,7 +1831,7 @@ int rkdg_batch_run(rkdg_ctx* c, double* x, double t_end, double cfl, double dt0,
       CUDA_TRY(c, rkdg::launch_limit(c->geom, c->p, 0, L, x, nullptr, c->stream));
       c->launches += 2;
     }
-    CUDA_TRY(c, zero_slot(c, c->s - 1, true));
+    CUDA_TRY(c, zero_slots(c, c->s - 1, 1, true));
     EpiParams<double> ep;
     std::memset(&ep, 0, sizeof ep);
     RhsParams P = rhs_params(c, 0, 1, 0);

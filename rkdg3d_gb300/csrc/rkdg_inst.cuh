@@ -41,7 +41,10 @@ cudaError_t launch_planar(const RhsParams& prm, const R* u, const EpiParams<R>& 
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   using S = Planar<G, P>;
-  k_node_planar<G, P, R><<<(prm.ne + S::EPB - 1) / S::EPB, S::NT, 0, st>>>(prm, u, ep);
+  if (prm.ne < 152 * S::EPB)
+    k_node_planar<G, P, R, S::SMALL><<<(prm.ne + S::SMALL - 1) / S::SMALL, S::threads(S::SMALL), 0, st>>>(prm, u, ep);
+  else
+    k_node_planar<G, P, R, S::EPB><<<(prm.ne + S::EPB - 1) / S::EPB, S::NT, 0, st>>>(prm, u, ep);
   return cudaGetLastError();
 }
 

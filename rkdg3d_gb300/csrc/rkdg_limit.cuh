@@ -91,9 +91,13 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
   constexpr int DIM = E::DIM, ND = E::ND, NEQ = E::NEQ, NFPE = E::NFPE, NQL = E::NQL, NV = E::NV;
   constexpr int L = T::L, NPT = T::NPT, NDP = T::NDP;
   constexpr bool F32 = std::is_same<R, float>::value;
-  // small float elements: the factor is applied nd times as the reference
-  // does (their limited runs amplify another rounding, see riemann())
-  constexpr bool REPEAT = F32 && ND <= 4;
+  // float states of hexahedra and of small planar elements: the factor is
+  // applied nd times as the reference does (their limited runs amplify another
+  // rounding, see riemann()); a float pair's power rounds far below that
+  constexpr bool REPEAT = F32 && (ND <= 4 || (G == 5 && !DS));
+  // the means' low parts: FP64 hexahedra (on 200x4 quads the extra pass over
+  // the values is 6% of a step, and a planar mesh's means change more per step)
+  constexpr bool LOW = !F32 && G == 5;
   using MeanT = typename std::conditional<F32, float2, double>::type;
   using IndT = typename std::conditional<F32, float, double>::type;
   const RefTables* tab = prm.tab;
@@ -360,7 +364,7 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
       }
       __syncthreads();
     }
-    if constexpr (!F32) {
+    if constexpr (LOW) {
       // what rounding the mean to FP64 left out: with it the limited values
       // average to the unrounded mean, and a limited run's rounding does not
       // accumulate one bit of every mean per stage
@@ -383,7 +387,7 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
         R& v = sU[(k * EPB + s) * NDP + j];
         const MeanT um = sM[k * EPB + s];
         if constexpr (!F32) {
-          const double l = sL[k * EPB + s], d = v - um;
+          const double l = LOW ? sL[k * EPB + s] : 0.0, d = v - um;
           v = um + (l + sMr[s] * (d - l));
         } else {
           const float2 m = reinterpret_cast<float2*>(sMr)[s];

@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(kNcFaceThreads) k_nc_face(const __grid_constan
     const R gamma = (R)(pb >= 0 ? prm.pgamma[pb] : prm.gamma);
     const R cov = (R)(pb >= 0 ? prm.pcov[pb] : prm.covolume);
     R F[NEQ];
-    lmax = checked_speed(prm, riemann<DIM>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e1, pb);
+    lmax = checked_speed(prm, riemann<DIM, R, true>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e1, pb);
     const R wq = (R)T->wf[q];
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) sF[lf][q][k] = (F[k] * wq) * jac;

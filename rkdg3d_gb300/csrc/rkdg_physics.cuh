@@ -324,11 +324,95 @@ __device__ __forceinline__ R rusanov_flux(const R* s1, const R* s2, const Frame<
   return maxE;
 }
 
+// The FP32 forms of hexahedra and Q1 quads (riemann() with PLAIN).
+//
+// FP32 pointwise state quantities with one reciprocal of the density and one
+// of the covolume factor: r = 1/rho, q = 1/(1 - rho b), the pressure (FP64
+// where E - |m|^2/(2 rho) cancels, as pressure() does) and |u| + c.  Returns
+// false where StateIsPhysicalSay fails (rho < 0, E <= 0, perfect-gas p <= 0,
+// NaN).  Same quantities as the double path, rounded in a different order.
+template <int DIM>
+__device__ __forceinline__ bool state_f32(const float* s, float gamma, float b, float& r, float& q,
+                                          float& p, float& speed) {
+  const float den = s[0], E = s[1 + DIM];
+  if (!(den >= 0.0f) || !(E > 0.0f)) return false;
+  r = __fdividef(1.0f, den);
+  float m2 = 0.0f;
+#pragma unroll
+  for (int d = 0; d < DIM; d++) m2 = fmaf(s[1 + d], s[1 + d], m2);
+  const float v2 = m2 * r;  // |m|^2 / rho
+  const float ie = E - 0.5f * v2;
+  if (!((gamma - 1.0f) * ie > 0.0f)) return false;
+  q = __fdividef(1.0f, 1.0f - den * b);
+  if (fabsf(ie) < 1e-3f * fabsf(E)) {
+    double m2d = 0.0;
+#pragma unroll
+    for (int d = 0; d < DIM; d++) m2d += (double)s[1 + d] * (double)s[1 + d];
+    p = (float)(((double)gamma - 1.0) * ((double)E - 0.5 * m2d / (double)den) /
+                (1.0 - (double)den * (double)b));
+  } else {
+    p = (gamma - 1.0f) * ie * q;
+  }
+  speed = fsq(v2 * r) + fsq(gamma * p * r * q);
+  return true;
+}
+
+// FP32 Rusanov flux (rs_rusanov.cpp:6-40) on unrotated states, built on
+// state_f32.  Returns the wave speed, or -1 for a non-physical state.
+template <int DIM>
+__device__ __forceinline__ float rusanov_f32(const float* s1, const float* s2, const float* n,
+                                             float* flux, float gamma, float b) {
+  constexpr int NEQ = DIM + 2;
+  float r1, q1, p1, e1, r2, q2, p2, e2;
+  if (!state_f32<DIM>(s1, gamma, b, r1, q1, p1, e1)) return -1.0f;
+  if (!state_f32<DIM>(s2, gamma, b, r2, q2, p2, e2)) return -1.0f;
+  const float maxE = e1 > e2 ? e1 : e2;
+  float d1 = 0.0f, d2 = 0.0f, nn = 0.0f;
+#pragma unroll
+  for (int d = 0; d < DIM; d++) {
+    d1 = fmaf(s1[1 + d], n[d], d1);
+    d2 = fmaf(s2[1 + d], n[d], d2);
+    nn = fmaf(n[d], n[d], nn);
+  }
+  const float h = 0.5f * rsqrtf(nn), a = 0.5f * maxE;
+  const float u1 = d1 * r1, u2 = d2 * r2;
+  flux[0] = h * (d1 + d2) - a * (s2[0] - s1[0]);
+#pragma unroll
+  for (int d = 0; d < DIM; d++)
+    flux[1 + d] = h * (fmaf(u1, s1[1 + d], p1 * n[d]) + fmaf(u2, s2[1 + d], p2 * n[d])) -
+                  a * (s2[1 + d] - s1[1 + d]);
+  flux[NEQ - 1] = h * (u1 * (s1[NEQ - 1] + p1) + u2 * (s2[NEQ - 1] + p2)) -
+                  a * (s2[NEQ - 1] - s1[NEQ - 1]);
+  return maxE;
+}
+
 // ComputeFlux (physics.cpp:143-168): F[k][d]; also returns |u|+c at the node
 // (FE_Evolution::GetFlux, fe_evolution.cpp:219-245).
 template <int DIM, typename R>
 __device__ __forceinline__ R flux_and_speed(const R* s, R F[DIM + 2][DIM], R gamma, R b) {
-  if constexpr (std::is_same<R, float>::value || std::is_same<R, double>::value) {
+  if constexpr (std::is_same<R, float>::value) {
+    float r, q, p, speed;
+    if (!state_f32<DIM>(s, gamma, b, r, q, p, speed)) {
+      // non-physical node: same arithmetic as the double path
+      r = __fdividef(1.0f, s[0]);
+      p = pressure<DIM>(s, gamma, b);
+      float m2 = 0.0f;
+#pragma unroll
+      for (int d = 0; d < DIM; d++) m2 += s[1 + d] * s[1 + d];
+      speed = fsq(m2 * r * r) + fsq(fdv(gamma * p * r, 1.0f - s[0] * b));
+    }
+#pragma unroll
+    for (int d = 0; d < DIM; d++) {
+      const float ud = s[1 + d] * r;
+      F[0][d] = s[1 + d];
+#pragma unroll
+      for (int i = 0; i < DIM; i++) F[1 + i][d] = s[1 + i] * ud;
+      F[1 + d][d] += p;
+      F[1 + DIM][d] = (s[1 + DIM] + p) * ud;
+    }
+    return speed;
+  }
+  if constexpr (std::is_same<R, double>::value) {
     R r, q, p, u2;
     if (!eos_state<DIM>(s, gamma, b, r, q, p, u2)) {
       // non-physical node: the same quantities without the checks
@@ -449,9 +533,8 @@ __device__ __forceinline__ void rotate(R* s, const R* n) {
     const R sp = n[2];
     const R cp = fsq(R(1) - sp * sp);
     const bool ok = fabs(cp) > R(1e-6);
-    const R ic = fdv(R(1), cp);
-    const R st = ok ? n[1] * ic : R(1);
-    const R ct = ok ? n[0] * ic : R(0);
+    const R st = ok ? fdv(n[1], cp) : R(1);
+    const R ct = ok ? fdv(n[0], cp) : R(0);
     const R mx = cp * ct * m[0] + cp * st * m[1] + sp * m[2];
     const R my = -st * m[0] + ct * m[1];
     const R mz = -sp * ct * m[0] - sp * st * m[1] + cp * m[2];
@@ -472,9 +555,8 @@ __device__ __forceinline__ void inverse_rotate(R* s, const R* n) {
     const R sp = n[2];
     const R cp = fsq(R(1) - sp * sp);
     const bool ok = fabs(cp) > R(1e-6);
-    const R ic = fdv(R(1), cp);
-    const R st = ok ? n[1] * ic : R(1);
-    const R ct = ok ? n[0] * ic : R(0);
+    const R st = ok ? fdv(n[1], cp) : R(1);
+    const R ct = ok ? fdv(n[0], cp) : R(0);
     const R mx = cp * ct * m[0] - st * m[1] - sp * ct * m[2];
     const R my = cp * st * m[0] + ct * m[1] - sp * st * m[2];
     const R mz = sp * m[0] + cp * m[2];
@@ -667,10 +749,11 @@ __device__ __forceinline__ R hll_family(R* s1, R* s2, const Frame<DIM, R>& fr, R
 // reference does through const_cast); n is the unit normal from side 1 to
 // side 2.  Returns the solver's wave speed, or -1 for a non-physical state.
 // float and double take the forms above; dual numbers the plain restatement
-// below, and so does float where PLAIN is set: the FP32 Q1 quads, whose
-// batched limited runs pass through thousands of elements that sit within
-// FP32 rounding of the limiter's +-1e-3 switches, so that any other rounding of
-// the flux moves their results by up to 2% in single elements.
+// below, and so does float where PLAIN is set: hexahedra and Q1 quads.  Their
+// limited runs pass through elements that sit within FP32 rounding of the
+// limiter's switches (the +-1e-3 thresholds, the Michalak function's step at 1),
+// where any other rounding of a flux moves single elements by up to 5%; so the
+// FP32 arithmetic of these elements is kept to the bit.
 template <int DIM, typename R>
 __device__ __forceinline__ R riemann(R* s1, R* s2, const Frame<DIM, R>& fr, R* flux, R gamma, R b, int rs,
                                      int avg) {
@@ -682,6 +765,8 @@ __device__ __forceinline__ R riemann(R* s1, R* s2, const R* n, R* flux, R gamma,
                                      int avg) {
   constexpr int NEQ = DIM + 2;
   if constexpr (std::is_same<R, float>::value || std::is_same<R, double>::value) {
+    if constexpr (PLAIN && std::is_same<R, float>::value)
+      if (rs == 0) return rusanov_f32<DIM>(s1, s2, n, flux, gamma, b);
     const Frame<DIM, R> fr = make_frame<DIM, R>(n);
     if (rs == 0) return rusanov_flux<DIM>(s1, s2, fr, flux, gamma, b);
     if constexpr (!PLAIN || std::is_same<R, double>::value) return hll_family<DIM>(s1, s2, fr, flux, gamma, b, rs, avg);

@@ -45,10 +45,13 @@ template <int G, int P>
 struct Planar {
   using E = El<G, P>;
   static constexpr int N1 = P + 1;
-  // elements per CTA of the node pass: whole warps (the wave-speed reductions)
+  // elements per CTA of the node pass; SMALL: one or two warps, for meshes that
+  // would leave SMs without a CTA
   static constexpr int EPB = G == 3 ? (P == 3 ? 12 : 32) : (P == 1 ? 64 : 32);
-  static constexpr int NT = EPB * E::ND;
-  static_assert(NT % 32 == 0, "whole warps");
+  static constexpr int SMALL = G == 3 ? (P == 1 ? 8 : (P == 2 ? 7 : 4)) : (P == 1 ? 10 : 5);
+  // threads of n elements: whole warps (the wave-speed reductions)
+  __host__ __device__ static constexpr int threads(int n) { return (n * E::ND + 31) / 32 * 32; }
+  static constexpr int NT = threads(EPB);
 };
 
 // Node jn (from the face point inwards along the normal axis) behind point q
@@ -97,6 +100,7 @@ __global__ void __launch_bounds__(128)
     }
   }
   if (live) {
+    bool skip = false;
     const int lf1 = face.z & 7;
     const R* fg = (const R*)prm.fgeo;
     R n[DIM];
@@ -131,9 +135,46 @@ __global__ void __launch_bounds__(128)
       }
     };
     R s1[NEQ], s2[NEQ], F[NEQ];
-    trace(e1, lf1, q, s1);
+    if constexpr (SPEED) {
+      // estimated in FP32, evaluated in FP64 only where the point could hold
+      // the maximum (see speed_state_margin)
+      if (face.y >= 0) {
+        float a1[NEQ], a2[NEQ], Ff[NEQ], nf[DIM], top[2][NEQ];
+        auto est = [&](int e, int lf, int qq, float* s, float* tp) {
+          const R* ue = u + (long long)e * ND;
+          constexpr int NT = G == 3 ? N1 : ND;  // terms of the trace
+          const int sd = quad_face_side(lf), i0 = G == 3 ? quad_face_node<N1>(lf, qq, 0) : 0;
+          const int st = G == 3 && !(lf & 1) ? N1 : 1;
+          const float* B = prm.pops->f.b + (lf * NQF + qq) * ND;
+#pragma unroll
+          for (int k = 0; k < NEQ; ++k) s[k] = tp[k] = 0.0f;
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            const float w = G == 3 ? (sd ? prm.pops->f.lend[N1 + j] : prm.pops->f.lend[j]) : B[j];
+#pragma unroll
+            for (int k = 0; k < NEQ; ++k) {
+              const float x = cut_f32((double)ue[k * NDa + i0 + j * st]);
+              s[k] += w * x;
+              tp[k] = fmaxf(tp[k], fabsf(x));
+            }
+          }
+        };
+        est(e1, lf1, q, a1, top[0]);
+        est(face.y, (face.z >> 3) & 7, (face.z >> 6) ? NQF - 1 - q : q, a2, top[1]);
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) nf[c] = (float)n[c];
+        const float g = (float)gamma, b = (float)cov;
+        const float mg = fmaxf(speed_state_margin(a1, DIM, top[0], 1, b), speed_state_margin(a2, DIM, top[1], 1, b));
+        if (mg < 1e8f && speed_below(riemann<DIM>(a1, a2, make_frame<DIM, float>(nf), Ff, g, b, prm.rs, prm.avg), mg,
+                                     prm.prob ? prm.pmcs + pb : prm.mcs, prm.rs, prm.avg))
+          skip = true;
+      }
+    }
+    if (!skip) trace(e1, lf1, q, s1);
     bool none = false;
-    if (face.y >= 0) {
+    if (skip) {
+      none = true;
+    } else if (face.y >= 0) {
       trace(face.y, (face.z >> 3) & 7, (face.z >> 6) ? NQF - 1 - q : q, s2);
     } else {
       const int nb = prm.fnbr[lf1 * ne + e1];
@@ -225,14 +266,14 @@ __device__ __forceinline__ void epi_node(const EpiParams<R>& ep, long long idx, 
   }
 }
 
-template <int G, int P, typename R>
-__global__ void __launch_bounds__(Planar<G, P>::NT)
+template <int G, int P, typename R, int EPB>
+__global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
     k_node_planar(const __grid_constant__ RhsParams prm, const R* __restrict__ u,
                   const __grid_constant__ EpiParams<R> ep) {
   using E = El<G, P>;
   using S = Planar<G, P>;
   constexpr int DIM = 2, ND = E::ND, NEQ = E::NEQ, NFPE = E::NFPE, NQF = E::NQF, N1 = P + 1;
-  constexpr int EPB = S::EPB, NT = S::NT;
+  constexpr int NT = S::threads(EPB);
   constexpr int NP = ND | 1;  // odd element stride in shared memory
   __shared__ R sG[DIM][NEQ][EPB * NP];
   // triangles: MD_r[i][m] and MB[i][lf][q], node i fastest; quadrilaterals:
@@ -248,12 +289,12 @@ __global__ void __launch_bounds__(Planar<G, P>::NT)
   for (int t = tid; t < (G == 2 ? DIM * ND * ND : N1 * N1); t += NT) sMD[t] = H.md[t];
   for (int t = tid; t < (G == 2 ? NFPE * NQF * ND : 2 * N1); t += NT) sMB[t] = H.mb[t];
   R gamma = (R)prm.gamma, cov = (R)prm.covolume;
-  bool live = e < ne;
+  bool live = sl < EPB && e < ne;
   double dts = 1.0;
   float2 dts2 = make_float2(1.0f, 0.0f);
   if (prm.act_cum) {
     const int na = *prm.act_n;
-    live = e < prm.act_cum[na];
+    live = sl < EPB && e < prm.act_cum[na];
     if (live) e = active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, pb);
   }
   if (live && prm.prob) {
@@ -381,7 +422,7 @@ __global__ void __launch_bounds__(Planar<G, P>::NT)
   if (need_means) {
     // cell means, one (element, equation) per thread and round
     __shared__ int sE[EPB];
-    if (i == 0) sE[sl] = live ? e : -1;
+    if (i == 0 && sl < EPB) sE[sl] = live ? e : -1;
     __syncthreads();
     for (int t = tid; t < EPB * NEQ; t += NT) {
       const int k = t / EPB, s = t - k * EPB, em = sE[s];
