@@ -137,7 +137,8 @@ struct HexOpsPair {
 
 // Operators of the planar (triangle, quadrilateral) kernels, in device memory.
 // Quadrilaterals use the sparse 1D forms: lend (basis at 0
-// and 1), md[i][m] = d1[i][m] / w_i and mb[side][i] = lend[side][i] / w_i.
+// and 1), md[i][m] = d1[i][m] / w_i and mb[side][i] = lend[side][i] / w_i
+// (and of order 1 the traces b).
 // Triangles the dense ones: b[lf][q][j] traces, md[r][m][i] = (M^-1 D_r)[i][m]
 // and mb[lf][q][i] = (M^-1)[i][:] . B[lf][q][:] w_q.
 template <typename R>
@@ -146,6 +147,10 @@ struct PlanarOps {
   R md[72];
   R mb[54];
   R lend[8];
+  R wf[4];   // face-rule weights
+  // elements of at most four nodes, the dense operators of the element pass:
+  // eb[lf][q][j] traces (triangles: times w_q), ed[r][j][m] = D_r, em = M^-1
+  R eb[32], ed[32], em[16];
   R wm[16];  // cell-mean weights
 };
 struct PlanarOpsPair {
@@ -263,8 +268,9 @@ struct RhsParams {
   const void* ngeo;
   HexOpsPair hops;      // hexahedra (order <= 2): 1D operators
   // face-pass kernels (planar elements and hexahedra): the faces in the order
-  // of their Elem1 (hexahedra: by normal axis first; boundary faces last), flist[f] = (Elem1, Elem2 or -1, local face of Elem1 + 8 *
-  // that of Elem2 + 64 * orientation, 0), and each element's faces.
+  // of their Elem1 (hexahedra: by normal axis first; boundary faces last), flist[f] = (Elem1, Elem2 or
+  // -1, local face of Elem1 + 8 * that of Elem2 + 64 * orientation, problem of a
+  // batch), and each element's faces.
   // Planar: orientation 1 where Elem2 runs through the points backwards,
   // fref[lf][e] = face * 4 + 2 on the Elem2 side + 1 where the points run
   // backwards, fslot the fluxes [neq][nface * nqf].  Hexahedra: orientation =

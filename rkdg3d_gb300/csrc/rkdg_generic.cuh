@@ -210,9 +210,14 @@ __device__ __forceinline__ void segmented_max_commit(R v, int pb, unsigned long 
 }
 
 // Batched problems with a map of the active work: the i-th element of the
-// active problems (in problem order), and its problem pb.
+// active problems (in problem order), and its problem pb.  While every problem
+// is active the map is the identity: one load instead of a chain of six to nine.
 __device__ __forceinline__ int active_element(const int* cum, const int* pid, const int* poff, int na,
-                                              int i, int& pb) {
+                                              int i, int ne, const int* prob, int& pb) {
+  if (cum[na] == ne) {
+    pb = prob[i];
+    return i;
+  }
   int lo = 0, hi = na;  // cum[lo] <= i < cum[lo + 1]
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -357,37 +362,30 @@ __device__ __forceinline__ void epilogue(const EpiParams<R>& ep, long long base_
   }
 }
 
-// ---- right-hand side --------------------------------------------------------
-// One thread per element, for the FP32 Q1 quads (the other planar elements run
-// rkdg_planar.cuh): their flux is rounded as it always was, see riemann().
+// ---- element pass of the planar right-hand side --------------------------------
+// One thread per element, for FP32 elements of at most 16 values: the faces'
+// fluxes come from the face pass (rkdg_planar.cuh), the element's own rows are
+// loaded once.  Q1 quads keep the arithmetic and the order of the sums of a kernel
+// that evaluated its faces itself, see riemann().
 template <int G, int P, typename R>
 __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>::ND>(),
                                   generic_min_blocks<R, El<G, P>::NEQ * El<G, P>::ND, false>())
-    k_rhs_generic(const RhsParams prm, const R* __restrict__ u, const EpiParams<R> ep) {
+    k_elem_planar(const __grid_constant__ RhsParams prm, const R* __restrict__ u,
+                  const __grid_constant__ EpiParams<R> ep) {
   using E = El<G, P>;
   constexpr int DIM = E::DIM, ND = E::ND, NEQ = E::NEQ, NFPE = E::NFPE, NQF = E::NQF;
   __shared__ R sB[NFPE][NQF][ND];
   __shared__ R sD[DIM][ND][ND];
   __shared__ R sMinv[ND][ND];
-  __shared__ R sW[NQF];
   __shared__ R sWm[ND];
-  __shared__ unsigned char sPerm[RKDG_MAX_PERM][NQF];
   const RefTables* T = prm.tab;
   // batched problems with a map of the active work: CTAs past it are idle
   if (prm.act_cum && (int)(blockIdx.x * blockDim.x) >= prm.act_cum[*prm.act_n]) return;
-  for (int t = threadIdx.x; t < NFPE * NQF * ND; t += blockDim.x) {
-    const int s = t % ND, q = (t / ND) % NQF, lf = t / (ND * NQF);
-    sB[lf][q][s] = (R)T->B[lf][q][s];
-  }
-  for (int t = threadIdx.x; t < DIM * ND * ND; t += blockDim.x) {
-    const int m = t % ND, j = (t / ND) % ND, r = t / (ND * ND);
-    sD[r][j][m] = (R)T->D[r][j][m];
-  }
-  for (int t = threadIdx.x; t < ND * ND; t += blockDim.x) sMinv[t / ND][t % ND] = (R)T->Minv[t / ND][t % ND];
-  for (int t = threadIdx.x; t < NQF; t += blockDim.x) sW[t] = (R)T->wf[t];
-  for (int t = threadIdx.x; t < ND; t += blockDim.x) sWm[t] = (R)T->wmean[t];
-  for (int t = threadIdx.x; t < RKDG_MAX_PERM * NQF; t += blockDim.x)
-    sPerm[t / NQF][t % NQF] = (unsigned char)T->perm[t / NQF][t % NQF];
+  const PlanarOps<R>& H = prm.pops->f;
+  for (int t = threadIdx.x; t < NFPE * NQF * ND; t += blockDim.x) (&sB[0][0][0])[t] = H.eb[t];
+  for (int t = threadIdx.x; t < DIM * ND * ND; t += blockDim.x) (&sD[0][0][0])[t] = H.ed[t];
+  for (int t = threadIdx.x; t < ND * ND; t += blockDim.x) (&sMinv[0][0])[t] = H.em[t];
+  for (int t = threadIdx.x; t < ND; t += blockDim.x) sWm[t] = H.wm[t];
   __syncthreads();
 
   const int ne = prm.ne;
@@ -402,7 +400,7 @@ __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>:
   if (prm.act_cum) {
     const int na = *prm.act_n;
     live = e < prm.act_cum[na];
-    if (live) e = active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, pb);
+    if (live) e = active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, prm.ne, prm.prob, pb);
   }
   if (live && prm.prob) {
     if (!prm.act_cum) pb = prm.prob[e];
@@ -430,75 +428,31 @@ __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>:
     for (int k = 0; k < NEQ; ++k)
 #pragma unroll
       for (int s = 0; s < ND; ++s) acc[k][s] = R(0);
-    // the element's own rows are loaded once, with vector loads, for its faces
-    // and volume term, and each neighbour's rows once per face
     R own[NEQ][ND];
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) ld_row<ND>(u + k * NDa + (long long)e * ND, own[k]);
-    const R* fg = (const R*)prm.fgeo;
+    const long long nf = (long long)prm.nface * NQF;
+#pragma unroll
     for (int lf = 0; lf < NFPE; ++lf) {
-      const int nb = prm.fnbr[lf * ne + e];
-      if (nb == -1) continue;
-      const int code = prm.fcode[lf * ne + e];
-      R n[DIM];
+      const int ref = prm.fref[lf * ne + e];
+      const R* fx = (const R*)prm.fslot + (long long)(ref >> 2) * NQF;
+      const R sg = (ref & 2) ? R(1) : R(-1);
+      R fl[NEQ][NQF];
 #pragma unroll
-      for (int c = 0; c < DIM; ++c) n[c] = fg[(long long)(lf * (DIM + 1) + c) * ne + e];
-      const R jac = fg[(long long)(lf * (DIM + 1) + DIM) * ne + e];
-      const int side = (code >> 3) & 1, lfo = code & 7, pid = code >> 4;
-      // sw: this element is side 2 of the face (the trace order of the
-      // Riemann solver), as in the general path below
-      const bool sw = nb >= 0 && side;
-      R nbr[NEQ][ND];
-      if (nb >= 0) {
+      for (int k = 0; k < NEQ; ++k) ld_row<NQF>(fx + k * nf, fl[k]);
+      // Elem1's points in order; this element may run through them backwards
 #pragma unroll
-        for (int k = 0; k < NEQ; ++k) ld_row<ND>(u + k * NDa + (long long)nb * ND, nbr[k]);
-      }
-      const R sg = side ? R(1) : R(-1);
       for (int q = 0; q < NQF; ++q) {
-        const int q2 = sPerm[pid][q];
-        R to[NEQ], tn[NEQ], s1[NEQ], s2[NEQ];
-        const R* Bw = sB[lf][sw ? q2 : q];
+        const R* Bo = sB[lf][(ref & 1) ? NQF - 1 - q : q];
 #pragma unroll
         for (int k = 0; k < NEQ; ++k) {
-          R v = R(0);
-#pragma unroll
-          for (int j = 0; j < ND; ++j) v += own[k][j] * Bw[j];
-          to[k] = v;
-        }
-        if (nb >= 0) {
-          const R* Bn = sB[lfo][sw ? q : q2];
-#pragma unroll
-          for (int k = 0; k < NEQ; ++k) {
-            R v = R(0);
-#pragma unroll
-            for (int j = 0; j < ND; ++j) v += nbr[k][j] * Bn[j];
-            tn[k] = v;
-          }
-#pragma unroll
-          for (int k = 0; k < NEQ; ++k) {
-            s1[k] = sw ? tn[k] : to[k];
-            s2[k] = sw ? to[k] : tn[k];
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < NEQ; ++k) s1[k] = to[k];
-          const BCSlot& bc = prm.bc[-2 - nb];
-          right_state<DIM>(bc.type, bc.state, s1, s2, n, gamma, cov, (decltype(gamma))prm.rgas);
-        }
-        R F[NEQ];
-        const R sp = checked_speed(prm, riemann<DIM, R, true>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e, pb);
-        lmax = fmax(lmax, sp);
-        const R* Bo = sB[lf][side ? q2 : q];
-        const R wq = sW[q];
-#pragma unroll
-        for (int k = 0; k < NEQ; ++k) {
-          const R t = sg * (F[k] * wq) * jac;
+          const R t = sg * fl[k][q];
 #pragma unroll
           for (int j = 0; j < ND; ++j) acc[k][j] += t * Bo[j];
         }
       }
     }
-    if (!prm.faces_only) {
+    {
       const R* eg = (const R*)prm.egeo;
       const R* ng = (const R*)prm.ngeo;  // per-node geometry (bilinear quads) or null
       R adj[DIM][DIM];
@@ -790,7 +744,7 @@ __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>:
   if (prm.act_cum) {  // batched problems: the i-th element of the active ones
     const int na = *prm.act_n;
     if (e >= prm.act_cum[na]) return;
-    e = active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, pmap);
+    e = active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, prm.ne, prm.prob, pmap);
   }
   if (e >= prm.ne) return;
   if (prm.prob && !prm.pactive[prm.act_cum ? pmap : prm.prob[e]]) return;

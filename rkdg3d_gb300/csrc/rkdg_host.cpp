@@ -405,13 +405,12 @@ cudaError_t launch_rhs_nc(rkdg_ctx* c, int prec, const RhsParams& P, const void*
 }
 
 // Kernels one right-hand-side launch issues: a face pass and a node pass
-// (the face pass alone for the wave speed), one kernel on FP32 Q1 quads and for
-// the other selectable variants of hexahedra.
+// (the face pass alone for the wave speed), one kernel for the other selectable
+// variants of hexahedra.
 int rhs_kernels(const rkdg_ctx* c, const RhsParams& P) {
-  const bool fp64 = P.fgeo == (const void*)c->d_fgeo64;
   if (P.faces_only) return 1;
   if (c->geom == RKDG_GEOM_CUBE) return c->hex_variant == 3 || c->hex_variant == 0 ? 2 : 1;
-  return c->geom == RKDG_GEOM_SQUARE && c->p == 1 && !fp64 ? 1 : 2;
+  return 2;
 }
 
 // Fluxes (planar) or moments (hexahedra) of the face-pass kernels, in the
@@ -614,7 +613,22 @@ void planar_tables(const rkdg_ctx* c, rkdg::PlanarOpsPair& ops) {
   rkdg::PlanarOps<double>& D = ops.d;
   std::memset(&ops, 0, sizeof ops);
   for (int j = 0; j < nd; ++j) D.wm[j] = T.wmean[j];
+  for (int q = 0; q < nqf; ++q) D.wf[q] = T.wf[q];
+  if (nd <= 4) {
+    for (int lf = 0; lf < nfpe; ++lf)
+      for (int q = 0; q < nqf; ++q)
+        for (int j = 0; j < nd; ++j)
+          D.eb[(lf * nqf + q) * nd + j] = T.B[lf][q][j] * (c->geom == RKDG_GEOM_TRIANGLE ? T.wf[q] : 1.0);
+    for (int j = 0; j < nd; ++j)
+      for (int m = 0; m < nd; ++m) {
+        D.em[j * nd + m] = T.Minv[j][m];
+        for (int r = 0; r < 2; ++r) D.ed[(r * nd + j) * nd + m] = T.D[r][j][m];
+      }
+  }
   if (c->geom == RKDG_GEOM_SQUARE) {
+    for (int lf = 0; lf < nfpe && c->p == 1; ++lf)
+      for (int q = 0; q < nqf; ++q)
+        for (int j = 0; j < nd; ++j) D.b[(lf * nqf + q) * nd + j] = T.B[lf][q][j];
     for (int i = 0; i < n1; ++i) {
       for (int m = 0; m < n1; ++m) D.md[i * n1 + m] = T.d1[i][m] / T.w1[i];
       for (int sd = 0; sd < 2; ++sd) {
@@ -1778,6 +1792,12 @@ int rkdg_batch_setup(rkdg_ctx* c, int nprob, const int* elem_offsets, const doub
     CUDA_TRY(c, cudaMemcpy(c->d_pcov32, c32.data(), nprob * sizeof(float), cudaMemcpyHostToDevice));
   }
   CUDA_TRY(c, cudaMemcpy(c->d_phmin, phmin.data(), nprob * sizeof(double), cudaMemcpyHostToDevice));
+  {  // each face's problem
+    std::vector<int4> fl(c->nface);
+    CUDA_TRY(c, cudaMemcpy(fl.data(), c->d_flist, fl.size() * sizeof(int4), cudaMemcpyDeviceToHost));
+    for (int4& f : fl) f.w = prob[f.x];
+    CUDA_TRY(c, cudaMemcpy(c->d_flist, fl.data(), fl.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  }
   return RKDG_OK;
 }
 

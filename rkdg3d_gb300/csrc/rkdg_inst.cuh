@@ -41,26 +41,22 @@ cudaError_t launch_planar(const RhsParams& prm, const R* u, const EpiParams<R>& 
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   using S = Planar<G, P>;
-  if (prm.ne < 152 * S::EPB)
+  if constexpr (std::is_same<R, float>::value && El<G, P>::NEQ * El<G, P>::ND <= 16) {
+    const int eb = prm.block ? std::min(generic_block(prm.block), 128) : spread_block(prm.ne, 128);
+    k_elem_planar<G, P, R><<<(prm.ne + eb - 1) / eb, eb, 0, st>>>(prm, u, ep);
+  } else if (prm.ne < 152 * S::EPB) {
     k_node_planar<G, P, R, S::SMALL><<<(prm.ne + S::SMALL - 1) / S::SMALL, S::threads(S::SMALL), 0, st>>>(prm, u, ep);
-  else
+  } else {
     k_node_planar<G, P, R, S::EPB><<<(prm.ne + S::EPB - 1) / S::EPB, S::NT, 0, st>>>(prm, u, ep);
+  }
   return cudaGetLastError();
 }
 
 template <int G, int P>
 cudaError_t launch_rhs_t(int prec, const RhsParams& prm, const void* u, const void* ep,
                          cudaStream_t st) {
-  if (prec == 0) return launch_planar<G, P, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st);
-  if constexpr (G == 3 && P == 1) {
-    constexpr int NVAL = El<G, P>::NEQ * El<G, P>::ND;
-    const int blk = std::min(generic_block(prm.block), generic_max_block<float, NVAL>());
-    k_rhs_generic<G, P, float><<<(prm.ne + blk - 1) / blk, blk, 0, st>>>(prm, (const float*)u,
-                                                                       *(const EpiParams<float>*)ep);
-    return cudaGetLastError();
-  } else {
-    return launch_planar<G, P, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
-  }
+  return prec == 0 ? launch_planar<G, P, double>(prm, (const double*)u, *(const EpiParams<double>*)ep, st)
+                   : launch_planar<G, P, float>(prm, (const float*)u, *(const EpiParams<float>*)ep, st);
 }
 
 // Threads per CTA of the limiter: the tuned value, or by the mesh's size.

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
     R gamma = (R)prm.gamma, cov = (R)prm.covolume;
     if (prm.act_cum) {  // batched problems: the i-th element of the active ones
       const int na = *prm.act_n;
-      e = e < prm.act_cum[na] ? active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, pb) : -1;
+      e = e < prm.act_cum[na] ? active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, prm.ne, prm.prob, pb) : -1;
     } else if (e >= ne) {
       e = -1;
     } else if (prm.prob) {

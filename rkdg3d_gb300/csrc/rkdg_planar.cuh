@@ -15,6 +15,10 @@
 //      Runge-Kutta epilogue.  Consecutive threads hold consecutive values of
 //      every array, so all state traffic is coalesced and a thread keeps
 //      neq values instead of neq * nd.
+// FP32 elements of at most 16 values (Q1 quads, P1 triangles) run the second pass
+// with a thread per element (k_elem_planar): there the instructions around a
+// node's few values outnumber its arithmetic three to one.
+//
 // On quadrilaterals the mass, trace and derivative tables of the collocated
 // Gauss-Legendre basis are sparse (the mass matrix is diagonal, a face point
 // sees one line of nodes): N1 terms instead of ND.
@@ -68,9 +72,11 @@ __global__ void __launch_bounds__(128)
     k_face_planar(const __grid_constant__ RhsParams prm, const R* __restrict__ u) {
   using E = El<G, P>;
   constexpr int DIM = 2, ND = E::ND, NEQ = E::NEQ, NFPE = E::NFPE, NQF = E::NQF, N1 = P + 1;
-  __shared__ R sB[G == 2 ? NFPE * NQF * ND : 1];
+  // FP32 Q1 quads: the plain arithmetic (see riemann()), traces from the dense table
+  constexpr bool PLAIN = G == 3 && P == 1 && std::is_same<R, float>::value;
+  __shared__ R sB[G == 2 || PLAIN ? NFPE * NQF * ND : 1];
   const PlanarOps<R>& H = planar_ops<R>(prm.pops);
-  if constexpr (G == 2) {
+  if constexpr (G == 2 || PLAIN) {
     for (int t = threadIdx.x; t < NFPE * NQF * ND; t += blockDim.x) sB[t] = H.b[t];
     __syncthreads();
   }
@@ -88,7 +94,7 @@ __global__ void __launch_bounds__(128)
     face = prm.flist[f];
     e1 = face.x;
     if (prm.prob) {
-      pb = prm.prob[e1];
+      pb = face.w;  // set with the batch
       live = prm.pactive[pb] != 0;
       if constexpr (std::is_same<R, float>::value) {
         gamma = prm.pgamma32 ? prm.pgamma32[pb] : (R)prm.pgamma[pb];
@@ -116,6 +122,10 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
         for (int j = 0; j < N1; ++j) le[j] = sd ? H.lend[N1 + j] : H.lend[j];
         const int i0 = quad_face_node<N1>(lf, qq, 0), st = (lf & 1) ? 1 : N1;
+        if constexpr (PLAIN) {
+#pragma unroll
+          for (int j = 0; j < N1; ++j) le[j] = sB[(lf * NQF + qq) * ND + i0 + j * st];
+        }
 #pragma unroll
         for (int k = 0; k < NEQ; ++k) {
           R v = R(0);
@@ -188,13 +198,18 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) F[k] = R(0);
     } else {
-      lmax = checked_speed(prm, riemann<DIM>(s1, s2, make_frame<DIM, R>(n), F, gamma, cov, prm.rs, prm.avg), e1, pb);
+      R sp;
+      if constexpr (PLAIN)
+        sp = riemann<DIM, R, true>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg);
+      else
+        sp = riemann<DIM>(s1, s2, make_frame<DIM, R>(n), F, gamma, cov, prm.rs, prm.avg);
+      lmax = checked_speed(prm, sp, e1, pb);
     }
     if constexpr (!SPEED) {
       R* out = (R*)prm.fslot + t;
       const long long nf = (long long)prm.nface * NQF;
 #pragma unroll
-      for (int k = 0; k < NEQ; ++k) out[k * nf] = F[k] * jac;
+      for (int k = 0; k < NEQ; ++k) out[k * nf] = PLAIN ? (F[k] * H.wf[q]) * jac : F[k] * jac;
     }
   }
   if (prm.prob)
@@ -295,7 +310,7 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
   if (prm.act_cum) {
     const int na = *prm.act_n;
     live = sl < EPB && e < prm.act_cum[na];
-    if (live) e = active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, pb);
+    if (live) e = active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, prm.ne, prm.prob, pb);
   }
   if (live && prm.prob) {
     if (!prm.act_cum) pb = prm.prob[e];
@@ -354,6 +369,13 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
     if constexpr (G == 3) {
       const int jx = i % N1, jy = i / N1;
 #pragma unroll
+      for (int m = 0; m < N1; ++m) {
+        const R d0 = sMD[jx * N1 + m], d1 = sMD[jy * N1 + m];
+#pragma unroll
+        for (int k = 0; k < NEQ; ++k)
+          acc[k] += d0 * sG[0][k][sl * NP + m + N1 * jy] + d1 * sG[1][k][sl * NP + jx + N1 * m];
+      }
+#pragma unroll
       for (int lf = 0; lf < NFPE; ++lf) {
         const int ref = prm.fref[lf * ne + e];
         const int t = (lf & 1) ? jy : jx;
@@ -364,13 +386,6 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
         const R* p = fx + (long long)(ref >> 2) * NQF + q;
 #pragma unroll
         for (int k = 0; k < NEQ; ++k) acc[k] += c * p[k * nf];
-      }
-#pragma unroll
-      for (int m = 0; m < N1; ++m) {
-        const R d0 = sMD[jx * N1 + m], d1 = sMD[jy * N1 + m];
-#pragma unroll
-        for (int k = 0; k < NEQ; ++k)
-          acc[k] += d0 * sG[0][k][sl * NP + m + N1 * jy] + d1 * sG[1][k][sl * NP + jx + N1 * m];
       }
     } else {
 #pragma unroll
