@@ -74,7 +74,8 @@ cudaError_t launch_nc_vjp(int geom, int p, const RhsParams& prm, const NcParams&
 template <int G, int P>
 static cudaError_t lim_vjp_t(const LimParams& prm, const double* z, const double* yb, double* zb,
                              double* cross, cudaStream_t st) {
-  k_limit_vjp<G, P><<<(prm.ne + 63) / 64, 64, 0, st>>>(prm, z, yb, zb, cross);
+  using S = LimVjp<G, P>;
+  k_limit_vjp<G, P><<<(prm.ne + S::EPB - 1) / S::EPB, S::NT, 0, st>>>(prm, z, yb, zb, cross);
   return cudaGetLastError();
 }
 cudaError_t launch_limit_vjp(int geom, int p, const LimParams& prm, const double* z,

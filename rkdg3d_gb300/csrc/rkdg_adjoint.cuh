@@ -19,9 +19,9 @@
 // Limiter (Multi, BJ-family indicator): the limited values are
 // v_i = mean + m^nd (u_i - mean) (the nd-fold application of
 // limiter_multiplier.cpp:24-38), m = density indicator.  The indicator is
-// recomputed with Dual numbers over the element's density DOFs and the
-// density means of its stencil; the derivative with respect to a
-// neighbour's mean is stored per face and gathered by the neighbour.
+// recomputed and differentiated at its minimising point; the derivative with
+// respect to a neighbour's mean is stored per element and gathered by the
+// neighbour.
 #pragma once
 
 #include "rkdg_common.h"
@@ -29,6 +29,7 @@
 #include "rkdg_flux_vjp.cuh"
 #include "rkdg_generic.cuh"
 #include "rkdg_hex_faces.cuh"
+#include "rkdg_limit.cuh"
 #include "rkdg_physics.cuh"
 
 namespace rkdg {
@@ -383,189 +384,222 @@ __device__ __forceinline__ unsigned hanging_faces(const LimParams& prm, int row)
   return m;
 }
 
-// Limiter VJP, own part.  The stencil's density minimum and maximum are
-// each one element's mean (the first one in stencil order on ties, as the
-// forward min/max keeps it); the derivative with respect to them goes to
-// cross[0..3][e] = (argmin element or -1 for e itself, d/dmin, argmax
-// element or -1, d/dmax), which k_limit_vjp_gather hands to those elements.
+// Limiter VJP, own part, with the forward limiter's threads per element
+// (LimTeam).  The indicator is a minimum over face points, so its gradient is
+// that of one point: the group finds the point (the first in order on ties, as
+// the forward minimum keeps it) and differentiates the limiter function there in
+// reverse, (d y_c/d y) (d y/d diff) times the point's row of basis values.
+// Likewise the stencil's minimum and maximum are each one element's mean; the
+// derivative with respect to them goes to cross[0..3][e] = (argmin element or -1
+// for e itself, d/dmin, argmax element or -1, d/dmax), which k_limit_vjp_gather
+// hands to those elements.  A thread per element that carried Dual<ND + 3>
+// through every point took 205 us on 20^3 Q1 hexahedra, spilling; this one about 60
 template <int G, int P>
-__global__ void __launch_bounds__(64)
+struct LimVjp {
+  using E = El<G, P>;
+  static constexpr int L = LimTeam<G, P>::L, NDP = LimTeam<G, P>::NDP;
+  // threads per CTA: the values and their cotangents within 30 KB
+  static constexpr int NT = 2 * 8 * E::NEQ * NDP * (128 / L) > 30000 ? 64 : 128;
+  static constexpr int EPB = NT / L;
+};
+
+template <int G, int P>
+__global__ void __launch_bounds__(LimVjp<G, P>::NT)
     k_limit_vjp(const LimParams prm, const double* __restrict__ z, const double* __restrict__ ybar,
                 double* __restrict__ zbar, double* __restrict__ cross) {
   using E = El<G, P>;
+  using S = LimVjp<G, P>;
   constexpr int DIM = E::DIM, ND = E::ND, NEQ = E::NEQ, NFPE = E::NFPE, NQL = E::NQL, NV = E::NV;
-  constexpr int NVAR = ND + 3;  // nodal densities, own mean, stencil min, stencil max
-  using D = Dual<NVAR>;
+  constexpr int L = S::L, NDP = S::NDP, NT = S::NT, EPB = S::EPB, NPT = NFPE * NQL;
+  __shared__ double sU[NEQ][EPB][NDP], sY[NEQ][EPB][NDP];  // values, cotangents
+  __shared__ double sBl[ND][NPT], sBv[ND][NV];
+  __shared__ double sM[NEQ][EPB], sSy[NEQ][EPB];  // means, sums of cotangents
+  // factor m^nd, d/d(values) = sGu * basis row sPt, d/d(own mean)
+  __shared__ double sMnd[EPB], sGu[EPB], sGm[EPB];
+  __shared__ int sPt[EPB];
   const RefTables* T = prm.tab;
-  const int ne = prm.ne;
+  const int ne = prm.ne, tid = threadIdx.x, e0 = blockIdx.x * EPB;
+  const int nel = min(EPB, ne - e0);
   const long long NDa = prm.ndofs;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  double el[NEQ][ND], yb[NEQ][ND], um[NEQ];
-  for (int k = 0; k < NEQ; ++k) {
-    um[k] = prm.means[(long long)k * ne + e];
-    for (int j = 0; j < ND; ++j) {
-      el[k][j] = z[k * NDa + (long long)e * ND + j];
-      yb[k][j] = ybar[k * NDa + (long long)e * ND + j];
+  for (int t = tid; t < ND * NPT; t += NT) {
+    const int j = t / NPT, pt = t - j * NPT;
+    sBl[j][pt] = T->Bl[pt / NQL][pt % NQL][j];
+  }
+  for (int t = tid; t < ND * NV; t += NT) sBv[t / NV][t % NV] = T->Bv[t % NV][t / NV];
+  for (int t = tid; t < NEQ * EPB; t += NT) {
+    const int k = t / EPB, s = t - k * EPB;
+    if (s < nel) sM[k][s] = prm.means[(long long)k * ne + e0 + s];
+  }
+  for (int t = tid; t < nel * ND; t += NT) {
+    const int s = t / ND, j = t - s * ND;
+#pragma unroll
+    for (int k = 0; k < NEQ; ++k) {
+      sU[k][s][j] = z[k * NDa + (long long)e0 * ND + t];
+      sY[k][s][j] = ybar[k * NDa + (long long)e0 * ND + t];
     }
   }
-  for (int i = 0; i < 4; ++i) cross[(long long)i * ne + e] = i == 0 || i == 2 ? -1.0 : 0.0;
-  const int row = lim_ncrow(prm, e);
-  const int nst = stencil_size(prm, row, NFPE);
-  const unsigned ncfaces = hanging_faces(prm, row);
-  double zb[NEQ][ND];
-  for (int k = 0; k < NEQ; ++k)
-    for (int j = 0; j < ND; ++j) zb[k][j] = 0.0;
-  // density indicator with derivatives
-  D m;
-  int amin = -1, amax = -1;
-  double elind_last = 1.0;
-  if (prm.indicator == 0) {
-    m = D(1.0);
-  } else if (prm.indicator == 1) {
-    m = D(0.0);
-    elind_last = 0.0;
-  } else {
-    D rho[ND];
-    for (int j = 0; j < ND; ++j) rho[j] = D::var(el[0][j], j);
-    const D mself = D::var(um[0], ND);
-    double mIv = um[0] < 1e9 ? um[0] : 1e9, MIv = um[0] > -1e9 ? um[0] : -1e9;
-    for (int i = 0; i < nst; ++i) {
-      const int nb = stencil_at(prm, e, row, NFPE, i);
-      if (nb < 0) continue;
-      const double v = prm.means[nb];
-      if (v < mIv) {
-        mIv = v;
-        amin = nb;
-      }
-      if (v > MIv) {
-        MIv = v;
-        amax = nb;
-      }
-    }
-    const D mI = amin >= 0 ? D::var(mIv, ND + 1) : (mself < D(1e9) ? mself : D(1e9));
-    const D MI = amax >= 0 ? D::var(MIv, ND + 2) : (mself > D(-1e9) ? mself : D(-1e9));
-    D yMin = D(1e9);
-    for (int lf = 0; lf < NFPE; ++lf) {
-      if (prm.fnbr[lf * ne + e] < 0 && !((ncfaces >> lf) & 1u)) continue;
-      for (int q = 0; q < NQL; ++q) {
-        D v = D(0.0);
-        for (int j = 0; j < ND; ++j) v += rho[j] * T->Bl[lf][q][j];
-        const D diff = v - mself;
-        D y;
-        if (diff > D(1e-3))
-          y = (MI - mself) / diff;
-        else if (diff < D(-1e-3))
-          y = (mI - mself) / diff;
-        else
-          y = D(1.0);
-        if (prm.function == 0) {
-          yMin = y < yMin ? y : yMin;
-          yMin = yMin > D(1.0) ? D(1.0) : yMin;
-        } else if (prm.function == 1) {
-          const D yc = (y * y + 2.0 * y) / (y * y + y + 2.0);
-          yMin = yc < yMin ? yc : yMin;
-        } else {
-          const double ys = 1.5;
-          const D yr = y / ys;
-          const D yc = y < D(1.0) ? y + (3.0 - 2.0 * ys) * yr * yr + (ys - 2.0) * yr * yr * yr : D(1.0);
-          yMin = yc < yMin ? yc : yMin;
-        }
-      }
-    }
-    m = yMin;
-    // FinDiff looks at the last equation's indicator; recompute it plainly
-    if (prm.limiter == 0) {
-      const int kl = NEQ - 1;
-      double mIl = um[kl], MIl = um[kl], yl = 1e9;
-      for (int i = 0; i < nst; ++i) {
+  __syncthreads();
+  const int slot = tid / L, lane = tid - slot * L;
+  const bool on = slot < nel;
+  const int e = e0 + slot;
+  const bool multi = prm.limiter == 1;
+  const int kind = multi ? 0 : NEQ - 1;  // the equation whose indicator counts
+  double m = prm.indicator == 1 ? 0.0 : 1.0;
+  double gu = 0.0, gm = 0.0, gmin = 0.0, gmax = 0.0;  // d m / d(values), own mean, min, max
+  int ptmin = -1, amin = -1, amax = -1;
+  if (prm.indicator >= 2) {
+    const double own = on ? sM[kind][slot] : 0.0;
+    double mI = own < 1e9 ? own : 1e9, MI = own > -1e9 ? own : -1e9;
+    int imin = -1, imax = -1;  // places in the stencil, -1 the element itself
+    unsigned inner = 0;
+    if (on) {
+      const int row = lim_ncrow(prm, e), nst = stencil_size(prm, row, NFPE);
+      if (row >= 0) inner = hanging_faces(prm, row);
+      for (int i = lane; i < nst; i += L) {
         const int nb = stencil_at(prm, e, row, NFPE, i);
         if (nb < 0) continue;
-        const double v = prm.means[(long long)kl * ne + nb];
-        mIl = v < mIl ? v : mIl;
-        MIl = v > MIl ? v : MIl;
+        if (i < NFPE) inner |= 1u << i;
+        const double v = prm.means[(long long)kind * ne + nb];
+        if (v < mI) mI = v, imin = i, amin = nb;
+        if (v > MI) MI = v, imax = i, amax = nb;
       }
-      for (int lf = 0; lf < NFPE; ++lf) {
-        if (prm.fnbr[lf * ne + e] < 0 && !((ncfaces >> lf) & 1u)) continue;
-        for (int q = 0; q < NQL; ++q) {
-          double v = 0.0;
-          for (int j = 0; j < ND; ++j) v += el[kl][j] * T->Bl[lf][q][j];
-          const double diff = v - um[kl];
-          double y = diff > 1e-3 ? (MIl - um[kl]) / diff : (diff < -1e-3 ? (mIl - um[kl]) / diff : 1.0);
-          double yc;
-          if (prm.function == 0) {
-            yc = y < 1.0 ? y : 1.0;
-          } else if (prm.function == 1) {
-            yc = (y * y + 2.0 * y) / (y * y + y + 2.0);
-          } else {
-            const double yr = y / 1.5;
-            yc = y < 1.0 ? y + 0.0 * yr * yr - 0.5 * yr * yr * yr : 1.0;
-          }
-          yl = yc < yl ? yc : yl;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1) {  // the smaller (mean, place)
+      const double a = __shfl_xor_sync(0xffffffffu, mI, o), b = __shfl_xor_sync(0xffffffffu, MI, o);
+      const int ia = __shfl_xor_sync(0xffffffffu, imin, o), ib = __shfl_xor_sync(0xffffffffu, imax, o);
+      const int na = __shfl_xor_sync(0xffffffffu, amin, o), nb = __shfl_xor_sync(0xffffffffu, amax, o);
+      if (a < mI || (a == mI && ia < imin)) mI = a, imin = ia, amin = na;
+      if (b > MI || (b == MI && ib < imax)) MI = b, imax = ib, amax = nb;
+      inner |= __shfl_xor_sync(0xffffffffu, inner, o);
+    }
+    double yMin = 1e9;
+    if (on)
+      for (int pt = lane; pt < NPT; pt += L) {
+        if (!((inner >> (pt / NQL)) & 1u)) continue;  // only interior faces carry indicator points
+        double v = 0.0;
+#pragma unroll
+        for (int j = 0; j < ND; ++j) v += sU[kind][slot][j] * sBl[j][pt];
+        const double diff = v - own;
+        const bool up = diff > 1e-3, dn = diff < -1e-3;
+        const double idiff = 1.0 / diff;
+        const double y = up ? (MI - own) / diff : (dn ? (mI - own) / diff : 1.0);
+        double yc, dy;  // limiter function and its derivative
+        if (prm.function == 0) {
+          yc = y <= 1.0 ? y : 1.0;
+          dy = y <= 1.0 ? 1.0 : 0.0;
+        } else if (prm.function == 1) {
+          const double den = y * y + y + 2.0;
+          yc = (y * y + 2.0 * y) / den;
+          dy = (2.0 * y + 2.0 - yc * (2.0 * y + 1.0)) / den;
+        } else {
+          const double ys = 1.5;
+          const double yr = y / ys;
+          yc = y < 1.0 ? y + (3.0 - 2.0 * ys) * yr * yr + (ys - 2.0) * yr * yr * yr : 1.0;
+          dy = y < 1.0 ? 1.0 + (2.0 * (3.0 - 2.0 * ys) * yr + 3.0 * (ys - 2.0) * yr * yr) / ys : 0.0;
+        }
+        if (yc < yMin) {
+          yMin = yc;
+          ptmin = pt;
+          const double g = up || dn ? dy * idiff : 0.0;
+          gu = -y * g;
+          gm = (y - 1.0) * g;
+          gmin = dn ? g : 0.0;
+          gmax = up ? g : 0.0;
         }
       }
-      elind_last = yl;
+    // the smaller (value, point) of the group
+    double yb = yMin;
+    int pb = ptmin;
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1) {
+      const double a = __shfl_xor_sync(0xffffffffu, yb, o);
+      const int p = __shfl_xor_sync(0xffffffffu, pb, o);
+      if (a < yb || (a == yb && (unsigned)p < (unsigned)pb)) yb = a, pb = p;
     }
+    m = yb;
+    // point pt belongs to lane pt % L
+    const int src = (tid & 31) - lane + (pb >= 0 ? pb % L : 0);
+    gu = __shfl_sync(0xffffffffu, gu, src);
+    gm = __shfl_sync(0xffffffffu, gm, src);
+    gmin = __shfl_sync(0xffffffffu, gmin, src);
+    gmax = __shfl_sync(0xffffffffu, gmax, src);
+    ptmin = pb;
+    // a minimum or maximum that is the element's own mean moves with it
+    if (amin < 0 && own < 1e9) gm += gmin;
+    if (amax < 0 && own > -1e9) gm += gmax;
   }
-  const double* w = T->wmn_e ? T->wmn_e + (long long)e * ND : T->wmean;
-  if (prm.limiter == 1) {
+  for (int k = lane; k < NEQ; k += L) {
+    double sy = 0.0;
+    if (on)
+      for (int i = 0; i < ND; ++i) sy += sY[k][slot][i];
+    sSy[k][slot] = sy;
+  }
+  __syncwarp();
+  double mnd = 1.0;  // FinDiff: as it is, or the mean
+  double mbar = 0.0;
+  if (multi) {
     const int reps = (prm.quirks & 1) ? 1 : ND;
-    const double mv = m.v;
     double pm1 = 1.0;  // m^(reps-1)
-    for (int i = 1; i < reps; ++i) pm1 *= mv;
-    const double mnd = pm1 * mv;
-    const double dmnd = reps * pm1;
-    // forward values to test the last-hope reset
-    bool reset = false;
-    if (prm.last_hope) {
-      for (int v = 0; v < NV && !reset; ++v) {
+    for (int i = 1; i < reps; ++i) pm1 *= m;
+    mnd = pm1 * m;
+    int bad = 0;
+    if (on && prm.last_hope)  // forward values at the vertices: the last-hope reset
+      for (int v = lane; v < NV; v += L) {
         double fv[NEQ];
+#pragma unroll
         for (int k = 0; k < NEQ; ++k) {
+          const double um = sM[k][slot];
           double s = 0.0;
-          for (int j = 0; j < ND; ++j) s += (um[k] + mnd * (el[k][j] - um[k])) * T->Bv[v][j];
+          for (int j = 0; j < ND; ++j) s += (um + mnd * (sU[k][slot][j] - um)) * sBv[j][v];
           fv[k] = s;
         }
-        if (!state_is_physical<DIM>(fv, prm.gamma, prm.covolume)) reset = true;
+        if (!state_is_physical<DIM>(fv, prm.gamma, prm.covolume)) bad = 1;
       }
-    }
-    if (reset) {
-      for (int k = 0; k < NEQ; ++k) {
-        double sy = 0.0;
-        for (int i = 0; i < ND; ++i) sy += yb[k][i];
-        for (int j = 0; j < ND; ++j) zb[k][j] += w[j] * sy;
+    __syncwarp();
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1) bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+    if (on && !bad && prm.indicator == 2)
+      for (int k = lane; k < NEQ; k += L) {
+        const double um = sM[k][slot];
+        double s = 0.0;
+        for (int i = 0; i < ND; ++i) s += sY[k][slot][i] * (sU[k][slot][i] - um);
+        mbar += s;
       }
-    } else {
-      double mbar = 0.0;
-      for (int k = 0; k < NEQ; ++k) {
-        double sy = 0.0;
-        for (int i = 0; i < ND; ++i) {
-          sy += yb[k][i];
-          mbar += yb[k][i] * dmnd * (el[k][i] - um[k]);
-        }
-        for (int j = 0; j < ND; ++j) zb[k][j] += w[j] * (1.0 - mnd) * sy + mnd * yb[k][j];
-      }
-      if (prm.indicator == 2) {
-        for (int j = 0; j < ND; ++j) zb[0][j] += mbar * (m.d[j] + m.d[ND] * w[j]);
-        cross[(long long)0 * ne + e] = amin;
-        cross[(long long)1 * ne + e] = mbar * m.d[ND + 1];
-        cross[(long long)2 * ne + e] = amax;
-        cross[(long long)3 * ne + e] = mbar * m.d[ND + 2];
-      }
-    }
-  } else {
-    if (elind_last < 0.999) {
-      for (int k = 0; k < NEQ; ++k) {
-        double sy = 0.0;
-        for (int i = 0; i < ND; ++i) sy += yb[k][i];
-        for (int j = 0; j < ND; ++j) zb[k][j] += w[j] * sy;
-      }
-    } else {
-      for (int k = 0; k < NEQ; ++k)
-        for (int j = 0; j < ND; ++j) zb[k][j] += yb[k][j];
+    __syncwarp();
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1) mbar += __shfl_xor_sync(0xffffffffu, mbar, o);
+    mbar *= reps * pm1;
+    if (bad) mnd = 0.0, mbar = 0.0, amin = amax = -1;
+  } else if (m < 0.999) {
+    mnd = 0.0;
+  }
+  if (lane == 0) {
+    const bool x = on && multi && prm.indicator == 2;
+    sMnd[slot] = mnd;
+    sGu[slot] = x && ptmin >= 0 ? mbar * gu : 0.0;
+    sGm[slot] = x ? mbar * gm : 0.0;
+    sPt[slot] = ptmin >= 0 ? ptmin : 0;
+    if (on) {
+      cross[e] = x ? amin : -1;
+      cross[(long long)ne + e] = x ? mbar * gmin : 0.0;
+      cross[2LL * ne + e] = x ? amax : -1;
+      cross[3LL * ne + e] = x ? mbar * gmax : 0.0;
     }
   }
-  for (int k = 0; k < NEQ; ++k)
-    for (int j = 0; j < ND; ++j) zbar[k * NDa + (long long)e * ND + j] = zb[k][j];
+  __syncthreads();
+  for (int t = tid; t < nel * ND; t += NT) {
+    const int s = t / ND, j = t - s * ND;
+    const double w = T->wmn_e ? T->wmn_e[(long long)e0 * ND + t] : T->wmean[j];
+    const double mn = sMnd[s], own = w * (1.0 - mn);
+#pragma unroll
+    for (int k = 0; k < NEQ; ++k) {
+      double r = own * sSy[k][s] + mn * sY[k][s][j];
+      if (k == 0) r += sGu[s] * sBl[j][sPt[s]] + sGm[s] * w;
+      zbar[k * NDa + (long long)e0 * ND + t] = r;
+    }
+  }
 }
 
 // Gather, for element c, the derivatives that the elements of its stencil
