@@ -156,18 +156,19 @@ int rkdg_set_precision(rkdg_ctx* ctx, int precision);
 /* Kernel tuning knobs (no counterpart in the reference; set by hand or by
  * rkdg_autotune).  RKDG_TUNE_HEX_KERNEL: 0 default, 1 warp per element,
  * 2 five-lane team per element, 3 face pass (each face once, its moments into
- * per-face slots) + node pass, the FP64 default,
+ * per-face slots) + node pass, the default,
  * 4 five-lane team over Morton-ordered groups of 24 elements whose faces
  * inside the group are evaluated once (order <= 2 hexahedra; the plain team
  * kernel when the mesh's face graph needs more than 8 rounds), 5 face-once
- * tiles of 32 Morton-ordered elements (order <= 2; the FP32 Q2 default),
+ * tiles of 32 Morton-ordered elements (order <= 2),
  * 6 the tile kernel with the collocated volume contraction on the tensor
  * cores (tcgen05 TF32 MMAs, operands split into TF32 hi + lo; FP32-bulk Q2
  * only, else the default).
  * RKDG_TUNE_GENERIC_BLOCK /
- * RKDG_TUNE_LIMITER_BLOCK: elements (threads) per CTA of the triangle/quad
- * right-hand-side kernel and of the limiter, 0 (default 128) or a multiple of
- * 32 up to 256. */
+ * RKDG_TUNE_LIMITER_BLOCK: threads per CTA of the element pass (FP32 Q1
+ * quadrilaterals and P1 triangles; the other planar passes have their own
+ * shapes) and of the limiter, 0 (default: 128, fewer on small meshes) or a
+ * multiple of 32 up to 256. */
 enum { RKDG_TUNE_HEX_KERNEL = 1, RKDG_TUNE_GENERIC_BLOCK = 2, RKDG_TUNE_LIMITER_BLOCK = 3 };
 int rkdg_set_tuning(rkdg_ctx* ctx, int key, int value);
 /* Autotuner (no counterpart in the reference): times each candidate launch

@@ -248,6 +248,11 @@ struct RhsParams {
   const int* act_pid;
   const int* act_n;
   const int* poff;
+  // their faces (planar face pass): prefix sums of the active problems' face
+  // counts, and per problem the first interior and the first other face in flist
+  const int* act_fcum;
+  const int* pfi;
+  const int* pfb;
   int block;            // threads per CTA of the generic kernels (0: default)
   void* fslot;          // fluxes / moments of the face-pass kernels (see flist below)
   const HexTeamSched* hsched;  // shared-face hexahedral kernel: one entry per CTA (or null)
@@ -401,6 +406,9 @@ struct BatchState {
   int* act_pid;         // [nprob]
   int* act_n;           // [1]
   const int* poff;      // [nprob + 1] element offsets
+  int* act_fcum;        // [nprob + 1] and, as the element offsets, of the
+  const int* pfi;       // interior faces and
+  const int* pfb;       // of the others
 };
 
 }  // namespace rkdg

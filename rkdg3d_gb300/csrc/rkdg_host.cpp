@@ -136,6 +136,8 @@ struct rkdg_ctx {
   // map of the active work of a batched run (see RhsParams)
   int* d_act_cum = nullptr;
   int* d_act_pid = nullptr;
+  int* d_act_fcum = nullptr;
+  int* d_pfi = nullptr;  // per problem: first interior face, then (from nprob + 1) first other face
   int* d_act_n = nullptr;
   int* d_poff = nullptr;
   int* d_pfail = nullptr;
@@ -212,6 +214,8 @@ void free_mesh(rkdg_ctx* c) {
   dfree(c->d_nactive);
   dfree(c->d_act_cum);
   dfree(c->d_act_pid);
+  dfree(c->d_act_fcum);
+  dfree(c->d_pfi);
   dfree(c->d_act_n);
   dfree(c->d_poff);
   dfree(c->d_pfail);
@@ -435,6 +439,9 @@ void set_batch(rkdg_ctx* c, RhsParams& P, int slot) {
   P.pactive = c->d_pactive;
   P.act_cum = c->d_act_cum;
   P.act_pid = c->d_act_pid;
+  P.act_fcum = c->d_act_fcum;
+  P.pfi = c->d_pfi;
+  P.pfb = c->d_pfi + c->nprob + 1;
   P.act_n = c->d_act_n;
   P.poff = c->d_poff;
   P.pmcs = c->d_pmcs + (size_t)slot * c->nprob;
@@ -1778,6 +1785,8 @@ int rkdg_batch_setup(rkdg_ctx* c, int nprob, const int* elem_offsets, const doub
   CUDA_TRY(c, dalloc(c->d_nactive, (size_t)1));
   CUDA_TRY(c, dalloc(c->d_act_cum, (size_t)nprob + 1));
   CUDA_TRY(c, dalloc(c->d_act_pid, (size_t)nprob));
+  CUDA_TRY(c, dalloc(c->d_act_fcum, (size_t)nprob + 1));
+  CUDA_TRY(c, dalloc(c->d_pfi, 2 * ((size_t)nprob + 1)));
   CUDA_TRY(c, dalloc(c->d_act_n, (size_t)1));
   CUDA_TRY(c, dalloc(c->d_poff, (size_t)nprob + 1));
   CUDA_TRY(c, cudaMemcpy(c->d_poff, elem_offsets, (nprob + 1) * sizeof(int), cudaMemcpyHostToDevice));
@@ -1792,11 +1801,21 @@ int rkdg_batch_setup(rkdg_ctx* c, int nprob, const int* elem_offsets, const doub
     CUDA_TRY(c, cudaMemcpy(c->d_pcov32, c32.data(), nprob * sizeof(float), cudaMemcpyHostToDevice));
   }
   CUDA_TRY(c, cudaMemcpy(c->d_phmin, phmin.data(), nprob * sizeof(double), cudaMemcpyHostToDevice));
-  {  // each face's problem
+  {  // each face's problem, and each problem's faces: the list holds the interior
+     // ones, then the others, both in the order of the elements
     std::vector<int4> fl(c->nface);
     CUDA_TRY(c, cudaMemcpy(fl.data(), c->d_flist, fl.size() * sizeof(int4), cudaMemcpyDeviceToHost));
-    for (int4& f : fl) f.w = prob[f.x];
+    std::vector<int> off(2 * ((size_t)nprob + 1), 0);
+    int* count[2] = {off.data() + 1, off.data() + nprob + 2};
+    for (int4& f : fl) {
+      f.w = prob[f.x];
+      ++count[f.y < 0][f.w];
+    }
+    off[nprob + 1] = c->nface - c->nbface;
+    for (int h = 0; h < 2; ++h)
+      for (int p = 0; p < nprob; ++p) count[h][p] += count[h][p - 1];
     CUDA_TRY(c, cudaMemcpy(c->d_flist, fl.data(), fl.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, cudaMemcpy(c->d_pfi, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice));
   }
   return RKDG_OK;
 }
@@ -1832,6 +1851,9 @@ int rkdg_batch_run(rkdg_ctx* c, double* x, double t_end, double cfl, double dt0,
   bs.nactive = c->d_nactive;
   bs.act_cum = c->d_act_cum;
   bs.act_pid = c->d_act_pid;
+  bs.act_fcum = c->d_act_fcum;
+  bs.pfi = c->d_pfi;
+  bs.pfb = c->d_pfi + np + 1;
   bs.act_n = c->d_act_n;
   bs.poff = c->d_poff;
   bs.mcs_last = c->d_pmcs + (size_t)(c->s - 1) * np;

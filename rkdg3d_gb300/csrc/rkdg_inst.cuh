@@ -27,6 +27,12 @@ inline int spread_block(long long n, int most) {
   return b;
 }
 
+// CTAs of a batch's face pass and limiter, which loop over the active work: a
+// CTA past it costs its launch and two loads, so at most 64 per SM (256 strips of
+// 4,400 quads need 35,000 with every problem active, and run two thirds of their
+// steps with less than half of them).
+inline unsigned batch_grid(unsigned grid) { return std::min(grid, 152u * 64u); }
+
 template <int G, int P, typename R>
 cudaError_t launch_planar(const RhsParams& prm, const R* u, const EpiParams<R>& ep, cudaStream_t st) {
   if (!prm.flist || !prm.fslot) return cudaErrorInvalidValue;
@@ -34,10 +40,16 @@ cudaError_t launch_planar(const RhsParams& prm, const R* u, const EpiParams<R>& 
   const int blk = spread_block(npt, 128);
   const unsigned grid = (unsigned)((npt + blk - 1) / blk);
   if (prm.faces_only) {
-    k_face_planar<G, P, R, true><<<grid, blk, 0, st>>>(prm, u);
+    if (prm.act_cum)
+      k_face_planar<G, P, R, true, true><<<batch_grid(grid), blk, 0, st>>>(prm, u);
+    else
+      k_face_planar<G, P, R, true, false><<<grid, blk, 0, st>>>(prm, u);
     return cudaGetLastError();
   }
-  k_face_planar<G, P, R, false><<<grid, blk, 0, st>>>(prm, u);
+  if (prm.act_cum)
+    k_face_planar<G, P, R, false, true><<<batch_grid(grid), blk, 0, st>>>(prm, u);
+  else
+    k_face_planar<G, P, R, false, false><<<grid, blk, 0, st>>>(prm, u);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   using S = Planar<G, P>;
@@ -75,7 +87,15 @@ cudaError_t launch_limit_mode(const LimParams& prm, R* u, float* ulo, cudaStream
   }
   static_assert(T::template smem_bytes<R, DS>(T::MAX_BLOCK) <= 48 * 1024, "shared memory of the largest CTA");
   const int blk = limit_block(prm.block, prm.ne, T::L), epb = blk / T::L;
-  k_limit_team<G, P, R, DS><<<(prm.ne + epb - 1) / epb, blk, T::template smem_bytes<R, DS>(blk), st>>>(prm, u, ulo);
+  const unsigned grid = (unsigned)((prm.ne + epb - 1) / epb);
+  const size_t smem = T::template smem_bytes<R, DS>(blk);
+  if constexpr (G != 5) {  // batches are planar
+    if (prm.act_cum) {
+      k_limit_team<G, P, R, DS, true><<<batch_grid(grid), blk, smem, st>>>(prm, u, ulo);
+      return cudaGetLastError();
+    }
+  }
+  k_limit_team<G, P, R, DS, false><<<grid, blk, smem, st>>>(prm, u, ulo);
   return cudaGetLastError();
 }
 

@@ -11,7 +11,7 @@ bool generic_supported(int geom, int p);
 // prec: 0 = FP64, 1 = FP32.  ep points to EpiParams<double> or EpiParams<float>.
 cudaError_t launch_rhs(int geom, int p, int prec, const RhsParams& prm, const void* u,
                        const void* ep, cudaStream_t st);
-// Same with a hexahedral kernel variant (0 default, 1 warp per element, 2 team).
+// Same with a hexahedral kernel variant (see launch_hex_variant).
 cudaError_t launch_rhs_v(int variant, int geom, int p, int prec, const RhsParams& prm,
                          const void* u, const void* ep, cudaStream_t st);
 cudaError_t launch_hex_variant(int variant, int p, int prec, const RhsParams& prm, const void* u,

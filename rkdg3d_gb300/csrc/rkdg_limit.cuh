@@ -83,7 +83,8 @@ __device__ __forceinline__ bool vertex_is_physical(const R* s, R gamma, R b) {
 // 32 us (287), 48x45x51 hex Q1 float pair 54 us (134), 33x27x21 hex Q1 FP64
 // 68 us (191), 524,288 P1 triangles FP64 245 us (459), FP32 47 us (45) and float
 // pair 71 us (76): there the arithmetic of the few values is what is left.
-template <int G, int P, typename R, bool DS>
+// MAP: a batch with a map of the active work (prm.act_cum).
+template <int G, int P, typename R, bool DS, bool MAP>
 __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
     k_limit_team(const LimParams prm, R* __restrict__ u, float* __restrict__ ulo) {
   using E = El<G, P>;
@@ -102,8 +103,7 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
   using IndT = typename std::conditional<F32, float, double>::type;
   const RefTables* tab = prm.tab;
   const int tid = threadIdx.x, NT = blockDim.x, EPB = NT / L;
-  // batched problems with a map of the active work: CTAs past it are idle
-  if (prm.act_cum && (int)(blockIdx.x * EPB) >= prm.act_cum[*prm.act_n]) return;
+  if (MAP && (int)(blockIdx.x * EPB) >= prm.act_cum[*prm.act_n]) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   MeanT* sM = reinterpret_cast<MeanT*>(smraw);                     // [NEQ][EPB]
   MeanT* sBl = sM + NEQ * EPB;                                     // [ND][NPT]
@@ -117,10 +117,26 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
   int* sF = sE + EPB;                                              // [EPB] 1 changed, 2 mean
   const int ne = prm.ne;
   const long long NDa = prm.ndofs;
+  for (int t = tid; t < ND * NPT; t += NT) {
+    const int j = t / NPT, pt = t - j * NPT;
+    if constexpr (F32)
+      sBl[t] = tab->Bl32[j][pt];
+    else
+      sBl[t] = tab->Bl[pt / NQL][pt % NQL][j];
+  }
+  for (int t = tid; t < ND * NV; t += NT) {
+    const int j = t / NV, v = t - j * NV;
+    if constexpr (F32)
+      sBv[t] = tab->Bv32[j][v];
+    else
+      sBv[t] = tab->Bv[v][j];
+  }
+  // MAP: CTAs run over the elements of the active problems
+  for (int blk = blockIdx.x;; blk += gridDim.x) {
   for (int s = tid; s < EPB; s += NT) {
-    int e = blockIdx.x * EPB + s, pb = -1;
+    int e = blk * EPB + s, pb = -1;
     R gamma = (R)prm.gamma, cov = (R)prm.covolume;
-    if (prm.act_cum) {  // batched problems: the i-th element of the active ones
+    if (MAP) {  // the i-th element of the active problems
       const int na = *prm.act_n;
       e = e < prm.act_cum[na] ? active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, prm.ne, prm.prob, pb) : -1;
     } else if (e >= ne) {
@@ -141,20 +157,6 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
     sE[s] = e;
     sG[s] = gamma;
     sG[EPB + s] = cov;
-  }
-  for (int t = tid; t < ND * NPT; t += NT) {
-    const int j = t / NPT, pt = t - j * NPT;
-    if constexpr (F32)
-      sBl[t] = tab->Bl32[j][pt];
-    else
-      sBl[t] = tab->Bl[pt / NQL][pt % NQL][j];
-  }
-  for (int t = tid; t < ND * NV; t += NT) {
-    const int j = t / NV, v = t - j * NV;
-    if constexpr (F32)
-      sBv[t] = tab->Bv32[j][v];
-    else
-      sBv[t] = tab->Bv[v][j];
   }
   __syncthreads();
   const bool multi = prm.limiter == 1;
@@ -281,31 +283,73 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
     } else {
       if (mI > 1e9) mI = 1e9;
       if (MI < -1e9) MI = -1e9;
+      // y = (stencil max or min - mean) / diff falls with |diff|, and every
+      // limiter function is smallest at the smallest y (Venkatakrishnan's,
+      // where that lies below 2): only the points of largest |diff| above and
+      // below the mean are divided for, one by the even and one by the odd
+      // lanes.  |diff| is compared as integers, off the FP64 pipe.
+      const long long dead = __double_as_longlong(1e-3), inf = 0x7ff0000000000000ll;
+      const long long sign = (long long)0x8000000000000000ull;
+      long long far[2] = {0, 0}, near[2] = {inf, inf};  // |diff| above, below
+      bool level = false;                               // some point within the +-1e-3 switch
       for (int pt = lane; pt < NPT; pt += L) {
         if (!((inner >> (pt / NQL)) & 1u)) continue;  // only interior faces carry indicator points
         double v = 0.0;
 #pragma unroll
         for (int j = 0; j < ND; ++j) v += un[j] * sBl[j * NPT + pt];
-        const double diff = v - own;
-        double y = 1.0;
-        if (diff > 1e-3 || diff < -1e-3) y = ((diff > 0.0 ? MI : mI) - own) / diff;
-        double yc;
-        if (prm.function == 0) {
-          yc = y > 1.0 ? 1.0 : y;
-        } else if (prm.function == 1) {
-          yc = (y * y + 2.0 * y) / (y * y + y + 2.0);
-        } else {
-          const double ys = 1.5;
-          const double yr = y / ys;
-          yc = y < 1.0 ? y + (3.0 - 2.0 * ys) * yr * yr + (ys - 2.0) * yr * yr * yr : 1.0;
+        const long long d = __double_as_longlong(v - own), ad = d & ~sign;
+        const bool in = ad <= dead || ad > inf;  // (NaN compares as neither)
+        level |= in;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const bool on = !in && (d < 0) == (h == 1);
+          far[h] = on && ad > far[h] ? ad : far[h];
+          near[h] = on && ad < near[h] ? ad : near[h];
         }
-        yMin = yc < yMin ? yc : yMin;
       }
+      __syncwarp();
 #pragma unroll
       for (int o = 1; o < L; o <<= 1) {
-        const double y = __shfl_xor_sync(0xffffffffu, yMin, o);
-        yMin = y < yMin ? y : yMin;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const long long x = __shfl_xor_sync(0xffffffffu, far[h], o);
+          far[h] = x > far[h] ? x : far[h];
+        }
+        level |= __shfl_xor_sync(0xffffffffu, (int)level, o) != 0;
       }
+      const int h = lane & 1;
+      const double num = h ? own - mI : MI - own;
+      auto function = [&](double y) {
+        if (prm.function == 0) return y > 1.0 ? 1.0 : y;
+        if (prm.function == 1) return (y * y + 2.0 * y) / (y * y + y + 2.0);
+        const double ys = 1.5;
+        const double yr = y / ys;
+        return y < 1.0 ? y + (3.0 - 2.0 * ys) * yr * yr + (ys - 2.0) * yr * yr * yr : 1.0;
+      };
+      if (level) yMin = prm.function == 1 ? 0.75 : 1.0;
+      const long long fh = h ? far[1] : far[0];
+      const double y = fh ? num / __longlong_as_double(fh) : 1e9;
+      if (fh) {
+        const double yc = function(y);
+        yMin = yc < yMin ? yc : yMin;
+      }
+      // Venkatakrishnan's function rises to y = 2 + sqrt(8), then falls to 1: with
+      // every y above 2 the largest may be the minimum
+      if (prm.function == 1 && __any_sync(0xffffffffu, y > 2.0 && fh)) {
+#pragma unroll
+        for (int o = 1; o < L; o <<= 1)
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            const long long x = __shfl_xor_sync(0xffffffffu, near[g], o);
+            near[g] = x < near[g] ? x : near[g];
+          }
+        if (fh) {
+          const double yc = function(num / __longlong_as_double(h ? near[1] : near[0]));
+          yMin = yc < yMin ? yc : yMin;
+        }
+      }
+      const double other = __shfl_xor_sync(0xffffffffu, yMin, 1);
+      yMin = other < yMin ? other : yMin;
     }
     ind = yMin;
   }
@@ -452,6 +496,9 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
         u[k * NDa + i0] = (f & 2) ? um : sU[(k * EPB + s) * NDP + j];
       }
     }
+  }
+  if (!MAP || (long long)(blk + gridDim.x) * EPB >= prm.act_cum[*prm.act_n]) break;
+  __syncthreads();
   }
 }
 

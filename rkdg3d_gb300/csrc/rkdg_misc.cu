@@ -214,30 +214,36 @@ __device__ __forceinline__ double bits_to_double(unsigned long long b) {
 __device__ void build_active_map(const BatchState& bs) {
   if (!bs.act_cum || threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
-  int run = 0, na = 0;
+  int run = 0, runf = 0, na = 0;
   for (int base = 0; base < bs.nprob; base += 32) {
     const int p = base + lane;
     const bool a = p < bs.nprob && bs.active[p];
     const int sz = a ? bs.poff[p + 1] - bs.poff[p] : 0;
-    int cs = sz, cf = a ? 1 : 0;  // inclusive scans of sizes and of active flags
+    const int sf = a ? bs.pfi[p + 1] - bs.pfi[p] + bs.pfb[p + 1] - bs.pfb[p] : 0;
+    int cs = sz, cf = a ? 1 : 0, cq = sf;  // inclusive scans of sizes, active flags, faces
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int ts = __shfl_up_sync(0xffffffffu, cs, o);
       const int tf = __shfl_up_sync(0xffffffffu, cf, o);
+      const int tq = __shfl_up_sync(0xffffffffu, cq, o);
       if (lane >= o) {
         cs += ts;
+        cq += tq;
         cf += tf;
       }
     }
     if (a) {
       bs.act_pid[na + cf - 1] = p;
       bs.act_cum[na + cf - 1] = run + cs - sz;
+      bs.act_fcum[na + cf - 1] = runf + cq - sf;
     }
+    runf += __shfl_sync(0xffffffffu, cq, 31);
     run += __shfl_sync(0xffffffffu, cs, 31);
     na += __shfl_sync(0xffffffffu, cf, 31);
   }
   if (lane == 0) {
     bs.act_cum[na] = run;
+    bs.act_fcum[na] = runf;
     bs.act_n[0] = na;
   }
 }

@@ -27,8 +27,8 @@
 // and SM): evaluating each face once and the sparse tables is what counts.
 // Against one thread per element with dense tables, which evaluated every face
 // from both sides: 301x203 quad Q2 FP64 right-hand side 0.32 ms (0.77), 317x211
-// quad Q3 FP32 stage 70 us (303), 302x101 P2 triangles FP64 stage 143 us (240),
-// 200x4 quad Q1 FP64 stage 27 us (105; 13 us a launch is one FP64 flux's chain).
+// quad Q3 FP32 stage 53 us (303), 302x101 P2 triangles FP64 stage 136 us (240),
+// 200x4 quad Q1 FP64 stage 18 us (105; 9 us a launch is one FP64 flux's chain).
 #pragma once
 
 #include "rkdg_common.h"
@@ -67,7 +67,8 @@ __device__ __forceinline__ int quad_face_node(int lf, int q, int jn) {
 }
 __device__ __forceinline__ int quad_face_side(int lf) { return lf == 1 || lf == 2; }
 
-template <int G, int P, typename R, bool SPEED>
+// MAP: a batch with a map of the active work (prm.act_cum).
+template <int G, int P, typename R, bool SPEED, bool MAP>
 __global__ void __launch_bounds__(128)
     k_face_planar(const __grid_constant__ RhsParams prm, const R* __restrict__ u) {
   using E = El<G, P>;
@@ -82,11 +83,17 @@ __global__ void __launch_bounds__(128)
   }
   const int ne = prm.ne;
   const long long NDa = prm.ndofs;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int f = t / NQF, q = t - f * NQF;
   R lmax = R(0);
+  // MAP: CTAs run over the points of the active problems' faces
+  const int na = MAP ? *prm.act_n : 0, nfa = MAP ? prm.act_fcum[na] : prm.nface;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x, next;; t = next) {
+  next = t + gridDim.x * blockDim.x;
+  int f = t / NQF;
+  const int q = t - f * NQF;
   int pb = -1;
-  bool live = f < prm.nface;
+  bool live = f < nfa;
+  if (MAP && live) f = active_face(prm, na, f);
+  lmax = R(0);
   int4 face = make_int4(0, -1, 0, 0);
   int e1 = 0;
   R gamma = (R)prm.gamma, cov = (R)prm.covolume;
@@ -206,16 +213,16 @@ __global__ void __launch_bounds__(128)
       lmax = checked_speed(prm, sp, e1, pb);
     }
     if constexpr (!SPEED) {
-      R* out = (R*)prm.fslot + t;
+      R* out = (R*)prm.fslot + (long long)f * NQF + q;
       const long long nf = (long long)prm.nface * NQF;
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) out[k * nf] = PLAIN ? (F[k] * H.wf[q]) * jac : F[k] * jac;
     }
   }
-  if (prm.prob)
-    segmented_max_commit<R>(lmax, live ? pb : -1, prm.pmcs);
-  else
-    block_max_commit<R>(lmax, prm.mcs);
+  if (prm.prob) segmented_max_commit<R>(lmax, live ? pb : -1, prm.pmcs);
+  if (!MAP || (long long)next - threadIdx.x >= (long long)nfa * NQF) break;
+  }
+  if (!prm.prob) block_max_commit<R>(lmax, prm.mcs);
 }
 
 // Runge-Kutta combination at one value; hi (and lo, for a float pair) receive
