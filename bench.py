@@ -51,11 +51,11 @@ def workload_config(case, n_elem_side):
     }
 
 
-# DRAM bytes (read + write) per element and stage launch of the C2 stage
-# kernel k_rhs_hex_tile<2,float>: mean of the three stage launches of one RK
-# step captured with ncu on the 64^3 pulse itself (840.2 MB / 262,144
-# elements); traffic scales with the element count.
-TRAFFIC_BYTES_PER_ELEMENT_LAUNCH = 3205.0
+# DRAM bytes (read + write) per element and stage of the C2 stage kernels
+# k_face_hex<2,float> + k_node_hex<2,float>: mean of the three stages of one RK
+# step captured with ncu on the 48^3 pulse (533.5 MB / 110,592 elements);
+# traffic scales with the element count.
+TRAFFIC_BYTES_PER_ELEMENT_STAGE = 4824.0
 
 
 def algorithmic_bytes_per_step(N, ne, precision):
@@ -325,12 +325,12 @@ def run_ours(args, rank, world, local):
     achieved = bps / (ms_step / 1e3) / 1e9
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak,
-            "traffic": args.traffic_per_launch or TRAFFIC_BYTES_PER_ELEMENT_LAUNCH * ctx32.ne,
-            "traffic_source": "ncu dram bytes per launch, 64^3 capture (per element, scaled by elements)"
+            "traffic": args.traffic_per_launch or TRAFFIC_BYTES_PER_ELEMENT_STAGE * ctx32.ne,
+            "traffic_source": "ncu dram bytes per stage (two launches), 48^3 capture (per element, scaled by elements)"
                               if not args.traffic_per_launch else "command line",
             "peak_source": peak_src,
-            "kernel": ("k_rhs_hex_tile<2,float> (face-once tiled stage kernel, 3 launches per step)"
-                       if args.hex_kernel in (0, 5) else f"hexahedral kernel variant {args.hex_kernel}"),
+            "kernel": ("k_face_hex<2,float> + k_node_hex<2,float> (face pass and node pass, 6 launches per step)"
+                       if args.hex_kernel in (0, 3) else f"hexahedral kernel variant {args.hex_kernel}"),
             "algorithmic_bytes_per_launch": bps / STAGES}
 
     cpu = None

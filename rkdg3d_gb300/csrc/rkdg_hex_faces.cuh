@@ -31,7 +31,8 @@
 //
 // FP64, per RK step: 32^3 Q2 2.91 ms against 4.9 with the shared-face team
 // kernel (the FP64 pipe is active 83-86% of the time); 33x27x21 Q1 limited
-// 0.83 ms against 1.5 with the team face and element passes, which wrote the fluxes once per side and applied a dense mass inverse.
+// 0.83 ms against 1.5 with the team face and element passes, which wrote the
+// fluxes once per side and applied a dense mass inverse.
 #pragma once
 
 #include "rkdg_common.h"

@@ -81,8 +81,9 @@ __device__ __forceinline__ bool vertex_is_physical(const R* s, R gamma, R b) {
 // evaluated every equation's indicator, applied the factor nd times per value
 // and spilled on Q2 hexahedra: 31x29x23 hex Q2 FP32 24 us (99) and float pair
 // 32 us (287), 48x45x51 hex Q1 float pair 54 us (134), 33x27x21 hex Q1 FP64
-// 68 us (191), 524,288 P1 triangles FP64 245 us (459), FP32 47 us (45) and float
-// pair 71 us (76): there the arithmetic of the few values is what is left.
+// 40 us (191), 524,288 P1 triangles FP64 187 us (459; 254 with a division for
+// every point), FP32 43 us (45) and float pair 66 us (76): there the arithmetic
+// of the few values is what is left.
 // MAP: a batch with a map of the active work (prm.act_cum).
 template <int G, int P, typename R, bool DS, bool MAP>
 __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)

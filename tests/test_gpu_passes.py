@@ -158,3 +158,29 @@ def test_float_pair_split_and_join_are_exact(cuda):
     xd = dev(x)
     ctx.step(xd, 0.0)
     assert np.array_equal(xd.cpu().numpy(), want)
+
+
+def test_batch_larger_than_its_grid(cuda):
+    """A batch whose CTAs loop over the active work, also when it starts in the
+    middle of the lists: a small problem that ends after a few steps before a
+    large one.  Each is bit-identical to the same problem run alone."""
+    meshes = [M.quad_grid(20, 20, 0, 1, 0, 0.7), M.quad_grid(900, 700, 2, 3, 0, 0.7)]
+    ne = [m.num_elements for m in meshes]
+    case = box(QUAD, (2, 2), 1)
+    case.limiter = (LIM_MULTI, IND_BJ, FUN_MICHALAK, 1, 0)
+    case.mesh = cases.union_mesh(meshes)
+    ctx = Context(case.mesh, 1, device=0, precision=FP64)
+    cases.configure_context(case, ctx)
+    ctx.batch_setup([0, ne[0], sum(ne)], [1.4, 1.4], [0.005, 0.005])
+    x = random_state(ctx.node_coords(), b=0.005, seed=37, amp=0.05, vel=0.1)
+    xd = dev(x)
+    info = ctx.batch_run(xd, 5e-4, 0.3)
+    assert 0 < info["steps"][0] < info["steps"][1]
+    got = xd.cpu().numpy().reshape(4, -1)
+    for p, cut in enumerate((slice(0, 4 * ne[0]), slice(4 * ne[0], None))):
+        case.mesh = meshes[p]
+        one = Context(case.mesh, 1, device=0, precision=FP64)
+        cases.configure_context(case, one)
+        xs = dev(np.ascontiguousarray(x.reshape(4, -1)[:, cut]).ravel())
+        assert one.run(xs, 5e-4, 0.3)["steps"] == info["steps"][p]
+        assert np.array_equal(got[:, cut], xs.cpu().numpy().reshape(4, -1))
