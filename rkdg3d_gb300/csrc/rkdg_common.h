@@ -143,14 +143,14 @@ struct HexOpsPair {
 // and mb[lf][q][i] = (M^-1)[i][:] . B[lf][q][:] w_q.
 template <typename R>
 struct PlanarOps {
-  R b[54];
+  R b[108];
   R md[72];
   R mb[54];
   R lend[8];
   R wf[4];   // face-rule weights
-  // elements of at most four nodes, the dense operators of the element pass:
+  // the dense operators of the element pass (at most four nodes, Q2 quads):
   // eb[lf][q][j] traces (triangles: times w_q), ed[r][j][m] = D_r, em = M^-1
-  R eb[32], ed[32], em[16];
+  R eb[108], ed[162], em[81];
   R wm[16];  // cell-mean weights
 };
 struct PlanarOpsPair {

@@ -621,7 +621,7 @@ void planar_tables(const rkdg_ctx* c, rkdg::PlanarOpsPair& ops) {
   std::memset(&ops, 0, sizeof ops);
   for (int j = 0; j < nd; ++j) D.wm[j] = T.wmean[j];
   for (int q = 0; q < nqf; ++q) D.wf[q] = T.wf[q];
-  if (nd <= 4) {
+  if (nd <= 4 || (c->geom == RKDG_GEOM_SQUARE && c->p == 2)) {
     for (int lf = 0; lf < nfpe; ++lf)
       for (int q = 0; q < nqf; ++q)
         for (int j = 0; j < nd; ++j)
@@ -633,7 +633,7 @@ void planar_tables(const rkdg_ctx* c, rkdg::PlanarOpsPair& ops) {
       }
   }
   if (c->geom == RKDG_GEOM_SQUARE) {
-    for (int lf = 0; lf < nfpe && c->p == 1; ++lf)
+    for (int lf = 0; lf < nfpe && c->p <= 2; ++lf)
       for (int q = 0; q < nqf; ++q)
         for (int j = 0; j < nd; ++j) D.b[(lf * nqf + q) * nd + j] = T.B[lf][q][j];
     for (int i = 0; i < n1; ++i) {

@@ -17,7 +17,9 @@
 //      neq values instead of neq * nd.
 // FP32 elements of at most 16 values (Q1 quads, P1 triangles) run the second pass
 // with a thread per element (k_elem_planar): there the instructions around a
-// node's few values outnumber its arithmetic three to one.
+// node's few values outnumber its arithmetic three to one.  So do the FP32 Q2
+// quads of a batch, for the order of its sums: shocks limited over many steps
+// amplify any other rounding (half of such batches ended 1e-4 to 1e-3 apart).
 //
 // On quadrilaterals the mass, trace and derivative tables of the collocated
 // Gauss-Legendre basis are sparse (the mass matrix is diagonal, a face point
@@ -73,8 +75,9 @@ __global__ void __launch_bounds__(128)
     k_face_planar(const __grid_constant__ RhsParams prm, const R* __restrict__ u) {
   using E = El<G, P>;
   constexpr int DIM = 2, ND = E::ND, NEQ = E::NEQ, NFPE = E::NFPE, NQF = E::NQF, N1 = P + 1;
-  // FP32 Q1 quads: the plain arithmetic (see riemann()), traces from the dense table
-  constexpr bool PLAIN = G == 3 && P == 1 && std::is_same<R, float>::value;
+  // FP32 Q1 quads, and Q2 quads of a batch (many steps of limited shocks): the
+  // plain arithmetic (see riemann()), traces from the dense table
+  constexpr bool PLAIN = G == 3 && (P == 1 || (P == 2 && MAP)) && std::is_same<R, float>::value;
   __shared__ R sB[G == 2 || PLAIN ? NFPE * NQF * ND : 1];
   const PlanarOps<R>& H = planar_ops<R>(prm.pops);
   if constexpr (G == 2 || PLAIN) {
@@ -201,10 +204,10 @@ __global__ void __launch_bounds__(128)
         right_state<DIM>(bc.type, bc.state, s1, s2, n, gamma, cov, (R)prm.rgas);
       }
     }
-    if (none) {
+    // no integrator, or a non-physical state: no flux
 #pragma unroll
-      for (int k = 0; k < NEQ; ++k) F[k] = R(0);
-    } else {
+    for (int k = 0; k < NEQ; ++k) F[k] = R(0);
+    if (!none) {
       R sp;
       if constexpr (PLAIN)
         sp = riemann<DIM, R, true>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg);

@@ -160,6 +160,33 @@ def test_float_pair_split_and_join_are_exact(cuda):
     assert np.array_equal(xd.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("limited", [False, True])
+def test_batch_fp32_q2_close_to_fp64(cuda, limited):
+    """FP32 Q2 batches take the element pass: two steps against the FP64 batch
+    (node pass), a smooth state; and the failed problem between them, whose
+    state is non-physical, ends with finite values."""
+    meshes = [M.quad_grid(n, 3, 2 * i, 2 * i + 1, 0, 0.7) for i, n in enumerate((5, 4, 33))]
+    off = np.concatenate([[0], np.cumsum([m.num_elements for m in meshes])])
+    case = box(QUAD, (2, 2), 2)
+    if limited:
+        case.limiter = (LIM_MULTI, IND_BJ, FUN_VENKATAKRISHNAN, 1, 0)
+    case.mesh = cases.union_mesh(meshes)
+    out = {}
+    for prec in (FP64, FP32_BULK):
+        ctx = Context(case.mesh, 2, device=0, precision=prec)
+        cases.configure_context(case, ctx)
+        ctx.batch_setup(off, [1.4] * 3, [0.005] * 3)
+        x = random_state(ctx.node_coords(), b=0.005, seed=38, amp=0.01, vel=0.1).reshape(4, -1)
+        x[3, 9 * off[1]:9 * off[2]] = 1e-3  # less than the kinetic energy
+        xd = dev(x.ravel())
+        info = ctx.batch_run(xd, 1e19, dt0=1e-3, dt_mode=2, max_steps=2, limit_initial=False)
+        out[prec] = xd.cpu().numpy().reshape(4, -1)
+        assert np.isfinite(out[prec]).all()
+        assert list(info["steps"][[0, 2]]) == [2, 2] and info["steps"][1] < 0
+    for cut in (slice(0, 9 * off[1]), slice(9 * off[2], None)):
+        assert rel_l1(out[FP32_BULK][:, cut], out[FP64][:, cut]) < TOL[FP32_BULK]
+
+
 def test_batch_larger_than_its_grid(cuda):
     """A batch whose CTAs loop over the active work, also when it starts in the
     middle of the lists: a small problem that ends after a few steps before a
