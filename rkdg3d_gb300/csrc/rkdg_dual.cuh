@@ -125,12 +125,12 @@ template <int N>
 __device__ inline Dual<N> fmax(const Dual<N>& a, const Dual<N>& b) { return a.v >= b.v ? a : b; }
 template <int N>
 __device__ inline Dual<N> fmin(const Dual<N>& a, const Dual<N>& b) { return a.v <= b.v ? a : b; }
-// a^e for a > 0
+// a^e; a negative a has a power only where e is whole, a constant then
 template <int N>
 __device__ inline Dual<N> pow(const Dual<N>& a, const Dual<N>& e) {
   Dual<N> r;
   r.v = ::pow(a.v, e.v);
-  const double la = ::log(a.v);
+  const double la = a.v > 0.0 ? ::log(a.v) : 0.0;
   const double da = e.v * ::pow(a.v, e.v - 1.0);
 #pragma unroll
   for (int i = 0; i < N; ++i) r.d[i] = da * a.d[i] + r.v * la * e.d[i];

@@ -133,7 +133,9 @@ __device__ __forceinline__ void hll_vjp(FluxSide<DIM>& A, FluxSide<DIM>& B, cons
     xz = whole ? root_n(x, n, 0.5 * gm1 / gamma) : exp2(log2(x) / iz);
     den = cL + cR * xz;
     t = (cL + cR - 0.5 * gm1 * (u2 - u1)) * rcp(den);
-    if (whole) {
+    if (t < 0.0) {
+      pl = trrs_negative_base(t, gamma);
+    } else if (whole) {
       pl = t;
       for (int i = 1; i < n; ++i) pl *= t;
     } else {

@@ -583,6 +583,19 @@ __device__ __forceinline__ float powr<float>(float a, float e) {
   return exp2f(e * log2f(a));
 }
 
+// (A/B)^(1/z) of TRRS where A/B is negative: velocity jumps above
+// 2 (cL + cR)/(gamma - 1), which open a vacuum.  The reference's pow
+// (physics.cpp:338) gives NaN there unless 1/z as it computes it, in FP64, is
+// exactly a whole number (10, 6, 4 for gamma = 1.25, 1.5, 2; for 4/3 and 1.2
+// rounding leaves a little more than 8 and 12), and NaN counts as no shock, like
+// the negative value of an odd power.  So: the even power, or 0.  (FP32 asks for
+// the FP32 gamma.)
+__device__ __forceinline__ double trrs_negative_base(double t, double gamma) {
+  const double iz = 1.0 / (0.5 * (gamma - 1.0) / gamma);
+  if (iz != 2.0 * floor(0.5 * iz)) return 0.0;
+  return exp2(iz * log2(-t));
+}
+
 // Wave-speed estimates on rotated states: TRRS ComputeToroCharSpeeds
 // (physics.cpp:309-350) or Einfeldt ComputeEinfeldtCharSpeeds (269-296).
 // Only lambda[0] and lambda[dim+1] are used by the solvers.
@@ -605,9 +618,10 @@ __device__ __forceinline__ void wave_speeds(const R* s1, const R* s2, R p1, R p2
   }
   const R uL = fdv(s1[1], s1[0]), uR = fdv(s2[1], s2[0]);
   const R z = fdv(R(0.5) * (gamma - R(1)), gamma);
-  const R pStar = powr(fdv(cL + cR - R(0.5) * (gamma - R(1)) * (uR - uL),
-                           fdv(cL, powr(p1, z)) + fdv(cR, powr(p2, z))),
-                       fdv(R(1), z));
+  const R base = fdv(cL + cR - R(0.5) * (gamma - R(1)) * (uR - uL), fdv(cL, powr(p1, z)) + fdv(cR, powr(p2, z)));
+  R pStar = powr(base, fdv(R(1), z));
+  if constexpr (std::is_same<R, float>::value)
+    if (base < 0.0f) pStar = (float)trrs_negative_base((double)base, (double)gamma);
   const R qL = pStar > p1 ? fsq(R(1) + fdv(R(0.5) * (gamma + R(1)) * (fdv(pStar, p1) - R(1)), gamma))
                           : R(1);
   const R qR = pStar > p2 ? fsq(R(1) + fdv(R(0.5) * (gamma + R(1)) * (fdv(pStar, p2) - R(1)), gamma))
@@ -649,7 +663,9 @@ __device__ __forceinline__ void trrs_speeds(R uL, R uR, R cL, R cR, R pL, R pR, 
   const R a = cL + cR - R(0.5) * gm1 * (uR - uL);
   const R t = quot(a, cL + cR * xz);
   R pl;  // pStar / pL
-  if (whole) {
+  if (t < R(0)) {
+    pl = R(trrs_negative_base((double)t, (double)gamma));
+  } else if (whole) {
     pl = t;
     for (int i = 1; i < n; ++i) pl *= t;
   } else {
