@@ -13,6 +13,7 @@
 
 #include "rkdg_common.h"
 #include "rkdg_physics.cuh"
+#include "rkdg_speed_bound.h"
 
 namespace rkdg {
 
@@ -139,31 +140,11 @@ __device__ __forceinline__ float cut_f32(double x) {
   return __uint_as_float(((t ^ 0x40000000u) & 0x7fffffffu) | ((unsigned)hi & 0x80000000u));
 }
 
-// Wave speeds only (the initial time step): which face points can be left at
-// an FP32 estimate.  A trace cut to FP32 and summed errs by less than 4e-6 of
-// the nodal maximum (nine roundings of 6e-8 and the cut's 1.2e-7, times a
-// Lebesgue sum below 4).  Where density and total energy are at least 3/4 of
-// their nodal maxima and the momenta at most sqrt(3 rho E), that is 2e-5 of E in
-// the internal energy, hence 4e-5 E/ie of |u| + c; TRRS speeds take that
-// through pStar's power of at most 16 under a root, 6.4e-4 E/ie.  A point need not
-// be evaluated in FP64 if its estimate lies below the largest FP64 speed so far
-// by more than that (and such a state is physical).
-// speed_state_margin: E / ie of a state, or a value too large for any margin.
-__device__ __forceinline__ float speed_state_margin(const float* s, int dim, const float* top, int stride, float b) {
-  float m2 = 0.0f, mt = 0.0f;
-  for (int d = 0; d < dim; ++d) {
-    m2 += s[1 + d] * s[1 + d];
-    mt = fmaxf(mt, top[(1 + d) * stride]);
-  }
-  const float r = s[0], E = s[1 + dim], re = r * E, ie = re - 0.5f * m2;  // rho times both energies
-  const bool ok = r >= 0.75f * top[0] && E >= 0.75f * top[(1 + dim) * stride] && mt * mt <= 3.0f * re &&
-                  r > 1e-15f && E > 1e-15f && E < 1e15f && r < 1e15f && ie >= 0.02f * re && 1.0f - r * b >= 0.5f;
-  return ok ? __fdividef(re, ie) : 1e9f;
-}
-__device__ __forceinline__ bool speed_below(float sp, float margin, const unsigned long long* mcs, int rs, int avg) {
+// The bound of a face point's speed (rkdg_speed_bound.h) lies below the largest
+// FP64 speed so far.
+__device__ __forceinline__ bool speed_below(float bound, const unsigned long long* mcs) {
   const double top = __longlong_as_double((long long)*(const volatile unsigned long long*)mcs);
-  const float m = (rs != 0 && avg == 0 ? 7e-4f : 5e-5f) * margin;
-  return sp >= 0.0f && m < 0.1f && sp * (1.0f + m) < (float)top * 0.999999f;
+  return bound < (float)top * 0.999999f;
 }
 
 __device__ __forceinline__ void flag_error(int* err, int code, int where) {

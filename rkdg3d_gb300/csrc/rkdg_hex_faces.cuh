@@ -233,10 +233,9 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
   block_max_commit<R>(lmax, prm.mcs);
 }
 
-// The largest face wave speed of an FP64 state.  Every face point is estimated
-// in FP32 first; only faces with a point that could hold the maximum, or whose
-// estimate is not to be trusted (speed_state_margin), and boundary faces are
-// evaluated in FP64.  48x45x51 Q1, HLL with TRRS speeds:
+// The largest face wave speed of an FP64 state.  Every face point is bounded in
+// FP32 first (rkdg_speed_bound.h); only faces with a point that could hold the
+// maximum, or that has no bound, and boundary faces are evaluated in FP64.  48x45x51 Q1, HLL with TRRS speeds:
 // 0.66 ms against 1.13 for every point in FP64; 48^3 Q2 Rusanov 0.4 against 1.4.
 template <int P>
 __global__ void __launch_bounds__(HexFaces<P>::NT)
@@ -299,7 +298,7 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
     const int4 fc = sF[fl];
     if (fc.y >= 0) {
       const int op = fc.z >> 6, t2 = op ? square_op(op, t1 % NQ1, t1 / NQ1, NQ1) : t1;
-      float s1[NEQ], s2[NEQ], F[NEQ], n[3];
+      float s1[NEQ], s2[NEQ], n[3];
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) {
         s1[k] = sb.f.t[0][k][fl][t1];
@@ -309,10 +308,10 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
       for (int c = 0; c < 3; ++c)
         n[c] = (float)__ldg((const double*)prm.fgeo + (long long)((fc.z & 7) * 4 + c) * ne + fc.x);
       const float g = (float)prm.gamma, b = (float)prm.covolume;
-      const float mg = fmaxf(speed_state_margin(s1, 3, sb.f.top + fl, 2 * FB, b),
-                             speed_state_margin(s2, 3, sb.f.top + FB + fl, 2 * FB, b));
-      const bool ok = mg < 1e8f && speed_below(riemann<3>(s1, s2, make_frame<3, float>(n), F, g, b, prm.rs, prm.avg),
-                                               mg, prm.mcs, prm.rs, prm.avg);
+      SpeedSide A, B;
+      const bool ok = speed_side<3>(s1, sb.f.top + fl, 2 * FB, n, g, b, A) &&
+                      speed_side<3>(s2, sb.f.top + FB + fl, 2 * FB, n, g, b, B) &&
+                      speed_below(speed_bound(A, B, g, prm.rs, prm.avg, prm.quirks & 1), prm.mcs);
       if (!ok) sNeed[fl] = 1;
     }
   }

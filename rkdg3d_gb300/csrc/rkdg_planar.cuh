@@ -156,10 +156,10 @@ __global__ void __launch_bounds__(128)
     };
     R s1[NEQ], s2[NEQ], F[NEQ];
     if constexpr (SPEED) {
-      // estimated in FP32, evaluated in FP64 only where the point could hold
-      // the maximum (see speed_state_margin)
+      // bounded in FP32, evaluated in FP64 only where the point could hold the
+      // maximum
       if (face.y >= 0) {
-        float a1[NEQ], a2[NEQ], Ff[NEQ], nf[DIM], top[2][NEQ];
+        float a1[NEQ], a2[NEQ], nf[DIM], top[2][NEQ];
         auto est = [&](int e, int lf, int qq, float* s, float* tp) {
           const R* ue = u + (long long)e * ND;
           constexpr int NT = G == 3 ? N1 : ND;  // terms of the trace
@@ -184,9 +184,9 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
         for (int c = 0; c < DIM; ++c) nf[c] = (float)n[c];
         const float g = (float)gamma, b = (float)cov;
-        const float mg = fmaxf(speed_state_margin(a1, DIM, top[0], 1, b), speed_state_margin(a2, DIM, top[1], 1, b));
-        if (mg < 1e8f && speed_below(riemann<DIM>(a1, a2, make_frame<DIM, float>(nf), Ff, g, b, prm.rs, prm.avg), mg,
-                                     prm.prob ? prm.pmcs + pb : prm.mcs, prm.rs, prm.avg))
+        SpeedSide A, B;
+        if (speed_side<DIM>(a1, top[0], 1, nf, g, b, A) && speed_side<DIM>(a2, top[1], 1, nf, g, b, B) &&
+            speed_below(speed_bound(A, B, g, prm.rs, prm.avg, prm.quirks & 1), prm.prob ? prm.pmcs + pb : prm.mcs))
           skip = true;
       }
     }
