@@ -65,7 +65,6 @@ struct RefTables {
   float2 Bl32[RKDG_MAX_ND][RKDG_MAX_NFPE * RKDG_MAX_NQL];
   float Bv32[RKDG_MAX_ND][RKDG_MAX_NV];
   double wmean[RKDG_MAX_ND];                 // cell-mean weights (sum = 1)
-  float2 wmean32[RKDG_MAX_ND];               // the same as float pairs
   // 1D tables for the sum-factorised tensor kernels
   double l1d[RKDG_MAX_NQF][8];   // 1D basis at 1D face-rule points  [a][j]
   double w1d[8];                 // 1D face-rule weights

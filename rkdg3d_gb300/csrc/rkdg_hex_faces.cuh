@@ -360,6 +360,48 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
   block_max_commit<double>(lmax, prm.mcs);
 }
 
+// Part of the mean of an element's float values (hi, and lo where given) with the
+// weights wm of the nodes, to FP64: the limiter's switches read the mean.  Order 1
+// takes all nodes at once, order 2 a plane of nine.  The values are summed in fixed
+// point with 32 bits below the last place of the largest one (nothing is lost but
+// what lies 2^-56 below it), those of one weight together (nodes of as many middle
+// indices), so that a mean takes one or nine FP64 products instead of 8 or 27 on
+// a pipe that issues two per clock and SM: those cost 31x29x23 Q2 limited 17 us a
+// stage.
+template <int P>
+__device__ __forceinline__ double pair_mean(const float* hi, const float* lo, const double* __restrict__ wm) {
+  constexpr int N = P == 2 ? 9 : 8, NC = P == 2 ? 3 : 1;
+  unsigned top = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) top = max(top, __float_as_uint(hi[j]) & 0x7fffffffu);
+  const int emax = (int)(top >> 23);
+  double m = 0.0;
+  if (emax < 64 || emax == 255) {  // tiny or not finite
+    for (int j = 0; j < N; ++j) m += wm[j] * (widen(hi[j]) + (lo ? widen(lo[j]) : 0.0));
+    return m;
+  }
+  auto fixed = [&](float x) {
+    const unsigned b = __float_as_uint(x);
+    const int e = (int)((b >> 23) & 0xff);
+    const unsigned mant = e ? (b & 0x7fffffu) | 0x800000u : 0u;
+    const long long v = (long long)(((unsigned long long)mant << 32) >> min(emax - e, 63));
+    return (b >> 31) ? -v : v;
+  };
+  long long S[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) S[c] = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const int c = P == 2 ? (j % 3 == 1) + (j / 3 == 1) : 0;
+    S[c] += fixed(hi[j]);
+    if (lo) S[c] += fixed(lo[j]);
+  }
+  constexpr int AT[3] = {0, 1, 4};  // a node of each weight
+#pragma unroll
+  for (int c = 0; c < NC; ++c) m += wm[AT[c]] * (double)S[c];
+  return m * __hiloint2double((emax - 182 + 1023) << 20, 0);
+}
+
 template <int P, typename R>
 __global__ void __launch_bounds__(HexFaces<P>::NTN)
     k_node_hex(const __grid_constant__ RhsParams prm, const R* __restrict__ u,
@@ -537,30 +579,39 @@ __global__ void __launch_bounds__(HexFaces<P>::NTN)
   }
   if (need_means) {
     __syncthreads();
-    // cell means, one (element, equation) per thread
+    // cell means, one (element, equation) per thread; float pairs of order 2: a
+    // plane of nodes per thread, three neighbouring lanes
     const double* wm = prm.tab->wmean;
-    for (int t = tid; t < EPB * NEQ; t += NT) {
+    constexpr int PL = F32 && P == 2 ? 3 : 1, W = 32 / PL;  // W means per warp
+    static_assert(PL == 1 || EPB * NEQ <= NT / 32 * W, "one round of whole warps");
+    const int lane = tid & 31, pl = lane % PL;
+    for (int t = (tid >> 5) * W + lane / PL; PL > 1 || t < EPB * NEQ; t += NT) {
       const int k = t / EPB, s = t - k * EPB, em = blockIdx.x * EPB + s;
-      if (em >= ne) continue;
-      if constexpr (std::is_same<R, double>::value) {
-        double m = 0.0;
+      const bool on = t < EPB * NEQ && lane < PL * W && em < ne;
+      double m = 0.0;
+      if (on) {
+        const int j0 = s * NP + pl * NF2;
+        if constexpr (F32) {
+          m = pair_mean<P>(sG[0][k] + j0, ep.final_stage ? sG[1][k] + j0 : nullptr, wm + pl * NF2);
+        } else {
 #pragma unroll
-        for (int j = 0; j < ND; ++j) m += wm[j] * sG[0][k][s * NP + j];
-        store_mean(ep, (long long)k * ne + em, m);
-      } else {
-        float mh = 0.0f, ml = 0.0f, ph, pl;
-#pragma unroll
-        for (int j = 0; j < ND; ++j) {
-          const float2 w = prm.tab->wmean32[j];
-          ds_mul_f(w.x, w.y, sG[0][k][s * NP + j], ph, pl);
-          ds_add(mh, ml, ph, pl);
-          if (ep.final_stage) ds_add(mh, ml, w.x * sG[1][k][s * NP + j], 0.0f);
+          for (int j = 0; j < ND; ++j) m += wm[j] * sG[0][k][j0 + j];
         }
-        if (ep.means32)
-          ep.means32[(long long)k * ne + em] = make_float2(mh, ml);
-        else
-          ep.means[(long long)k * ne + em] = (double)mh + (double)ml;
       }
+      if constexpr (PL > 1) m += __shfl_down_sync(0xffffffffu, m, 1) + __shfl_down_sync(0xffffffffu, m, 2);
+      if (on && pl == 0) {
+        if constexpr (F32) {
+          float h, l;
+          split_value(m, h, l);
+          if (ep.means32)
+            ep.means32[(long long)k * ne + em] = make_float2(h, l);
+          else
+            ep.means[(long long)k * ne + em] = m;
+        } else {
+          store_mean(ep, (long long)k * ne + em, m);
+        }
+      }
+      if (PL > 1) break;
     }
   }
   block_max_commit<R, std::is_same<R, double>::value>(lmax, prm.mcs);

@@ -366,10 +366,7 @@ bool build_ref_tables(int geom, int p, RefTables& T, std::vector<FacePoint>* fpt
       for (int j = 0; j < nd; ++j) m0[j] += r.w[q] * phi[j];
     }
     for (int j = 0; j < nd; ++j) tot += m0[j];
-    for (int j = 0; j < nd; ++j) {
-      const double w = T.wmean[j] = m0[j] / tot;
-      T.wmean32[j] = {(float)w, (float)(w - (double)(float)w)};
-    }
+    for (int j = 0; j < nd; ++j) T.wmean[j] = m0[j] / tot;
   }
   // face points of the right-hand side
   {
