@@ -147,7 +147,7 @@ struct PlanarOps {
   R mb[54];
   R lend[8];
   R wf[4];   // face-rule weights
-  // the dense operators of the element pass (at most four nodes, Q2 quads):
+  // the dense operators of the element pass (at most four nodes) and of Q2 quads:
   // eb[lf][q][j] traces (triangles: times w_q), ed[r][j][m] = D_r, em = M^-1
   R eb[108], ed[162], em[81];
   R wm[16];  // cell-mean weights

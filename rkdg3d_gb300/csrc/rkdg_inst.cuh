@@ -54,13 +54,6 @@ cudaError_t launch_planar(const RhsParams& prm, const R* u, const EpiParams<R>& 
   if (e != cudaSuccess) return e;
   using S = Planar<G, P>;
   constexpr bool F32 = std::is_same<R, float>::value;
-  if constexpr (F32 && G == 3 && P == 2) {
-    if (prm.act_cum) {
-      const int eb = prm.block ? generic_block(prm.block) : spread_block(prm.ne, 128);
-      k_elem_planar<G, P, R><<<(prm.ne + eb - 1) / eb, eb, 0, st>>>(prm, u, ep);
-      return cudaGetLastError();
-    }
-  }
   if constexpr (F32 && El<G, P>::NEQ * El<G, P>::ND <= 16) {
     const int eb = prm.block ? std::min(generic_block(prm.block), 128) : spread_block(prm.ne, 128);
     k_elem_planar<G, P, R><<<(prm.ne + eb - 1) / eb, eb, 0, st>>>(prm, u, ep);

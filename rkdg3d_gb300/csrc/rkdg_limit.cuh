@@ -93,10 +93,10 @@ __global__ void __launch_bounds__(LimTeam<G, P>::MAX_BLOCK)
   constexpr int DIM = E::DIM, ND = E::ND, NEQ = E::NEQ, NFPE = E::NFPE, NQL = E::NQL, NV = E::NV;
   constexpr int L = T::L, NPT = T::NPT, NDP = T::NDP;
   constexpr bool F32 = std::is_same<R, float>::value;
-  // float states of hexahedra, small planar elements and batches: the factor is
+  // float states of hexahedra, small planar elements and Q2 quads: the factor is
   // applied nd times as the reference does (their limited runs amplify another
   // rounding, see riemann()); a float pair's power rounds far below that
-  constexpr bool REPEAT = F32 && (ND <= 4 || (G == 5 && !DS) || (G == 3 && P == 2 && MAP));
+  constexpr bool REPEAT = F32 && (ND <= 4 || (G == 5 && !DS) || (G == 3 && P == 2));
   // the means' low parts: FP64 hexahedra (on 200x4 quads the extra pass over
   // the values is 6% of a step, and a planar mesh's means change more per step)
   constexpr bool LOW = !F32 && G == 5;

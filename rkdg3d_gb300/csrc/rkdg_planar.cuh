@@ -17,9 +17,7 @@
 //      neq values instead of neq * nd.
 // FP32 elements of at most 16 values (Q1 quads, P1 triangles) run the second pass
 // with a thread per element (k_elem_planar): there the instructions around a
-// node's few values outnumber its arithmetic three to one.  So do the FP32 Q2
-// quads of a batch, for the order of its sums: shocks limited over many steps
-// amplify any other rounding (half of such batches ended 1e-4 to 1e-3 apart).
+// node's few values outnumber its arithmetic three to one.
 //
 // On quadrilaterals the mass, trace and derivative tables of the collocated
 // Gauss-Legendre basis are sparse (the mass matrix is diagonal, a face point
@@ -75,9 +73,9 @@ __global__ void __launch_bounds__(128)
     k_face_planar(const __grid_constant__ RhsParams prm, const R* __restrict__ u) {
   using E = El<G, P>;
   constexpr int DIM = 2, ND = E::ND, NEQ = E::NEQ, NFPE = E::NFPE, NQF = E::NQF, N1 = P + 1;
-  // FP32 Q1 quads, and Q2 quads of a batch (many steps of limited shocks): the
-  // plain arithmetic (see riemann()), traces from the dense table
-  constexpr bool PLAIN = G == 3 && (P == 1 || (P == 2 && MAP)) && std::is_same<R, float>::value;
+  // FP32 Q1 and Q2 quads: the plain arithmetic (see riemann()), traces from the
+  // dense table
+  constexpr bool PLAIN = G == 3 && P <= 2 && std::is_same<R, float>::value;
   __shared__ R sB[G == 2 || PLAIN ? NFPE * NQF * ND : 1];
   const PlanarOps<R>& H = planar_ops<R>(prm.pops);
   if constexpr (G == 2 || PLAIN) {
@@ -300,10 +298,23 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
   constexpr int DIM = 2, ND = E::ND, NEQ = E::NEQ, NFPE = E::NFPE, NQF = E::NQF, N1 = P + 1;
   constexpr int NT = S::threads(EPB);
   constexpr int NP = ND | 1;  // odd element stride in shared memory
+  // FP32 Q2 quads: the plain arithmetic (see riemann()), and the terms in the
+  // order in which dense tables, their zeros left out, add them: the faces, then the
+  // nodes of the row and the column in ascending order, then the inverse mass.  Many
+  // limited steps part by 1e-4 to 1e-3 under any other rounding.  Batches and
+  // problems alone take the same arithmetic.  9 x 1563 x 4 quads, 20 limited steps:
+  // 4.87 ms against 6.39 with a thread per element; alone, 301x203 quads, 111 us a step
+  // against 105 with the contravariant node fluxes (limited 207 against 186, with the
+  // factor applied nd times).
+  constexpr bool PLAIN = G == 3 && P == 2 && std::is_same<R, float>::value;
+  constexpr int NTERM = 2 * N1;
   __shared__ R sG[DIM][NEQ][EPB * NP];
   // triangles: MD_r[i][m] and MB[i][lf][q], node i fastest; quadrilaterals:
-  // d1[i][m] / w_i and lend[side][i] / w_i
-  __shared__ R sMD[G == 2 ? DIM * ND * ND : N1 * N1], sMB[G == 2 ? NFPE * NQF * ND : 2 * N1];
+  // d1[i][m] / w_i and lend[side][i] / w_i; PLAIN: each node's D_r[i][m] in order
+  // (places in sG: sAt), 1 / w_i and traces [lf][i]
+  __shared__ R sMD[G == 2 ? DIM * ND * ND : (PLAIN ? ND * NTERM + ND : N1 * N1)];
+  __shared__ R sMB[G == 2 ? NFPE * NQF * ND : (PLAIN ? NFPE * ND : 2 * N1)];
+  __shared__ int sAt[PLAIN ? ND * NTERM : 1];
   const PlanarOps<R>& H = planar_ops<R>(prm.pops);
   const int tid = threadIdx.x, ne = prm.ne;
   const long long NDa = prm.ndofs;
@@ -311,8 +322,25 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
   int e = blockIdx.x * EPB + sl, pb = -1;
   // batched problems with a map of the active work: CTAs past it are idle
   if (prm.act_cum && (int)(blockIdx.x * EPB) >= prm.act_cum[*prm.act_n]) return;
-  for (int t = tid; t < (G == 2 ? DIM * ND * ND : N1 * N1); t += NT) sMD[t] = H.md[t];
-  for (int t = tid; t < (G == 2 ? NFPE * NQF * ND : 2 * N1); t += NT) sMB[t] = H.mb[t];
+  if constexpr (PLAIN) {
+    for (int t = tid; t < ND * NTERM; t += NT) {
+      const int n = t / NTERM, x = n % N1, y = n / N1, o = t - n * NTERM - y;
+      // the column below, the row with the node's own column term after its row
+      // term, the column above
+      const bool row = o >= 0 && o <= N1 && o != x + 1;
+      const int m = row ? N1 * y + (o <= x ? o : o - 1) : x + N1 * (o < 0 ? o + y : (o == x + 1 ? y : y + o - N1));
+      sMD[t] = H.ed[((row ? 0 : 1) * ND + n) * ND + m];
+      sAt[t] = (row ? 0 : NEQ * EPB * NP) + m;
+    }
+    for (int t = tid; t < ND; t += NT) sMD[ND * NTERM + t] = H.em[t * ND + t];
+    for (int t = tid; t < NFPE * ND; t += NT) {
+      const int lf = t / ND, n = t - lf * ND, x = (lf & 1) ? n / N1 : n % N1;
+      sMB[t] = H.b[(lf * NQF + (lf >= 2 ? N1 - 1 - x : x)) * ND + n];
+    }
+  } else {
+    for (int t = tid; t < (G == 2 ? DIM * ND * ND : N1 * N1); t += NT) sMD[t] = H.md[t];
+    for (int t = tid; t < (G == 2 ? NFPE * NQF * ND : 2 * N1); t += NT) sMB[t] = H.mb[t];
+  }
   R gamma = (R)prm.gamma, cov = (R)prm.covolume;
   bool live = sl < EPB && e < ne;
   double dts = 1.0;
@@ -361,41 +389,66 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
                        : ((const R*)prm.egeo)[(long long)(r * DIM + d) * ne + e];
     idet = ng ? ng[((long long)(DIM * DIM) * ND + i) * ne + e]
               : ((const R*)prm.egeo)[(long long)(DIM * DIM) * ne + e];
-    const NodeFlux<DIM, R> N(st, gamma, cov);
-    lmax = N.speed;
+    if constexpr (PLAIN) {
+      R F[NEQ][DIM];
+      lmax = flux_and_speed<DIM>(st, F, gamma, cov);
 #pragma unroll
-    for (int r = 0; r < DIM; ++r) {
-      R G[NEQ];
-      N.contra(st, adj[r], G);
+      for (int r = 0; r < DIM; ++r)
 #pragma unroll
-      for (int k = 0; k < NEQ; ++k) sG[r][k][sl * NP + i] = G[k];
+        for (int k = 0; k < NEQ; ++k) sG[r][k][sl * NP + i] = fmaf(adj[r][1], F[k][1], adj[r][0] * F[k][0]);
+    } else {
+      const NodeFlux<DIM, R> N(st, gamma, cov);
+      lmax = N.speed;
+#pragma unroll
+      for (int r = 0; r < DIM; ++r) {
+        R G[NEQ];
+        N.contra(st, adj[r], G);
+#pragma unroll
+        for (int k = 0; k < NEQ; ++k) sG[r][k][sl * NP + i] = G[k];
+      }
     }
   }
+  const R* fx = (const R*)prm.fslot;
+  const long long nf = (long long)prm.nface * NQF;
+  // a quad's faces: the slot of each, its side and direction
+  auto quad_faces = [&]() {
+    const int jx = i % N1, jy = i / N1;
+#pragma unroll
+    for (int lf = 0; lf < NFPE; ++lf) {
+      const int ref = prm.fref[lf * ne + e];
+      const int t = (lf & 1) ? jy : jx;
+      int q = lf >= 2 ? N1 - 1 - t : t;
+      if (ref & 1) q = N1 - 1 - q;
+      const R b = PLAIN ? sMB[lf * ND + i] : sMB[quad_face_side(lf) * N1 + ((lf & 1) ? jx : jy)];
+      const R c = (ref & 2) ? b : -b;
+      const R* p = fx + (long long)(ref >> 2) * NQF + q;
+#pragma unroll
+      for (int k = 0; k < NEQ; ++k) acc[k] += c * p[k * nf];
+    }
+  };
   __syncthreads();
   if (live) {
-    // faces: the slot of each, its side and direction
-    const R* fx = (const R*)prm.fslot;
-    const long long nf = (long long)prm.nface * NQF;
     if constexpr (G == 3) {
       const int jx = i % N1, jy = i / N1;
+      if constexpr (PLAIN) {
+        quad_faces();
+        const R* g = &sG[0][0][sl * NP];
 #pragma unroll
-      for (int m = 0; m < N1; ++m) {
-        const R d0 = sMD[jx * N1 + m], d1 = sMD[jy * N1 + m];
+        for (int o = 0; o < NTERM; ++o) {
+          const R d = sMD[i * NTERM + o];
+          const int at = sAt[i * NTERM + o];
 #pragma unroll
-        for (int k = 0; k < NEQ; ++k)
-          acc[k] += d0 * sG[0][k][sl * NP + m + N1 * jy] + d1 * sG[1][k][sl * NP + jx + N1 * m];
-      }
+          for (int k = 0; k < NEQ; ++k) acc[k] += d * g[k * EPB * NP + at];
+        }
+      } else {
 #pragma unroll
-      for (int lf = 0; lf < NFPE; ++lf) {
-        const int ref = prm.fref[lf * ne + e];
-        const int t = (lf & 1) ? jy : jx;
-        int q = lf >= 2 ? N1 - 1 - t : t;
-        if (ref & 1) q = N1 - 1 - q;
-        const R b = sMB[quad_face_side(lf) * N1 + ((lf & 1) ? jx : jy)];
-        const R c = (ref & 2) ? b : -b;
-        const R* p = fx + (long long)(ref >> 2) * NQF + q;
+        for (int m = 0; m < N1; ++m) {
+          const R d0 = sMD[jx * N1 + m], d1 = sMD[jy * N1 + m];
 #pragma unroll
-        for (int k = 0; k < NEQ; ++k) acc[k] += c * p[k * nf];
+          for (int k = 0; k < NEQ; ++k)
+            acc[k] += d0 * sG[0][k][sl * NP + m + N1 * jy] + d1 * sG[1][k][sl * NP + jx + N1 * m];
+        }
+        quad_faces();
       }
     } else {
 #pragma unroll
@@ -423,12 +476,21 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
       const int ix = prm.ncidx[e];
       if (ix >= 0) {
         const R* xf = (const R*)prm.xface + (long long)ix * NEQ * ND;
-        for (int j = 0; j < ND; ++j) {
-          const R m = (R)prm.tab->Minv[i][j];
+        if constexpr (PLAIN) {
 #pragma unroll
-          for (int k = 0; k < NEQ; ++k) acc[k] += m * xf[k * ND + j];
+          for (int k = 0; k < NEQ; ++k) acc[k] += xf[k * ND + i];
+        } else {
+          for (int j = 0; j < ND; ++j) {
+            const R m = (R)prm.tab->Minv[i][j];
+#pragma unroll
+            for (int k = 0; k < NEQ; ++k) acc[k] += m * xf[k * ND + j];
+          }
         }
       }
+    }
+    if constexpr (PLAIN) {
+#pragma unroll
+      for (int k = 0; k < NEQ; ++k) acc[k] *= sMD[ND * NTERM + i];
     }
   }
   const bool need_means = ep.mode == 1 && (ep.means || ep.means32);
