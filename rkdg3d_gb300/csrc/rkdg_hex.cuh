@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(256)
           const BCSlot& bc = prm.bc[-2 - nb];
           right_state<3>(bc.type, bc.state, s1, s2, n, gamma, cov, (R)prm.rgas);
         }
-        R F[NEQ];
+        R F[NEQ] = {};  // a non-physical state leaves it: no flux
         const R sp = checked_speed(prm, riemann<3, R, true>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e);
         lmax = fmax(lmax, sp);
         const R sg = side ? R(1) : R(-1);

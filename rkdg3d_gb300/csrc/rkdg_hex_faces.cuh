@@ -170,10 +170,10 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
           right_state<3>(bc.type, bc.state, s1, s2, n, gamma, cov, (R)prm.rgas);
         }
       }
-      if (none) {
+      // no integrator, or a non-physical state: no flux
 #pragma unroll
-        for (int k = 0; k < NEQ; ++k) F[k] = R(0);
-      } else {
+      for (int k = 0; k < NEQ; ++k) F[k] = R(0);
+      if (!none) {
         R sp;
         if constexpr (F32) {
           const R n[3] = {sFr[fl][0], sFr[fl][1], sFr[fl][2]};

@@ -477,7 +477,7 @@ __device__ __forceinline__ void warp_fluxes(const int LF, const RhsParams& prm, 
       const BCSlot& bc = prm.bc[-2 - nb];
       right_state<3>(bc.type, bc.state, s1, s2, n, gamma, cov, (R)prm.rgas);
     }
-    R F[NEQ];
+    R F[NEQ] = {};  // a non-physical state leaves it: no flux
     const R sp = checked_speed(prm, riemann<3, R, true>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e0 + el);
     lmax = fmax(lmax, sp);
     const R w = (side ? R(1) : R(-1)) * wf[q] * jac;
@@ -597,7 +597,7 @@ __device__ __forceinline__ void shared_rounds(const RhsParams& prm, const R* __r
         const BCSlot& bc = prm.bc[-2 - nb];
         right_state<3>(bc.type, bc.state, s1, s2, n, gamma, cov, (R)prm.rgas);
       }
-      R F[NEQ];
+      R F[NEQ] = {};  // a non-physical state leaves it: no flux
       const R sp = checked_speed(prm, riemann<3, R, true>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), S.el[fs]);
       lmax = fmax(lmax, sp);
       const R w = wf[q] * jac;

@@ -223,7 +223,7 @@ __device__ __forceinline__ void tile_fluxes(const RhsParams& prm, const HexTile&
   for (int pt = threadIdx.x; pt < npt; pt += NT) {
     TilePoint<R> A;
     tile_point<P, R>(prm, T, ax, pt, sT, sH, eg, perm, fab, wf, gamma, cov, A);
-    R F[5];
+    R F[5] = {};  // a non-physical state leaves it: no flux
     const R sp = riemann<3, R, true>(A.s1, A.s2, A.n, F, gamma, cov, prm.rs, prm.avg);
     if (!A.zero) lmax = fmax(lmax, checked_speed(prm, sp, A.ge));
     tile_point_store(A, F);

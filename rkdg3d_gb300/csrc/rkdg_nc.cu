@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kNcFaceThreads) k_nc_face(const __grid_constan
     }
     const R gamma = (R)(pb >= 0 ? prm.pgamma[pb] : prm.gamma);
     const R cov = (R)(pb >= 0 ? prm.pcov[pb] : prm.covolume);
-    R F[NEQ];
+    R F[NEQ] = {};  // a non-physical state leaves it: no flux
     lmax = checked_speed(prm, riemann<DIM, R, true>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg), e1, pb);
     const R wq = (R)T->wf[q];
 #pragma unroll
