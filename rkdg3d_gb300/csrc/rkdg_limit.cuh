@@ -34,7 +34,9 @@ __device__ __forceinline__ float2 shfl_xor_mean(float2 v, int o) {
 
 // StateIsPhysical (physics.cpp:6-50) without its quotients: the covolume
 // pressure has the sign of (gamma - 1) (rho E - |m|^2 / 2) (1 - rho b).  Float
-// states that cancel are judged in FP64.
+// states that cancel, or so small that the products leave the normal numbers
+// (FP32 flushes below 1.2e-38), are judged in FP64; FP64 states as small with the
+// quotients.
 template <int DIM, typename R>
 __device__ __forceinline__ bool vertex_is_physical(const R* s, R gamma, R b) {
   if (!(s[0] >= R(0)) || !(s[1 + DIM] > R(0))) return false;
@@ -44,12 +46,14 @@ __device__ __forceinline__ bool vertex_is_physical(const R* s, R gamma, R b) {
   const R re = s[0] * s[1 + DIM];
   R x = re - R(0.5) * m2;
   if constexpr (std::is_same<R, float>::value) {
-    if (fabsf(x) < 1e-3f * re) {
+    if (!(fabsf(x) > fmaxf(1e-3f * re, 1e-30f))) {
       double m2d = 0.0;
 #pragma unroll
       for (int d = 0; d < DIM; d++) m2d += (double)s[1 + d] * (double)s[1 + d];
-      x = (float)((double)s[0] * (double)s[1 + DIM] - 0.5 * m2d);
+      x = (double)s[0] * (double)s[1 + DIM] - 0.5 * m2d > 0.0 ? 1.0f : -1.0f;
     }
+  } else {
+    if (!(re > 1e-290)) return state_is_physical<DIM>(s, gamma, b);
   }
   return (gamma - R(1)) * x * (R(1) - s[0] * b) > R(0);
 }
