@@ -67,7 +67,8 @@ __global__ void k_riemann_batch(int n, const double* u1, const double* u2, const
   }
 #pragma unroll
   for (int d = 0; d < DIM; ++d) nn[d] = (R)nor[(long long)i * DIM + d];
-  const R sp = riemann<DIM>(s1, s2, nn, F, (R)gamma, (R)cov, rs, avg);
+  // FP32: the form of hexahedra, Q1 and Q2 quads and hanging faces
+  const R sp = riemann<DIM, R, true>(s1, s2, nn, F, (R)gamma, (R)cov, rs, avg);
   speed[i] = (double)sp;
   // -1 flags a non-physical state; HLLC's signed max(SL, SR) may be negative
   // with a valid flux
