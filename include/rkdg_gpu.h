@@ -165,10 +165,10 @@ int rkdg_set_precision(rkdg_ctx* ctx, int precision);
  * cores (tcgen05 TF32 MMAs, operands split into TF32 hi + lo; FP32-bulk Q2
  * only, else the default).
  * RKDG_TUNE_GENERIC_BLOCK /
- * RKDG_TUNE_LIMITER_BLOCK: threads per CTA of the element pass (FP32 Q1
- * quadrilaterals and P1 triangles; the other planar passes have their own
- * shapes) and of the limiter, 0 (default: 128, fewer on small meshes) or a
- * multiple of 32 up to 256. */
+ * RKDG_TUNE_LIMITER_BLOCK: threads per CTA of the planar face pass (and of the
+ * element pass of FP32 Q1 quadrilaterals and P1 triangles, at most 128 there) and
+ * of the limiter, 0 (default: 128, fewer on small meshes) or a multiple of 32 up
+ * to 256. */
 enum { RKDG_TUNE_HEX_KERNEL = 1, RKDG_TUNE_GENERIC_BLOCK = 2, RKDG_TUNE_LIMITER_BLOCK = 3 };
 int rkdg_set_tuning(rkdg_ctx* ctx, int key, int value);
 /* Autotuner (no counterpart in the reference): times each candidate launch

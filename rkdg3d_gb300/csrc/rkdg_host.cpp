@@ -2200,8 +2200,8 @@ long long rkdg_kernel_launches(rkdg_ctx* c) { return c ? c->launches : -1; }
 // limiter when one is active) on the caller's state, times them with CUDA
 // events on the context's stream and keeps the fastest.  Candidates: the
 // hexahedral kernel (warp per element with 8 elements per CTA, five-lane team
-// with 24, face pass + node pass, tiles, ...) or, on triangles and quads,
-// 64 / 128 / 256 elements per CTA.
+// with 24, face pass + node pass, tiles, ...) or, on triangles and quads, 64 /
+// 128 / 256 threads per CTA of the face pass (and the element pass).
 int rkdg_autotune(rkdg_ctx* c, const double* x, int* hex_kernel, int* generic_block,
                   int* limiter_block) {
   NEED_MESH(c);

@@ -37,7 +37,7 @@ template <int G, int P, typename R>
 cudaError_t launch_planar(const RhsParams& prm, const R* u, const EpiParams<R>& ep, cudaStream_t st) {
   if (!prm.flist || !prm.fslot) return cudaErrorInvalidValue;
   const long long npt = (long long)prm.nface * El<G, P>::NQF;
-  const int blk = spread_block(npt, 128);
+  const int blk = prm.block ? generic_block(prm.block) : spread_block(npt, 128);
   const unsigned grid = (unsigned)((npt + blk - 1) / blk);
   if (prm.faces_only) {
     if (prm.act_cum)

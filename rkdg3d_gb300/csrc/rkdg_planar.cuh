@@ -69,7 +69,7 @@ __device__ __forceinline__ int quad_face_side(int lf) { return lf == 1 || lf == 
 
 // MAP: a batch with a map of the active work (prm.act_cum).
 template <int G, int P, typename R, bool SPEED, bool MAP>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kGenericMaxBlock)
     k_face_planar(const __grid_constant__ RhsParams prm, const R* __restrict__ u) {
   using E = El<G, P>;
   constexpr int DIM = 2, ND = E::ND, NEQ = E::NEQ, NFPE = E::NFPE, NQF = E::NQF, N1 = P + 1;
