@@ -408,30 +408,34 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
       }
     }
   }
-  const R* fx = (const R*)prm.fslot;
-  const long long nf = (long long)prm.nface * NQF;
-  // a quad's faces: the slot of each, its side and direction
-  auto quad_faces = [&]() {
-    const int jx = i % N1, jy = i / N1;
-#pragma unroll
-    for (int lf = 0; lf < NFPE; ++lf) {
-      const int ref = prm.fref[lf * ne + e];
-      const int t = (lf & 1) ? jy : jx;
-      int q = lf >= 2 ? N1 - 1 - t : t;
-      if (ref & 1) q = N1 - 1 - q;
-      const R b = PLAIN ? sMB[lf * ND + i] : sMB[quad_face_side(lf) * N1 + ((lf & 1) ? jx : jy)];
-      const R c = (ref & 2) ? b : -b;
-      const R* p = fx + (long long)(ref >> 2) * NQF + q;
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) acc[k] += c * p[k * nf];
-    }
-  };
   __syncthreads();
   if (live) {
+    // faces: the slot of each, its side and direction
+    const R* fx = (const R*)prm.fslot;
+    const long long nf = (long long)prm.nface * NQF;
     if constexpr (G == 3) {
       const int jx = i % N1, jy = i / N1;
+      // (the volume before the faces but in PLAIN's order)
+#pragma unroll
+      for (int m = 0; m < (PLAIN ? 0 : N1); ++m) {
+        const R d0 = sMD[jx * N1 + m], d1 = sMD[jy * N1 + m];
+#pragma unroll
+        for (int k = 0; k < NEQ; ++k)
+          acc[k] += d0 * sG[0][k][sl * NP + m + N1 * jy] + d1 * sG[1][k][sl * NP + jx + N1 * m];
+      }
+#pragma unroll
+      for (int lf = 0; lf < NFPE; ++lf) {
+        const int ref = prm.fref[lf * ne + e];
+        const int t = (lf & 1) ? jy : jx;
+        int q = lf >= 2 ? N1 - 1 - t : t;
+        if (ref & 1) q = N1 - 1 - q;
+        const R b = PLAIN ? sMB[lf * ND + i] : sMB[quad_face_side(lf) * N1 + ((lf & 1) ? jx : jy)];
+        const R c = (ref & 2) ? b : -b;
+        const R* p = fx + (long long)(ref >> 2) * NQF + q;
+#pragma unroll
+        for (int k = 0; k < NEQ; ++k) acc[k] += c * p[k * nf];
+      }
       if constexpr (PLAIN) {
-        quad_faces();
         const R* g = &sG[0][0][sl * NP];
 #pragma unroll
         for (int o = 0; o < NTERM; ++o) {
@@ -440,15 +444,6 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
 #pragma unroll
           for (int k = 0; k < NEQ; ++k) acc[k] += d * g[k * EPB * NP + at];
         }
-      } else {
-#pragma unroll
-        for (int m = 0; m < N1; ++m) {
-          const R d0 = sMD[jx * N1 + m], d1 = sMD[jy * N1 + m];
-#pragma unroll
-          for (int k = 0; k < NEQ; ++k)
-            acc[k] += d0 * sG[0][k][sl * NP + m + N1 * jy] + d1 * sG[1][k][sl * NP + jx + N1 * m];
-        }
-        quad_faces();
       }
     } else {
 #pragma unroll
