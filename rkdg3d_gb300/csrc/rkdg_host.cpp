@@ -54,8 +54,8 @@ struct rkdg_ctx {
   int nface = 0, nbface = 0;  // nbface: faces without a second element
   int4* d_flist = nullptr;
   int* d_fref = nullptr;
-  double* d_fcoef = nullptr;  // fluxes / moments of the face-pass kernels
-  size_t fcoef_n = 0;
+  unsigned char* d_fcoef = nullptr;  // fluxes / moments of the face-pass kernels
+  size_t fcoef_n = 0;                // bytes
   rkdg::PlanarOpsPair* d_pops = nullptr;
   HexTeamSched* d_hsched = nullptr;  // per-CTA schedules of the shared-face hexahedral kernel
   int hsched_rounds = 0;
@@ -417,19 +417,6 @@ int rhs_kernels(const rkdg_ctx* c, const RhsParams& P) {
   return 2;
 }
 
-// Fluxes (planar) or moments (hexahedra) of the face-pass kernels, in the
-// widest precision.
-int ensure_fcoef(rkdg_ctx* c) {
-  const int per = c->geom == RKDG_GEOM_CUBE ? (c->p + 1) * (c->p + 1) : c->tab.nqf;
-  const size_t n = (size_t)c->nface * c->neq * per;
-  if (c->d_fcoef && c->fcoef_n == n) return RKDG_OK;
-  dfree(c->d_fcoef);
-  c->fcoef_n = 0;
-  CUDA_TRY(c, dalloc(c->d_fcoef, n));
-  c->fcoef_n = n;
-  return RKDG_OK;
-}
-
 void set_batch(rkdg_ctx* c, RhsParams& P, int slot) {
   P.prob = c->d_prob;
   P.pgamma = c->d_pgamma;
@@ -474,6 +461,21 @@ LimParams lim_params(rkdg_ctx* c) {
   return L;
 }
 
+// Fluxes (planar) or moments (hexahedra) of the face-pass kernels in the context's
+// precision; none for the hexahedral variants of one kernel.
+int ensure_fcoef(rkdg_ctx* c) {
+  const bool hex = c->geom == RKDG_GEOM_CUBE;
+  const size_t per = hex ? (c->p + 1) * (c->p + 1) : c->tab.nqf;
+  size_t n = (size_t)c->nface * c->neq * per * (c->precision == RKDG_FP64 ? sizeof(double) : sizeof(float));
+  if (hex && c->hex_variant != 0 && c->hex_variant != 3) n = 0;
+  if (c->fcoef_n == n) return RKDG_OK;
+  dfree(c->d_fcoef);
+  c->fcoef_n = 0;
+  if (n) CUDA_TRY(c, dalloc(c->d_fcoef, n));
+  c->fcoef_n = n;
+  return RKDG_OK;
+}
+
 int ensure_scratch(rkdg_ctx* c) {
   const size_t n = (size_t)c->ndofs * c->neq;
   const int nk = std::max(c->s - 1, 0);
@@ -501,7 +503,7 @@ int ensure_scratch(rkdg_ctx* c) {
     if (!c->d_xh) CUDA_TRY(c, dalloc(c->d_xh, n));
     if (!c->d_xl) CUDA_TRY(c, dalloc(c->d_xl, n));
   }
-  return RKDG_OK;
+  return ensure_fcoef(c);
 }
 
 // TF32 part of an FP32 value (10 explicit mantissa bits, rounded to nearest).
@@ -1082,7 +1084,9 @@ int rkdg_set_tuning(rkdg_ctx* c, int key, int value) {
   if (!c) return RKDG_ERR_INVALID;
   if (key == RKDG_TUNE_HEX_KERNEL && value >= 0 && value <= 6) {
     c->hex_variant = value;
-    return RKDG_OK;
+    if (!c->has_mesh) return RKDG_OK;
+    cudaSetDevice(c->device);
+    return ensure_fcoef(c);
   }
   const bool block_ok = value == 0 || (value >= 32 && value <= 256 && value % 32 == 0);
   if (key == RKDG_TUNE_GENERIC_BLOCK && block_ok) {
@@ -1557,8 +1561,6 @@ int rkdg_upload_mesh(rkdg_ctx* c, const rkdg_mesh_desc* m) {
       CUDA_TRY(c, cudaMemcpy(c->d_pops, &ops, sizeof ops, cudaMemcpyHostToDevice));
     }
   }
-  st = ensure_fcoef(c);
-  if (st) return st;
   if ((c->quirks & RKDG_LIMITER_LINEARIZE) && c->lim == RKDG_LIM_MULTI &&
       c->geom != RKDG_GEOM_TRIANGLE && !c->tab.lin_ok)
     return fail(c, RKDG_ERR_UNSUPPORTED,
@@ -2259,10 +2261,11 @@ int rkdg_autotune(rkdg_ctx* c, const double* x, int* hex_kernel, int* generic_bl
       if (v == 6 && !(c->d_htile && c->d_tcb && c->precision != RKDG_FP64)) continue;
       c->hex_variant = v;
       float ms = 0.0f;
-      if ((st = time_rhs(&ms))) return st;
+      if ((st = ensure_fcoef(c)) || (st = time_rhs(&ms))) return st;
       if (best == 0 || ms < tbest) best = v, tbest = ms;
     }
     c->hex_variant = best;
+    if ((st = ensure_fcoef(c))) return st;
   } else {
     int best = 0;
     float tbest = 0.0f;
