@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(VjpSize<G, P>::NT)
   for (int k = 0; k < NEQ; ++k) acc[k] = 0.0;
   for (int lf = 0; lf < NFPE; ++lf) {
     const int ref = prm.fref[G == 5 ? (long long)e * 8 + lf : (long long)lf * ne + e], code = prm.fcode[lf * ne + e];
-    const int f = G == 5 ? ref >> 1 : ref >> 2, side = G == 5 ? ref & 1 : (ref >> 1) & 1;
+    const int f = G == 5 ? ref >> 1 : ref_face(ref), side = G == 5 ? ref & 1 : (ref >> 1) & 1;
     const double* g = gb + (long long)side * NEQ * npt + (long long)f * NQF;
     const int* pm = T->perm[code >> 4];
     if constexpr (G == 3) {  // one point of the face sees this node

@@ -208,6 +208,20 @@ struct HexTile {
   unsigned char hlf[3][RKDG_TILE_HMAX];     // halo: its local face
 };
 
+// A planar element's reference to one of its faces (RhsParams::fref): the face, whether
+// the element is its Elem2 and whether it runs through the points backwards.
+// Unsigned: 2^30 faces, as many as local face x element indices in an int hold.
+constexpr int planar_ref(int face, int elem2, int back) {
+  return (int)((unsigned)face * 4u + (unsigned)elem2 * 2u + (unsigned)back);
+}
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int ref_face(int ref) {
+  return (int)((unsigned)ref >> 2);
+}
+static_assert(ref_face(planar_ref((1 << 30) - 1, 1, 1)) == (1 << 30) - 1, "the largest face");
+
 // Per-element face table entry codes (fcode): bits 0-2 local face of the
 // other element, bit 3 = 1 if this element is the face's Elem2, bits 4..
 // permutation id.  fnbr: neighbour element id, -1 = boundary face with no

@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>:
 #pragma unroll
     for (int lf = 0; lf < NFPE; ++lf) {
       const int ref = prm.fref[lf * ne + e];
-      const R* fx = (const R*)prm.fslot + (long long)(ref >> 2) * NQF;
+      const R* fx = (const R*)prm.fslot + (long long)ref_face(ref) * NQF;
       const R sg = (ref & 2) ? R(1) : R(-1);
       R fl[NEQ][NQF];
 #pragma unroll

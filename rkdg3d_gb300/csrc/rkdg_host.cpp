@@ -585,7 +585,7 @@ bool face_tables(const rkdg_ctx* c, std::vector<int4>& flist, std::vector<int>& 
         if (hex)
           fref[(size_t)e * 8 + lf] = f * 2;
         else
-          fref[i] = f * 4;
+          fref[i] = rkdg::planar_ref(f, 0, 0);
         if (e2 >= 0) {
           const int lf2 = fc & 7, pid = fc >> 4;
           const size_t i2 = (size_t)lf2 * ne + e2;
@@ -605,7 +605,7 @@ bool face_tables(const rkdg_ctx* c, std::vector<int4>& flist, std::vector<int>& 
             fref[(size_t)e2 * 8 + lf2] = f * 2 + 1;
             fref[(size_t)e2 * 8 + 6] |= inverse[op] << (3 * lf2);
           } else {
-            fref[i2] = f * 4 + 2 + op;
+            fref[i2] = rkdg::planar_ref(f, 1, op);
           }
           r.y = e2;
           r.z = lf + 8 * lf2 + 64 * op;

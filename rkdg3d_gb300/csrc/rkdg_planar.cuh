@@ -87,10 +87,11 @@ __global__ void __launch_bounds__(kGenericMaxBlock)
   R lmax = R(0);
   // MAP: CTAs run over the points of the active problems' faces
   const int na = MAP ? *prm.act_n : 0, nfa = MAP ? prm.act_fcum[na] : prm.nface;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x, next;; t = next) {
+  // (face points: unsigned, up to four per face)
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x, next;; t = next) {
   next = t + gridDim.x * blockDim.x;
-  int f = t / NQF;
-  const int q = t - f * NQF;
+  int f = (int)(t / NQF);
+  const int q = (int)(t - (unsigned)f * NQF);
   int pb = -1;
   bool live = f < nfa;
   if (MAP && live) f = active_face(prm, na, f);
@@ -431,7 +432,7 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
         if (ref & 1) q = N1 - 1 - q;
         const R b = PLAIN ? sMB[lf * ND + i] : sMB[quad_face_side(lf) * N1 + ((lf & 1) ? jx : jy)];
         const R c = (ref & 2) ? b : -b;
-        const R* p = fx + (long long)(ref >> 2) * NQF + q;
+        const R* p = fx + (long long)ref_face(ref) * NQF + q;
 #pragma unroll
         for (int k = 0; k < NEQ; ++k) acc[k] += c * p[k * nf];
       }
@@ -449,7 +450,7 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
 #pragma unroll
       for (int lf = 0; lf < NFPE; ++lf) {
         const int ref = prm.fref[lf * ne + e];
-        const R* p = fx + (long long)(ref >> 2) * NQF;
+        const R* p = fx + (long long)ref_face(ref) * NQF;
 #pragma unroll
         for (int q = 0; q < NQF; ++q) {
           const R b = sMB[(lf * NQF + q) * ND + i];
