@@ -1981,23 +1981,27 @@ struct Adj {
 
 int adj_bufs(rkdg_ctx* c, Adj& A) {
   const size_t n = (size_t)c->ndofs * c->neq;
-  const size_t nvec = 5 + 16;
+  // five vectors, two per stage and two more per stage after the first
+  const int ns = c->s;
+  const size_t nvec = 5 + 2 * ns + 2 * (ns - 1);
   // + the limiter's min/max derivatives and the face points' trace cotangents
   const size_t need = nvec * n + (size_t)4 * c->ne + (size_t)2 * c->neq * c->nface * c->tab.nqf;
   if (c->adj_n < need) {
+    c->adj_n = 0;
     CUDA_TRY(c, dalloc(c->d_adj, need));
     c->adj_n = need;
   }
   double* p = c->d_adj;
+  A = Adj{};
   A.r = p; p += n;
   A.ub = p; p += n;
   A.zb = p; p += n;
   A.acc = p; p += n;
   A.w = p; p += n;
-  for (int i = 0; i < 4; ++i) { A.kb[i] = p; p += n; }
-  for (int i = 0; i < 4; ++i) { A.z[i] = p; p += n; }
-  for (int i = 0; i < 4; ++i) { A.y[i] = p; p += n; }
-  for (int i = 0; i < 4; ++i) { A.k[i] = p; p += n; }
+  for (int i = 0; i < ns; ++i) { A.kb[i] = p; p += n; }
+  for (int i = 0; i < ns; ++i) { A.k[i] = p; p += n; }
+  for (int i = 1; i < ns; ++i) { A.z[i] = p; p += n; }
+  for (int i = 1; i < ns; ++i) { A.y[i] = p; p += n; }
   A.cross = p;
   A.g = p + (size_t)4 * c->ne;
   return RKDG_OK;

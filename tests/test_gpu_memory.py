@@ -38,3 +38,26 @@ def test_face_slots_follow_precision_and_variant(cuda, prec, width):
     before = torch.cuda.mem_get_info()[0]
     ctx.set_tuning(TUNE_HEX_KERNEL, 0)
     assert abs(before - torch.cuda.mem_get_info()[0] - slots * (12 - width) // width) <= page
+
+
+@pytest.mark.parametrize("stages", [1, 3])
+def test_adjoint_scratch_follows_the_tableau(cuda, stages):
+    """Order 1 hexahedra and SSP-RK3: the reverse step's vectors, the traces'
+    cotangents (6.75 state vectors) and the limiter's derivatives take no more than
+    22 state vectors."""
+    case = cases.pulse3d(n=40, order=1)
+    ctx = Context(case.mesh, case.order, device=0, precision=FP64)
+    cases.configure_context(case, ctx)
+    if stages == 1:
+        ctx.set_tableau(1, [0.0], [1.0], [0.0])
+    x = torch.tensor(random_state(ctx.node_coords(), seed=97, amp=0.02, vel=0.05), device="cuda")
+    k, out, g = torch.randn_like(x), torch.empty_like(x), torch.randn_like(x)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    ctx.rhs_vjp(x, k, out)
+    used = free - torch.cuda.mem_get_info()[0]
+    vectors = used / (8 * ctx.n)
+    assert vectors < (22 if stages == 3 else 14.2)
+    ctx.step_vjp(x, 1e-4, g)  # runs within them
+    assert free - torch.cuda.mem_get_info()[0] == used
+    assert torch.isfinite(g).all()
