@@ -34,11 +34,20 @@ namespace rkdg {
 constexpr float kTraceErr = 6e-6f;
 constexpr float kNoBound = 1e30f;
 
+// division and square root to 2 ulp
 RKDG_HD float bdiv(float a, float b) {
 #ifdef __CUDA_ARCH__
   return __fdividef(a, b);
 #else
   return a / b;
+#endif
+}
+
+RKDG_HD float bsqrt(float x) {
+#ifdef __CUDA_ARCH__
+  return x > 0.0f ? x * rsqrtf(x) : 0.0f;
+#else
+  return sqrtf(x);
 #endif
 }
 
@@ -61,7 +70,7 @@ RKDG_HD bool speed_side(const float* s, const float* top, int stride, const floa
     mn += n[d] * s[1 + d];
     mt = fmaxf(mt, top[(1 + d) * stride]);
   }
-  const float ir = bdiv(1.0f, r), m = sqrtf(m2), dm = (DIM == 3 ? 1.7321f : 1.4143f) * kTraceErr * mt;
+  const float ir = bdiv(1.0f, r), m = bsqrt(m2), dm = (DIM == 3 ? 1.7321f : 1.4143f) * kTraceErr * mt;
   const float er = kTraceErr * top[0] * ir, ee = bdiv(kTraceErr * top[(1 + DIM) * stride], E);
   const float re = r * E, ie = re - 0.5f * m2, f = 1.0f - r * b;  // ie: rho times the internal energy
   if (!(ie >= 0.02f * re && f >= 0.5f)) return false;
@@ -74,7 +83,7 @@ RKDG_HD bool speed_side(const float* s, const float* top, int stride, const floa
   S.u = mn * ir;
   S.v = m * ir;
   S.du = 1.2f * (dm * ir + S.v * er) + 3e-6f * S.v;
-  S.c = sqrtf(gamma * (gamma - 1.0f) * ie) * g;
+  S.c = bsqrt(gamma * (gamma - 1.0f) * ie) * g;
   S.dc = S.c * (0.6f * e2 + 1e-5f);
   S.p = ie * g;  // pressure / (gamma - 1)
   S.er = er;
@@ -89,10 +98,10 @@ RKDG_HD float speed_bound(const SpeedSide& L, const SpeedSide& R, float gamma, i
   const float D = R.u - L.u;
   float SLlo, SLhi, SRlo, SRhi;
   if (avg == 1) {
-    const float t = sqrtf(bdiv(R.r, L.r)), wL = bdiv(1.0f, 1.0f + t), wR = t * wL;
+    const float t = bsqrt(bdiv(R.r, L.r)), wL = bdiv(1.0f, 1.0f + t), wR = t * wL;
     const float et = 0.6f * (L.er + R.er) + 1e-6f;
     const float uav = wL * L.u + wR * R.u;
-    const float cav = sqrtf(wL * L.c * L.c + wR * R.c * R.c + 0.5f * wL * wR * D * D);
+    const float cav = bsqrt(wL * L.c * L.c + wR * R.c * R.c + 0.5f * wL * wR * D * D);
     const float err = fmaxf(L.du, R.du) + fmaxf(L.dc, R.dc) + 0.36f * (L.du + R.du) +
                       (0.6f * et + 1e-6f) * (fabsf(D) + cav) + 1e-6f * (fabsf(L.u) + fabsf(R.u));
     SLlo = uav - cav - err;
@@ -111,8 +120,8 @@ RKDG_HD float speed_bound(const SpeedSide& L, const SpeedSide& R, float gamma, i
     const float t = bdiv(A + dA, B - dB);
     const float pl = exp2f(iz * log2f(t)) * (1.00001f + 1e-6f * iz), pr = pl * x * (1.00001f + 1.1f * ex);
     const float hg = bdiv(0.5f * (gamma + 1.0f), gamma);
-    const float qL = pl > 1.0f ? sqrtf(1.0f + hg * (pl - 1.0f)) * 1.000001f : 1.0f;
-    const float qR = pr > 1.0f ? sqrtf(1.0f + hg * (pr - 1.0f)) * 1.000001f : 1.0f;
+    const float qL = pl > 1.0f ? bsqrt(1.0f + hg * (pl - 1.0f)) * 1.000001f : 1.0f;
+    const float qR = pr > 1.0f ? bsqrt(1.0f + hg * (pr - 1.0f)) * 1.000001f : 1.0f;
     SLlo = L.u - L.du - qL * (L.c + L.dc);
     SLhi = L.u + L.du - (L.c - L.dc);
     SRlo = R.u - R.du + (R.c - R.dc);
