@@ -393,7 +393,8 @@ __device__ __forceinline__ unsigned hanging_faces(const LimParams& prm, int row)
 // derivative with respect to them goes to cross[0..3][e] = (argmin element or -1
 // for e itself, d/dmin, argmax element or -1, d/dmax), which k_limit_vjp_gather
 // hands to those elements.  A thread per element that carried Dual<ND + 3>
-// through every point took 205 us on 20^3 Q1 hexahedra, spilling; this one about 60
+// through every point took 205 us on 20^3 Q1 hexahedra, spilling; this one about
+// 60.
 template <int G, int P>
 struct LimVjp {
   using E = El<G, P>;

@@ -1,7 +1,6 @@
-// Hexahedra: register-resident team kernels (rkdg_hex_team.cuh) for the
-// right-hand side, the warp-per-element sum-factorised kernel
-// (rkdg_hex.cuh) for the FP64 path, plus the generic limiter and cell-mean
-// kernels.
+// Hexahedra: the face pass and the node pass (rkdg_hex_faces.cuh), the default; the
+// other selectable right-hand sides, team kernels (rkdg_hex_team.cuh) and a warp
+// per element (rkdg_hex.cuh); the limiter and the cell means.
 #include "rkdg_hex.cuh"
 #include "rkdg_hex_faces.cuh"
 #include "rkdg_hex_team.cuh"

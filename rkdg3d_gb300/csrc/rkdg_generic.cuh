@@ -1,14 +1,7 @@
-// Generic (dense reference-operator) element kernels, one thread per element,
-// and what the kernels share: float-pair arithmetic, row loads, the wave-speed
-// reductions and the Runge-Kutta epilogue.  Reference operators live in
-// shared memory, converted to the arithmetic type R.  The right-hand side of
-// one element is the reference's FE_Evolution::Mult restricted to that
-// element (fe_evolution.cpp:102-216): every face of the element computes the
-// numerical flux at the face points with the arguments ordered (Elem1,
-// Elem2, Elem1-outward normal) exactly as FaceIntegrator::AssembleFaceVector
-// (face_integrator.cpp:11-276), so the two elements of a face obtain
-// bit-identical fluxes and the scheme stays conservative to round-off
-// without atomics.
+// What the kernels share: float-pair arithmetic, row loads, conversions, the
+// wave-speed reductions, the map of a batch's active work and the Runge-Kutta
+// epilogue; and the kernels of one thread per element: the FP32 element pass, the
+// Shu indicator's limiter and the cell means.
 #pragma once
 
 #include "rkdg_common.h"
@@ -17,15 +10,15 @@
 
 namespace rkdg {
 
-// Largest CTA the generic (thread-per-element) kernels are launched with.
+// Largest CTA of the kernels of one thread per element or face point.
 constexpr int kGenericMaxBlock = 256;
-// The FP32 right-hand-side and limiter kernels of small elements (Q1 quads,
-// P1 triangles: NEQ * ND <= 16 values) are latency bound at the occupancy
-// their registers allow: they run at most 128 threads per CTA and are compiled
-// for six (right-hand side, 80 registers) or five (limiter, 96 registers) CTAs
-// per SM with a few spilled values, which measured 7-8% faster on the batched
-// and triangle workloads than the 12-16 warps of their uncapped registers.
-// Larger elements would spill kilobytes at that cap and keep the default.
+// The element pass and the Shu limiter of FP32 elements of at most 16 values (Q1
+// quads, P1 triangles) are latency bound at the occupancy their registers allow:
+// they run at most 128 threads per CTA and are compiled for six (element pass, 80
+// registers) or five (limiter, 96 registers) CTAs per SM with a few spilled values,
+// which measured 7-8% faster on the batched and triangle workloads than the 12-16
+// warps of their uncapped registers.  Larger elements would spill kilobytes at that
+// cap and keep the default.
 template <typename R, int NVAL>
 __host__ __device__ constexpr bool generic_small() {
   return std::is_same<R, float>::value && NVAL <= 16;
@@ -394,8 +387,9 @@ __device__ __forceinline__ void epilogue(const EpiParams<R>& ep, long long base_
 // fluxes come from the face pass (rkdg_planar.cuh), the element's own rows are
 // loaded once.  524,288 P1 triangles: 59 us against 76 for a thread per node;
 // 253,064 Q1 quads of a batch: 45 + 48 us for the two passes against 96 for one
-// kernel that evaluated every face from both sides.  Q1 quads keep the arithmetic and the order of the sums of a kernel
-// that evaluated its faces itself, see riemann().
+// kernel that evaluated every face from both sides.  Q1 quads keep the arithmetic
+// and the order of the sums of a kernel that evaluated its faces itself, see
+// riemann().
 template <int G, int P, typename R>
 __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>::ND>(),
                                   generic_min_blocks<R, El<G, P>::NEQ * El<G, P>::ND, false>())
@@ -432,7 +426,6 @@ __global__ void __launch_bounds__(generic_max_block<R, El<G, P>::NEQ * El<G, P>:
     if (live) e = active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, prm.ne, prm.prob, pb);
   }
   if (live && prm.prob) {
-    if (!prm.act_cum) pb = prm.prob[e];
     live = prm.pactive[pb] != 0;
     if constexpr (std::is_same<R, float>::value) {
       // FP32 copies: no FP64 conversions per element

@@ -445,24 +445,24 @@ __global__ void __launch_bounds__(HexFaces<P>::NTN)
     const int refs[6] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y}, ops = rb.z;
     auto faces = [&](auto turned) {  // turned: some face is indexed another way by its Elem1
 #pragma unroll
-    for (int o = 0; o < 6; ++o) {
-      constexpr int AX[6] = {2, 1, 0, 1, 0, 2}, SD[6] = {0, 0, 1, 1, 0, 1};
-      // float: the order in which the team (Q1) and tile (Q2) kernels add them
-      constexpr int ORD[6] = {4, 2, 1, 3, 0, 5};
-      const int lf = F32 && P == 2 ? ORD[o] : o;
-      const int ref = refs[lf];
-      const int t0 = AX[lf] == 0 ? jy : jx, t1 = AX[lf] == 2 ? jy : jz;
-      const int jn = AX[lf] == 0 ? jx : (AX[lf] == 1 ? jy : jz);
-      const R* mb = (F32 ? H.lend : H.mb) + SD[lf] * N1;
-      R b = mb[0];  // by selection: an indexed constant is read lane by lane
+      for (int o = 0; o < 6; ++o) {
+        constexpr int AX[6] = {2, 1, 0, 1, 0, 2}, SD[6] = {0, 0, 1, 1, 0, 1};
+        // float: the order in which the team (Q1) and tile (Q2) kernels add them
+        constexpr int ORD[6] = {4, 2, 1, 3, 0, 5};
+        const int lf = F32 && P == 2 ? ORD[o] : o;
+        const int ref = refs[lf];
+        const int t0 = AX[lf] == 0 ? jy : jx, t1 = AX[lf] == 2 ? jy : jz;
+        const int jn = AX[lf] == 0 ? jx : (AX[lf] == 1 ? jy : jz);
+        const R* mb = (F32 ? H.lend : H.mb) + SD[lf] * N1;
+        R b = mb[0];  // by selection: an indexed constant is read lane by lane
 #pragma unroll
-      for (int j = 1; j < N1; ++j) b = jn == j ? mb[j] : b;
-      const R c = (ref & 1) ? b : -b;
-      const int at = turned.value ? square_op((ops >> (3 * lf)) & 7, t0, t1, N1) : t0 + N1 * t1;
-      const R* p = (const R*)prm.fslot + (long long)(ref >> 1) * (NEQ * NF2) + at;
+        for (int j = 1; j < N1; ++j) b = jn == j ? mb[j] : b;
+        const R c = (ref & 1) ? b : -b;
+        const int at = turned.value ? square_op((ops >> (3 * lf)) & 7, t0, t1, N1) : t0 + N1 * t1;
+        const R* p = (const R*)prm.fslot + (long long)(ref >> 1) * (NEQ * NF2) + at;
 #pragma unroll
-      for (int k = 0; k < NEQ; ++k) acc[k] += c * __ldg(p + k * NF2);
-    }
+        for (int k = 0; k < NEQ; ++k) acc[k] += c * __ldg(p + k * NF2);
+      }
     };
     if (ops)
       faces(std::true_type{});

@@ -325,7 +325,7 @@ __device__ __forceinline__ R rusanov_flux(const R* s1, const R* s2, const Frame<
   return maxE;
 }
 
-// The FP32 forms of hexahedra and Q1 quads (riemann() with PLAIN).
+// The FP32 forms of hexahedra, Q1 and Q2 quads (riemann() with PLAIN).
 //
 // FP32 pointwise state quantities with one reciprocal of the density and one
 // of the covolume factor: r = 1/rho, q = 1/(1 - rho b), the pressure (FP64
@@ -765,7 +765,7 @@ __device__ __forceinline__ R hll_family(R* s1, R* s2, const Frame<DIM, R>& fr, R
 // reference does through const_cast); n is the unit normal from side 1 to
 // side 2.  Returns the solver's wave speed, or -1 for a non-physical state.
 // float and double take the forms above; dual numbers the plain restatement
-// below, and so does float where PLAIN is set: hexahedra and Q1 quads.  Their
+// below, and so does float where PLAIN is set: hexahedra, Q1 and Q2 quads.  Their
 // limited runs pass through elements that sit within FP32 rounding of the
 // limiter's switches (the +-1e-3 thresholds, the Michalak function's step at 1),
 // where any other rounding of a flux moves single elements by up to 5%; so the

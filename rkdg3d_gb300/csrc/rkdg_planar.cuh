@@ -19,6 +19,11 @@
 // with a thread per element (k_elem_planar): there the instructions around a
 // node's few values outnumber its arithmetic three to one.
 //
+// Quads add the volume before the faces, triangles and FP32 Q2 quads the faces
+// first.  Neither order is the more accurate; a Sod run over its whole time (877
+// steps, chaotic at one ulp) keeps the oracle's number of steps with this one, and
+// about one rounding variant in seven gives 878.
+//
 // On quadrilaterals the mass, trace and derivative tables of the collocated
 // Gauss-Legendre basis are sparse (the mass matrix is diagonal, a face point
 // sees one line of nodes): N1 terms instead of ND.
@@ -89,140 +94,140 @@ __global__ void __launch_bounds__(kGenericMaxBlock)
   const int na = MAP ? *prm.act_n : 0, nfa = MAP ? prm.act_fcum[na] : prm.nface;
   // (face points: unsigned, up to four per face)
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x, next;; t = next) {
-  next = t + gridDim.x * blockDim.x;
-  int f = (int)(t / NQF);
-  const int q = (int)(t - (unsigned)f * NQF);
-  int pb = -1;
-  bool live = f < nfa;
-  if (MAP && live) f = active_face(prm, na, f);
-  lmax = R(0);
-  int4 face = make_int4(0, -1, 0, 0);
-  int e1 = 0;
-  R gamma = (R)prm.gamma, cov = (R)prm.covolume;
-  if (live) {
-    face = prm.flist[f];
-    e1 = face.x;
-    if (prm.prob) {
-      pb = face.w;  // set with the batch
-      live = prm.pactive[pb] != 0;
-      if constexpr (std::is_same<R, float>::value) {
-        gamma = prm.pgamma32 ? prm.pgamma32[pb] : (R)prm.pgamma[pb];
-        cov = prm.pcov32 ? prm.pcov32[pb] : (R)prm.pcov[pb];
-      } else {
-        gamma = (R)prm.pgamma[pb];
-        cov = (R)prm.pcov[pb];
+    next = t + gridDim.x * blockDim.x;
+    int f = (int)(t / NQF);
+    const int q = (int)(t - (unsigned)f * NQF);
+    int pb = -1;
+    bool live = f < nfa;
+    if (MAP && live) f = active_face(prm, na, f);
+    lmax = R(0);
+    int4 face = make_int4(0, -1, 0, 0);
+    int e1 = 0;
+    R gamma = (R)prm.gamma, cov = (R)prm.covolume;
+    if (live) {
+      face = prm.flist[f];
+      e1 = face.x;
+      if (prm.prob) {
+        pb = face.w;  // set with the batch
+        live = prm.pactive[pb] != 0;
+        if constexpr (std::is_same<R, float>::value) {
+          gamma = prm.pgamma32 ? prm.pgamma32[pb] : (R)prm.pgamma[pb];
+          cov = prm.pcov32 ? prm.pcov32[pb] : (R)prm.pcov[pb];
+        } else {
+          gamma = (R)prm.pgamma[pb];
+          cov = (R)prm.pcov[pb];
+        }
       }
     }
-  }
-  if (live) {
-    bool skip = false;
-    const int lf1 = face.z & 7;
-    const R* fg = (const R*)prm.fgeo;
-    R n[DIM];
+    if (live) {
+      bool skip = false;
+      const int lf1 = face.z & 7;
+      const R* fg = (const R*)prm.fgeo;
+      R n[DIM];
 #pragma unroll
-    for (int c = 0; c < DIM; ++c) n[c] = fg[(long long)(lf1 * (DIM + 1) + c) * ne + e1];
-    const R jac = fg[(long long)(lf1 * (DIM + 1) + DIM) * ne + e1];
-    // a side's trace at its own face point
-    auto trace = [&](int e, int lf, int qq, R* s) {
-      const R* ue = u + (long long)e * ND;
-      if constexpr (G == 3) {
-        R le[N1];
-        const int sd = quad_face_side(lf);
+      for (int c = 0; c < DIM; ++c) n[c] = fg[(long long)(lf1 * (DIM + 1) + c) * ne + e1];
+      const R jac = fg[(long long)(lf1 * (DIM + 1) + DIM) * ne + e1];
+      // a side's trace at its own face point
+      auto trace = [&](int e, int lf, int qq, R* s) {
+        const R* ue = u + (long long)e * ND;
+        if constexpr (G == 3) {
+          R le[N1];
+          const int sd = quad_face_side(lf);
 #pragma unroll
-        for (int j = 0; j < N1; ++j) le[j] = sd ? H.lend[N1 + j] : H.lend[j];
-        const int i0 = quad_face_node<N1>(lf, qq, 0), st = (lf & 1) ? 1 : N1;
-        if constexpr (PLAIN) {
+          for (int j = 0; j < N1; ++j) le[j] = sd ? H.lend[N1 + j] : H.lend[j];
+          const int i0 = quad_face_node<N1>(lf, qq, 0), st = (lf & 1) ? 1 : N1;
+          if constexpr (PLAIN) {
 #pragma unroll
-          for (int j = 0; j < N1; ++j) le[j] = sB[(lf * NQF + qq) * ND + i0 + j * st];
-        }
-#pragma unroll
-        for (int k = 0; k < NEQ; ++k) {
-          R v = R(0);
-#pragma unroll
-          for (int j = 0; j < N1; ++j) v += le[j] * ue[k * NDa + i0 + j * st];
-          s[k] = v;
-        }
-      } else {
-        const R* B = sB + (lf * NQF + qq) * ND;
-#pragma unroll
-        for (int k = 0; k < NEQ; ++k) {
-          R v = R(0);
-#pragma unroll
-          for (int j = 0; j < ND; ++j) v += B[j] * ue[k * NDa + j];
-          s[k] = v;
-        }
-      }
-    };
-    R s1[NEQ], s2[NEQ], F[NEQ];
-    if constexpr (SPEED) {
-      // bounded in FP32, evaluated in FP64 only where the point could hold the
-      // maximum
-      if (face.y >= 0) {
-        float a1[NEQ], a2[NEQ], nf[DIM], top[2][NEQ];
-        auto est = [&](int e, int lf, int qq, float* s, float* tp) {
-          const R* ue = u + (long long)e * ND;
-          constexpr int NT = G == 3 ? N1 : ND;  // terms of the trace
-          const int sd = quad_face_side(lf), i0 = G == 3 ? quad_face_node<N1>(lf, qq, 0) : 0;
-          const int st = G == 3 && !(lf & 1) ? N1 : 1;
-          const float* B = prm.pops->f.b + (lf * NQF + qq) * ND;
-#pragma unroll
-          for (int k = 0; k < NEQ; ++k) s[k] = tp[k] = 0.0f;
-#pragma unroll
-          for (int j = 0; j < NT; ++j) {
-            const float w = G == 3 ? (sd ? prm.pops->f.lend[N1 + j] : prm.pops->f.lend[j]) : B[j];
-#pragma unroll
-            for (int k = 0; k < NEQ; ++k) {
-              const float x = cut_f32((double)ue[k * NDa + i0 + j * st]);
-              s[k] += w * x;
-              tp[k] = fmaxf(tp[k], fabsf(x));
-            }
+            for (int j = 0; j < N1; ++j) le[j] = sB[(lf * NQF + qq) * ND + i0 + j * st];
           }
-        };
-        est(e1, lf1, q, a1, top[0]);
-        est(face.y, (face.z >> 3) & 7, (face.z >> 6) ? NQF - 1 - q : q, a2, top[1]);
 #pragma unroll
-        for (int c = 0; c < DIM; ++c) nf[c] = (float)n[c];
-        const float g = (float)gamma, b = (float)cov;
-        SpeedSide A, B;
-        if (speed_side<DIM>(a1, top[0], 1, nf, g, b, A) && speed_side<DIM>(a2, top[1], 1, nf, g, b, B) &&
-            speed_below(speed_bound(A, B, g, prm.rs, prm.avg, prm.quirks & 1), prm.prob ? prm.pmcs + pb : prm.mcs))
-          skip = true;
+          for (int k = 0; k < NEQ; ++k) {
+            R v = R(0);
+#pragma unroll
+            for (int j = 0; j < N1; ++j) v += le[j] * ue[k * NDa + i0 + j * st];
+            s[k] = v;
+          }
+        } else {
+          const R* B = sB + (lf * NQF + qq) * ND;
+#pragma unroll
+          for (int k = 0; k < NEQ; ++k) {
+            R v = R(0);
+#pragma unroll
+            for (int j = 0; j < ND; ++j) v += B[j] * ue[k * NDa + j];
+            s[k] = v;
+          }
+        }
+      };
+      R s1[NEQ], s2[NEQ], F[NEQ];
+      if constexpr (SPEED) {
+        // bounded in FP32, evaluated in FP64 only where the point could hold the
+        // maximum
+        if (face.y >= 0) {
+          float a1[NEQ], a2[NEQ], nf[DIM], top[2][NEQ];
+          auto est = [&](int e, int lf, int qq, float* s, float* tp) {
+            const R* ue = u + (long long)e * ND;
+            constexpr int NT = G == 3 ? N1 : ND;  // terms of the trace
+            const int sd = quad_face_side(lf), i0 = G == 3 ? quad_face_node<N1>(lf, qq, 0) : 0;
+            const int st = G == 3 && !(lf & 1) ? N1 : 1;
+            const float* B = prm.pops->f.b + (lf * NQF + qq) * ND;
+#pragma unroll
+            for (int k = 0; k < NEQ; ++k) s[k] = tp[k] = 0.0f;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+              const float w = G == 3 ? (sd ? prm.pops->f.lend[N1 + j] : prm.pops->f.lend[j]) : B[j];
+#pragma unroll
+              for (int k = 0; k < NEQ; ++k) {
+                const float x = cut_f32((double)ue[k * NDa + i0 + j * st]);
+                s[k] += w * x;
+                tp[k] = fmaxf(tp[k], fabsf(x));
+              }
+            }
+          };
+          est(e1, lf1, q, a1, top[0]);
+          est(face.y, (face.z >> 3) & 7, (face.z >> 6) ? NQF - 1 - q : q, a2, top[1]);
+#pragma unroll
+          for (int c = 0; c < DIM; ++c) nf[c] = (float)n[c];
+          const float g = (float)gamma, b = (float)cov;
+          SpeedSide A, B;
+          if (speed_side<DIM>(a1, top[0], 1, nf, g, b, A) && speed_side<DIM>(a2, top[1], 1, nf, g, b, B) &&
+              speed_below(speed_bound(A, B, g, prm.rs, prm.avg, prm.quirks & 1), prm.prob ? prm.pmcs + pb : prm.mcs))
+            skip = true;
+        }
       }
-    }
-    if (!skip) trace(e1, lf1, q, s1);
-    bool none = false;
-    if (skip) {
-      none = true;
-    } else if (face.y >= 0) {
-      trace(face.y, (face.z >> 3) & 7, (face.z >> 6) ? NQF - 1 - q : q, s2);
-    } else {
-      const int nb = prm.fnbr[lf1 * ne + e1];
-      none = nb == -1;  // no integrator
+      if (!skip) trace(e1, lf1, q, s1);
+      bool none = false;
+      if (skip) {
+        none = true;
+      } else if (face.y >= 0) {
+        trace(face.y, (face.z >> 3) & 7, (face.z >> 6) ? NQF - 1 - q : q, s2);
+      } else {
+        const int nb = prm.fnbr[lf1 * ne + e1];
+        none = nb == -1;  // no integrator
+        if (!none) {
+          const BCSlot& bc = prm.bc[-2 - nb];
+          right_state<DIM>(bc.type, bc.state, s1, s2, n, gamma, cov, (R)prm.rgas);
+        }
+      }
+      // no integrator, or a non-physical state: no flux
+#pragma unroll
+      for (int k = 0; k < NEQ; ++k) F[k] = R(0);
       if (!none) {
-        const BCSlot& bc = prm.bc[-2 - nb];
-        right_state<DIM>(bc.type, bc.state, s1, s2, n, gamma, cov, (R)prm.rgas);
+        R sp;
+        if constexpr (PLAIN)
+          sp = riemann<DIM, R, true>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg);
+        else
+          sp = riemann<DIM>(s1, s2, make_frame<DIM, R>(n), F, gamma, cov, prm.rs, prm.avg);
+        lmax = checked_speed(prm, sp, e1, pb);
+      }
+      if constexpr (!SPEED) {
+        R* out = (R*)prm.fslot + (long long)f * NQF + q;
+        const long long nf = (long long)prm.nface * NQF;
+#pragma unroll
+        for (int k = 0; k < NEQ; ++k) out[k * nf] = PLAIN ? (F[k] * H.wf[q]) * jac : F[k] * jac;
       }
     }
-    // no integrator, or a non-physical state: no flux
-#pragma unroll
-    for (int k = 0; k < NEQ; ++k) F[k] = R(0);
-    if (!none) {
-      R sp;
-      if constexpr (PLAIN)
-        sp = riemann<DIM, R, true>(s1, s2, n, F, gamma, cov, prm.rs, prm.avg);
-      else
-        sp = riemann<DIM>(s1, s2, make_frame<DIM, R>(n), F, gamma, cov, prm.rs, prm.avg);
-      lmax = checked_speed(prm, sp, e1, pb);
-    }
-    if constexpr (!SPEED) {
-      R* out = (R*)prm.fslot + (long long)f * NQF + q;
-      const long long nf = (long long)prm.nface * NQF;
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) out[k * nf] = PLAIN ? (F[k] * H.wf[q]) * jac : F[k] * jac;
-    }
-  }
-  if (prm.prob) segmented_max_commit<R>(lmax, live ? pb : -1, prm.pmcs);
-  if (!MAP || (long long)next - threadIdx.x >= (long long)nfa * NQF) break;
+    if (prm.prob) segmented_max_commit<R>(lmax, live ? pb : -1, prm.pmcs);
+    if (!MAP || (long long)next - threadIdx.x >= (long long)nfa * NQF) break;
   }
   if (!prm.prob) block_max_commit<R>(lmax, prm.mcs);
 }
@@ -352,7 +357,6 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
     if (live) e = active_element(prm.act_cum, prm.act_pid, prm.poff, na, e, prm.ne, prm.prob, pb);
   }
   if (live && prm.prob) {
-    if (!prm.act_cum) pb = prm.prob[e];
     live = prm.pactive[pb] != 0;
     if constexpr (std::is_same<R, float>::value) {
       // FP32 copies: no FP64 conversions per element
