@@ -53,9 +53,10 @@ def workload_config(case, n_elem_side):
 
 # DRAM bytes (read + write) per element and stage of the C2 stage kernels
 # k_face_hex<2,float> + k_node_hex<2,float>: mean of the three stages of one RK
-# step captured with ncu on the 48^3 pulse (533.5 MB / 110,592 elements);
-# traffic scales with the element count.
-TRAFFIC_BYTES_PER_ELEMENT_STAGE = 4824.0
+# step captured with ncu on this pulse at 64^3 (1513.9 MB / 262,144 elements).
+# Smaller meshes move less per element: part of the faces' moments (142 MB here)
+# stays in L2 (4,824 B on 48^3).
+TRAFFIC_BYTES_PER_ELEMENT_STAGE = 5775.0
 
 
 def algorithmic_bytes_per_step(N, ne, precision):
@@ -326,7 +327,7 @@ def run_ours(args, rank, world, local):
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak,
             "traffic": args.traffic_per_launch or TRAFFIC_BYTES_PER_ELEMENT_STAGE * ctx32.ne,
-            "traffic_source": "ncu dram bytes per stage (two launches), 48^3 capture (per element, scaled by elements)"
+            "traffic_source": "ncu dram bytes per stage (two launches), 64^3 capture"
                               if not args.traffic_per_launch else "command line",
             "peak_source": peak_src,
             "kernel": ("k_face_hex<2,float> + k_node_hex<2,float> (face pass and node pass, 6 launches per step)"

@@ -26,11 +26,11 @@
 // loads in flight); it is bound by issue (64% of the slots), the node pass by the
 // latency of its loads at 36 warps per SM.  Per RK step: 48^3 Q2 0.94 ms against
 // 1.04 (tiles) and 1.5 (rows read by the trace threads), 48x45x51 Q1 with HLL
-// 0.46 ms against 0.78 (team), with the limiter 0.61 against 1.12, 31x29x23 Q2
-// limited 0.31 against 0.53, whose means were summed in FP64.
+// 0.46 ms against 0.78 (team), with the limiter 0.62 against 1.12, 31x29x23 Q2
+// limited 0.30 against 0.53.
 //
 // FP64, per RK step: 32^3 Q2 2.91 ms against 4.9 with the shared-face team
-// kernel (the FP64 pipe is active 83-86% of the time); 33x27x21 Q1 limited
+// kernel (the FP64 pipe is active 84-87% of the time); 33x27x21 Q1 limited
 // 0.83 ms against 1.5 with the team face and element passes, which wrote the
 // fluxes once per side and applied a dense mass inverse.
 #pragma once
@@ -235,8 +235,11 @@ __global__ void __launch_bounds__(HexFaces<P>::NT)
 
 // The largest face wave speed of an FP64 state.  Every face point is bounded in
 // FP32 first (rkdg_speed_bound.h); only faces with a point that could hold the
-// maximum, or that has no bound, and boundary faces are evaluated in FP64.  48x45x51 Q1, HLL with TRRS speeds:
-// 0.66 ms against 1.13 for every point in FP64; 48^3 Q2 Rusanov 0.4 against 1.4.
+// maximum, or that has no bound, and boundary faces are evaluated in FP64.  A
+// call on Gaussian pulses, 48x45x51 Q1, HLL with TRRS speeds: 0.35 ms against
+// 1.32 with every point in FP64; 48^3 Q2 acoustic pulse, Rusanov: 0.46 against 1.65
+// (planar: 524,288 P1 triangles 0.17 against 0.57, 317x211 quad Q3 0.09 against
+// 0.15).
 template <int P>
 __global__ void __launch_bounds__(HexFaces<P>::NT)
     k_speed_hex(const __grid_constant__ RhsParams prm, const double* __restrict__ u) {
