@@ -147,14 +147,18 @@ struct PlanarOps {
   R mb[54];
   R lend[8];
   R wf[4];   // face-rule weights
-  // the dense operators of the element pass (at most four nodes) and of Q2 quads:
+  // the dense operators of the element pass (at most four nodes):
   // eb[lf][q][j] traces (triangles: times w_q), ed[r][j][m] = D_r, em = M^-1
-  R eb[108], ed[162], em[81];
+  R eb[48], ed[32], em[16];
   R wm[16];  // cell-mean weights
+  // Q2 quads: each node's six derivative terms in the order of the dense tables
+  // (their places: PlanarOpsPair::at), the inverse mass, the traces [lf][node]
+  R pd[54], pm[9], pb[36];
 };
 struct PlanarOpsPair {
   PlanarOps<float> f;
   PlanarOps<double> d;
+  int at[54];  // 16 * direction + node
 };
 
 // Schedule of one CTA of the shared-face hexahedral team kernel: the CTA's

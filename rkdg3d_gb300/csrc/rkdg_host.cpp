@@ -623,7 +623,7 @@ void planar_tables(const rkdg_ctx* c, rkdg::PlanarOpsPair& ops) {
   std::memset(&ops, 0, sizeof ops);
   for (int j = 0; j < nd; ++j) D.wm[j] = T.wmean[j];
   for (int q = 0; q < nqf; ++q) D.wf[q] = T.wf[q];
-  if (nd <= 4 || (c->geom == RKDG_GEOM_SQUARE && c->p == 2)) {
+  if (nd <= 4) {
     for (int lf = 0; lf < nfpe; ++lf)
       for (int q = 0; q < nqf; ++q)
         for (int j = 0; j < nd; ++j)
@@ -655,6 +655,23 @@ void planar_tables(const rkdg_ctx* c, rkdg::PlanarOpsPair& ops) {
           D.b[(lf * nqf + q) * nd + i] = T.B[lf][q][i];
           for (int j = 0; j < nd; ++j) D.mb[(lf * nqf + q) * nd + i] += T.Minv[i][j] * T.B[lf][q][j] * T.wf[q];
         }
+    }
+  }
+  if (c->geom == RKDG_GEOM_SQUARE && c->p == 2) {
+    for (int n = 0; n < 9; ++n) {
+      const int x = n % 3, y = n / 3;
+      int o = 6 * n;
+      for (int m = 0; m < 9; ++m)  // the row's nodes, and the column's, in order
+        for (int r = 0; r < 2; ++r)
+          if (r == 0 ? m / 3 == y : m % 3 == x) {
+            D.pd[o] = T.D[r][n][m];
+            ops.at[o++] = 16 * r + m;
+          }
+      D.pm[n] = T.Minv[n][n];
+      for (int lf = 0; lf < 4; ++lf) {
+        const int t = (lf & 1) ? y : x;
+        D.pb[lf * 9 + n] = T.B[lf][lf >= 2 ? 2 - t : t][n];
+      }
     }
   }
   const double* src = reinterpret_cast<const double*>(&ops.d);

@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
   // nodes of the row and the column in ascending order, then the inverse mass.  Many
   // limited steps part by 1e-4 to 1e-3 under any other rounding.  Batches and
   // problems alone take the same arithmetic.  9 x 1563 x 4 quads, 20 limited steps:
-  // 4.87 ms against 6.39 with a thread per element; alone, 301x203 quads, 111 us a step
+  // 4.74 ms against 6.24 with a thread per element; alone, 301x203 quads, 108 us a step
   // against 105 with the contravariant node fluxes (limited 207 against 186, with the
   // factor applied nd times).
   constexpr bool PLAIN = G == 3 && P == 2 && std::is_same<R, float>::value;
@@ -330,19 +330,12 @@ __global__ void __launch_bounds__(Planar<G, P>::threads(EPB))
   if (prm.act_cum && (int)(blockIdx.x * EPB) >= prm.act_cum[*prm.act_n]) return;
   if constexpr (PLAIN) {
     for (int t = tid; t < ND * NTERM; t += NT) {
-      const int n = t / NTERM, x = n % N1, y = n / N1, o = t - n * NTERM - y;
-      // the column below, the row with the node's own column term after its row
-      // term, the column above
-      const bool row = o >= 0 && o <= N1 && o != x + 1;
-      const int m = row ? N1 * y + (o <= x ? o : o - 1) : x + N1 * (o < 0 ? o + y : (o == x + 1 ? y : y + o - N1));
-      sMD[t] = H.ed[((row ? 0 : 1) * ND + n) * ND + m];
-      sAt[t] = (row ? 0 : NEQ * EPB * NP) + m;
+      const int at = prm.pops->at[t];
+      sMD[t] = H.pd[t];
+      sAt[t] = (at >> 4) * (NEQ * EPB * NP) + (at & 15);
     }
-    for (int t = tid; t < ND; t += NT) sMD[ND * NTERM + t] = H.em[t * ND + t];
-    for (int t = tid; t < NFPE * ND; t += NT) {
-      const int lf = t / ND, n = t - lf * ND, x = (lf & 1) ? n / N1 : n % N1;
-      sMB[t] = H.b[(lf * NQF + (lf >= 2 ? N1 - 1 - x : x)) * ND + n];
-    }
+    for (int t = tid; t < ND; t += NT) sMD[ND * NTERM + t] = H.pm[t];
+    for (int t = tid; t < NFPE * ND; t += NT) sMB[t] = H.pb[t];
   } else {
     for (int t = tid; t < (G == 2 ? DIM * ND * ND : N1 * N1); t += NT) sMD[t] = H.md[t];
     for (int t = tid; t < (G == 2 ? NFPE * NQF * ND : 2 * N1); t += NT) sMB[t] = H.mb[t];
